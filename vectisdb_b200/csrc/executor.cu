@@ -839,7 +839,9 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	const auto &props = Runtime::Get().props();
 	const int F = PipelineCodegen::StateWords(gb);
 	const uint64_t domain = 1ull << shift;
-	const bool direct = domain * static_cast<uint64_t>(F) * 8 <= 96 * 1024;  // 8-byte words per slot bound the choice
+	// 8-byte words per slot bound the choice; more than 2^13 slots never fit, and the product of a wide key
+	// space (60 bits and up) would wrap
+	const bool direct = shift <= 13 && domain * static_cast<uint64_t>(F) * 8 <= 96 * 1024;
 	// FP64 sums of the one-pass group-by in L2-resident per-CTA tables (VGPU_GB_DIRECT_F64_L2=1)
 	const char *env_dl2 = std::getenv("VGPU_GB_DIRECT_F64_L2");
 	const int direct_f64 = PipelineCodegen::F64Fields(gb);
