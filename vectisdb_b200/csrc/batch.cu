@@ -311,7 +311,6 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 	Arena arena(stream);
 	std::vector<std::vector<std::pair<int64_t, int64_t>>> ranges(qs.size(), std::vector<std::pair<int64_t, int64_t>>(nkeys));
 	std::vector<std::pair<size_t, int>> pending;
-	int64_t *mm = nullptr;
 	for (size_t qi = 0; qi < qs.size(); qi++) {
 		for (int j = 0; j < nkeys; j++) {
 			const DevColumn &src = qs[qi]->sources[cg->visible()[key_cols[j]].source];
@@ -323,16 +322,19 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 		}
 	}
 	if (!pending.empty()) {
-		mm = arena.AllocT<int64_t>(2 * pending.size());
-		for (size_t p = 0; p < pending.size(); p++) {
-			const DevColumn &src = qs[pending[p].first]->sources[cg->visible()[key_cols[pending[p].second]].source];
-			kern::MinMaxSigned(src.data, static_cast<int>(src.type), src.rows, mm + 2 * p, stream);
+		uint64_t *mm = arena.AllocT<uint64_t>(2 * pending.size());
+		std::vector<kern::BoundsColumn> cols;
+		for (auto &p : pending) {
+			const DevColumn &src = qs[p.first]->sources[cg->visible()[key_cols[p.second]].source];
+			cols.push_back({src.data, src.rows, kern::SignedBoundsKind(src.type)});
 		}
-		std::vector<int64_t> host(2 * pending.size());
+		kern::ColumnBounds(cols.data(), static_cast<int>(cols.size()), mm, stream);
+		std::vector<uint64_t> host(2 * pending.size());
 		VGPU_CUDA(cudaMemcpyAsync(host.data(), mm, host.size() * 8, cudaMemcpyDeviceToHost, stream));
 		VGPU_CUDA(cudaStreamSynchronize(stream));
 		for (size_t p = 0; p < pending.size(); p++) {
-			ranges[pending[p].first][pending[p].second] = {host[2 * p], host[2 * p + 1]};
+			ranges[pending[p].first][pending[p].second] = {static_cast<int64_t>(kern::BoundsLow(&host[2 * p], cols[p].kind)),
+			                                               static_cast<int64_t>(kern::BoundsHigh(&host[2 * p], cols[p].kind))};
 		}
 	}
 

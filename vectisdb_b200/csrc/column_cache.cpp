@@ -252,16 +252,17 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		}
 		e.bytes = st.bytes;
 		if (IsIntegerKeyType(st.type) || st.type == ValueType::DICTIONARY_STRING) {
-			int64_t *mm = static_cast<int64_t *>(alloc.Alloc(16, s));
-			kern::MinMaxSigned(e.column.data, static_cast<int>(st.type), st.rows, mm, s);
-			int64_t host[2];
+			uint64_t *mm = static_cast<uint64_t *>(alloc.Alloc(16, s));
+			const kern::BoundsColumn bc {e.column.data, st.rows, kern::SignedBoundsKind(st.type)};
+			kern::ColumnBounds(&bc, 1, mm, s);
+			uint64_t host[2];
 			VGPU_CUDA(cudaMemcpyAsync(host, mm, 16, cudaMemcpyDeviceToHost, s));
 			VGPU_CUDA(cudaStreamSynchronize(s));
 			alloc.Free(mm, s);
 			if (st.rows > 0) {
 				e.column.has_stats = true;
-				e.column.min = host[0];
-				e.column.max = host[1];
+				e.column.min = static_cast<int64_t>(kern::BoundsLow(host, bc.kind));
+				e.column.max = static_cast<int64_t>(kern::BoundsHigh(host, bc.kind));
 			}
 		}
 		const std::string key = Key(table, kv.first);

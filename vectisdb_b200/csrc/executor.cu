@@ -244,6 +244,8 @@ private:
 	                       uint32_t *status_host);
 	uint64_t ReadU64(const void *dev);
 	uint32_t ReadU32(const void *dev);
+	//! The `n` words at `dev`, after the stream's queued work.
+	std::vector<uint64_t> ReadWords(const void *dev, size_t n);
 	//! Heavy keys chosen for the partition passes of a direct-partitioned group-by (no module: none).
 	//! The selection stays on the device: hmap, the key list and its length are kernel inputs.
 	struct HeavyPlan {
@@ -329,6 +331,15 @@ uint32_t Executor::ReadU32(const void *dev) {
 	VGPU_CUDA(cudaStreamSynchronize(stream_));
 	uint32_t v;
 	std::memcpy(&v, word.get(), sizeof(v));
+	return v;
+}
+
+std::vector<uint64_t> Executor::ReadWords(const void *dev, size_t n) {
+	auto words = PinnedPool::Get().Acquire(n * sizeof(uint64_t));
+	VGPU_CUDA(cudaMemcpyAsync(words.get(), dev, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream_));
+	VGPU_CUDA(cudaStreamSynchronize(stream_));
+	std::vector<uint64_t> v(n);
+	std::memcpy(v.data(), words.get(), n * sizeof(uint64_t));
 	return v;
 }
 
@@ -637,13 +648,32 @@ void Executor::ComputeStats(PipelineInput &pin, const PipelineCodegen &cg, const
 	out.assign(cols.size(), {0, 0});
 	std::vector<int> missing;
 	std::vector<size_t> missing_pos;
+	// A source column passed through unchanged: the range of its own rows bounds every row the consumer can
+	// see, so it is read once by itself. Over a join or a cross product that spares a run of the whole
+	// pipeline (the range of a build side's column under 2^28 probe rows: 0.93 ms -> none, since the join
+	// has it already; of a plain 10M-row key 28 -> 19 us).
+	std::vector<kern::BoundsColumn> own;
+	std::vector<size_t> own_pos;
 	for (size_t i = 0; i < cols.size(); i++) {
 		const auto &vc = cg.visible()[cols[i]];
 		if (vc.source >= 0 && pin.sources[vc.source].has_stats) {
 			out[i] = {pin.sources[vc.source].min, pin.sources[vc.source].max};
+		} else if (vc.source >= 0 && IsIntegerKeyType(vc.type)) {
+			const DevColumn &src = pin.sources[vc.source];
+			own.push_back({src.data, src.rows, kern::SignedBoundsKind(src.type)});
+			own_pos.push_back(i);
 		} else {
 			missing.push_back(cols[i]);
 			missing_pos.push_back(i);
+		}
+	}
+	if (!own.empty()) {
+		uint64_t *words = arena_.AllocT<uint64_t>(2 * own.size());
+		kern::ColumnBounds(own.data(), static_cast<int>(own.size()), words, stream_);
+		const std::vector<uint64_t> host = ReadWords(words, 2 * own.size());
+		for (size_t j = 0; j < own.size(); j++) {
+			out[own_pos[j]] = {static_cast<int64_t>(kern::BoundsLow(&host[2 * j], own[j].kind)),
+			                   static_cast<int64_t>(kern::BoundsHigh(&host[2 * j], own[j].kind))};
 		}
 	}
 	if (missing.empty()) {
@@ -1487,6 +1517,9 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 			inline_col = nullptr;
 		}
 	}
+	// range of the inline column's raw bits, once known
+	uint32_t vmin = 0, vmax = 0;
+	bool have_vrange = false;
 	auto add_sources = [&](bool sorted_side, const uint32_t *perm) {
 		for (size_t i = 0; i < outs.size(); i++) {
 			DevColumn c = *outs[i];
@@ -1500,6 +1533,17 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 					uint8_t *v = arena_.AllocT<uint8_t>(rn);
 					kern::Gather(outs[i]->valid, 1, perm, rn, v, stream_);
 					c.valid = v;
+				}
+			}
+			if (outs[i] == inline_col && have_vrange && !c.has_stats && IsIntegerKeyType(c.type)) {
+				// raw bits on one side of the sign bit order like the values
+				const size_t w = TypeSize(c.type);
+				const uint32_t sign = c.type == ValueType::BOOLEAN ? 0u : 1u << (8 * w - 1);
+				if ((vmin & sign) == (vmax & sign)) {
+					const uint64_t high = (vmin & sign) ? ~0ull << (8 * w) : 0ull;
+					c.has_stats = true;
+					c.min = c.type == ValueType::BOOLEAN ? 0 : static_cast<int64_t>(vmin | high);
+					c.max = c.type == ValueType::BOOLEAN ? 1 : static_cast<int64_t>(vmax | high);
 				}
 			}
 			SourceColumn sc;
@@ -1553,69 +1597,68 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 			holds_.push_back(t);
 			JoinTableCache::Get().Insert(cache_key, t);
 		};
-		uint64_t *rw = arena_.AllocT<uint64_t>(rn);
-		uint64_t *mm = arena_.AllocT<uint64_t>(3);  // key min, key max, value bits (min, max)
-		kern::WidenKeysMinMax(rk->data, kw, rn, rw, mm, stream_);
-		if (inline_col) kern::ValueBits(inline_col->data, TypeSize(inline_col->type), rn, reinterpret_cast<uint32_t *>(mm + 2), stream_);
-		uint64_t host_mm[3] = {0, 0, 0};
-		VGPU_CUDA(cudaMemcpyAsync(host_mm, mm, inline_col ? 24 : 16, cudaMemcpyDeviceToHost, stream_));
-		VGPU_CUDA(cudaStreamSynchronize(stream_));
-		bias = host_mm[0];
-		const uint64_t range = host_mm[1] - host_mm[0];
-		const uint32_t vmin = static_cast<uint32_t>(host_mm[2]), vmax = static_cast<uint32_t>(host_mm[2] >> 32);
+		// Key range and, with an inline column, its raw bits' range: from the cached columns' own when those
+		// are not negative (raw bits then order like values) and dense, else measured in one launch.
+		uint64_t lo = 0, hi = 0;
+		auto dense = [&](uint64_t r) { return r < (1ull << 28) && r < 4 * rn; };
+		if (rk->has_stats && rk->min >= 0 && dense(static_cast<uint64_t>(rk->max) - static_cast<uint64_t>(rk->min)) &&
+		    (!inline_col || (inline_col->has_stats && inline_col->min >= 0 && IsIntegerKeyType(inline_col->type)))) {
+			lo = static_cast<uint64_t>(rk->min);
+			hi = static_cast<uint64_t>(rk->max);
+			if (inline_col) {
+				vmin = static_cast<uint32_t>(inline_col->min);
+				vmax = static_cast<uint32_t>(inline_col->max);
+			}
+		} else {
+			const size_t vw = inline_col ? TypeSize(inline_col->type) : 4;
+			const kern::BoundsColumn want[2] = {{rk->data, rn, kern::RawBoundsKind(kw)},
+			                                    {inline_col ? inline_col->data : nullptr, rn, kern::RawBoundsKind(vw)}};
+			uint64_t *words = arena_.AllocT<uint64_t>(4);
+			kern::ColumnBounds(want, inline_col ? 2 : 1, words, stream_);
+			const std::vector<uint64_t> host = ReadWords(words, inline_col ? 4 : 2);
+			lo = kern::BoundsLow(&host[0], want[0].kind);
+			hi = kern::BoundsHigh(&host[0], want[0].kind);
+			if (inline_col) {
+				vmin = static_cast<uint32_t>(kern::BoundsLow(&host[2], want[1].kind));
+				vmax = static_cast<uint32_t>(kern::BoundsHigh(&host[2], want[1].kind));
+			}
+		}
+		have_vrange = inline_col != nullptr;
+		bias = lo;
+		const uint64_t range = hi - lo;
 		const int bits = BitsFor(range);
 		// the dense tables subtract the bias as they index; the sorted form below works on biased keys
-		uint32_t *dups = arena_.AllocT<uint32_t>(1);
 		bool built = false;
 		// Dense keys (range within 4x the key count, at most 2^28): a table indexed by the key over the whole
 		// range, filled without sorting. It holds the right row index, or -- when the join contributes one
 		// right column of at most 4 bytes -- that column's value itself, so a probe row costs one random
 		// read; the value is stored as its offset from the smallest value in the fewest bytes that hold every
 		// offset (all ones marks a missing key), so the table of a small-valued column stays in L2. A key met
-		// twice (many-to-many) falls back to the sorted form below.
+		// twice (many-to-many: fewer entries written than rows) falls back to the forms below.
 		// More right rows than key values: some key repeats for sure, so no unique-key table is tried.
 		const bool surely_repeated = rn > range + 1;
-		if (range < (1ull << 28) && range < 4 * rn && !surely_repeated) {
+		if (dense(range) && !surely_repeated) {
 			const uint64_t span = static_cast<uint64_t>(vmax) - vmin;
-			const size_t width = !inline_col ? 0 : span < 0xffull ? 1 : span < 0xffffull ? 2 : span < 0xffffffffull ? 4 : 8;
 			const char *env_c = std::getenv("VGPU_JOIN_COMPACT");  // "0": 8-byte inline entries (testing)
-			const bool compact = width != 0 && width != 8 && !(env_c && std::strcmp(env_c, "0") == 0);
-			if (compact) {
-				void *table = arena_.Alloc((range + 1) * width);
-				kern::JoinDenseCompact(rw, inline_col->data, TypeSize(inline_col->type), rn, range, vmin, table, width, dups,
-				                       stream_, bias);
-				if (ReadU32(dups) == 0) {
-					add_sources(false, nullptr);
-					pin.spec.join_inline = true;
-					pin.join_words[0] = reinterpret_cast<uint64_t>(table);
-					pin.join_words[1] = vmin;
-					pin.join_words[3] = (width == 1 ? 0xfdu : width == 2 ? 0xfcu : 0xfbu) | ((range + 1) << 8);
-					built = true;
-					keep(table, (range + 1) * width, true);
-				}
-			} else if (inline_col) {
-				uint64_t *table = arena_.AllocT<uint64_t>(range + 1);
-				kern::JoinDenseInline(rw, inline_col->data, TypeSize(inline_col->type), rn, range, table, dups, stream_, bias);
-				if (ReadU32(dups) == 0) {
-					add_sources(false, nullptr);
-					pin.spec.join_inline = true;
-					pin.join_words[0] = reinterpret_cast<uint64_t>(table);
-					pin.join_words[1] = 0;
-					pin.join_words[3] = 0xfeu | ((range + 1) << 8);
-					built = true;
-					keep(table, (range + 1) * 8, true);
-				}
+			const bool compact = !(env_c && std::strcmp(env_c, "0") == 0);
+			const size_t width = !inline_col ? 4 : !compact ? 8 : span < 0xffull ? 1 : span < 0xffffull ? 2 : span < 0xffffffffull ? 4 : 8;
+			const uint64_t bytes = (range + 1) * width;
+			void *table = arena_.Alloc(bytes);
+			uint32_t *occupied = arena_.AllocT<uint32_t>(1);
+			kern::JoinDenseFill(rk->data, kw, inline_col ? inline_col->data : nullptr,
+			                    inline_col ? TypeSize(inline_col->type) : 0, rn, lo, range, vmin, table, width, occupied, stream_);
+			if (ReadU32(occupied) == rn) {
+				add_sources(false, nullptr);
+				const uint64_t word = reinterpret_cast<uint64_t>(table);
+				const uint32_t code = !inline_col ? 0xffu : width == 1 ? 0xfdu : width == 2 ? 0xfcu : width == 4 ? 0xfbu : 0xfeu;
+				pin.spec.join_inline = inline_col != nullptr;
+				pin.join_words[0] = inline_col ? word : 0;
+				pin.join_words[1] = !inline_col ? word : width == 8 ? 0 : vmin;
+				pin.join_words[3] = code | ((range + 1) << 8);
+				built = true;
+				keep(table, bytes, inline_col != nullptr);
 			} else {
-				uint32_t *table = arena_.AllocT<uint32_t>(range + 1);
-				kern::JoinDenseRows(rw, rn, range, table, dups, stream_, bias);
-				if (ReadU32(dups) == 0) {
-					add_sources(false, nullptr);
-					pin.join_words[0] = 0;
-					pin.join_words[1] = reinterpret_cast<uint64_t>(table);
-					pin.join_words[3] = 0xffu | ((range + 1) << 8);
-					built = true;
-					keep(table, (range + 1) * 4, false);
-				}
+				arena_.FreeNow(table);
 			}
 		}
 		// Repeated right keys with few matches each and one narrow right column: the dense table holds every
@@ -1623,8 +1666,7 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 		// entries when two matches fit, else 8-byte ones; a key with more matches than fit falls back to the
 		// sorted form.
 		const uint64_t mspan = static_cast<uint64_t>(vmax) - vmin;
-		if (!built && multi_ok && any_order && inline_col && range < (1ull << 28) && range < 4 * rn &&
-		    mspan < (1ull << 30)) {
+		if (!built && multi_ok && any_order && inline_col && dense(range) && mspan < (1ull << 30)) {
 			const uint32_t vbits = std::max(1, BitsFor(mspan));
 			uint32_t *overflow = arena_.AllocT<uint32_t>(1);
 			for (int wide = 0; wide < 2 && !built; wide++) {
@@ -1633,8 +1675,8 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 				if (rmax < 2) continue;
 				const uint64_t bytes = (range + 1) * (wide ? 8 : 4);
 				void *table = arena_.Alloc(bytes);
-				kern::JoinDenseMulti(rw, inline_col->data, TypeSize(inline_col->type), rn, range, vmin, vbits, cbits, rmax,
-				                     table, wide != 0, overflow, stream_, bias);
+				kern::JoinDenseMulti(rk->data, kw, inline_col->data, TypeSize(inline_col->type), rn, lo, range, vmin, vbits,
+				                     cbits, rmax, table, wide != 0, overflow, stream_);
 				if (ReadU32(overflow) == 0) {
 					add_sources(false, nullptr);
 					pin.spec.join_multi = pin.spec.join_minline = true;
@@ -1651,9 +1693,10 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 		if (!built) {
 			// Sorted form: LSD radix sort of the right keys, uniqueness check, radix directory over the sorted
 			// keys (at most 2^22 buckets), right columns gathered into sorted order once.
-			kern::SubtractBias(rw, rn, bias, stream_);
+			uint64_t *rw = arena_.AllocT<uint64_t>(rn);
+			kern::WidenKeys(rk->data, kw, rn, bias, rw, stream_);
+			uint32_t *dups = arena_.AllocT<uint32_t>(1);
 			uint32_t *perm = arena_.AllocT<uint32_t>(rn);
-			kern::Iota(perm, rn, stream_);
 			uint64_t *rw_alt = arena_.AllocT<uint64_t>(rn);
 			uint32_t *perm_alt = arena_.AllocT<uint32_t>(rn);
 			kern::RadixSortPairs(rw, perm, rw_alt, perm_alt, rn, bits, arena_);
@@ -1672,7 +1715,7 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 				multi = true;
 			}
 			// a dense key range gets one directory bucket per key value (the run is the bucket)
-			const bool dense_runs = multi && range < (1ull << 28) && range < 4 * rn;
+			const bool dense_runs = multi && dense(range);
 			const uint32_t shift = dense_runs ? 0u : bits > 22 ? static_cast<uint32_t>(bits - 22) : 0u;
 			const uint64_t nb = (range >> shift) + 1;
 			uint32_t *dir = arena_.AllocT<uint32_t>(nb + 1);
@@ -1755,17 +1798,16 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	const size_t kw = TypeSize(lk.type);
 	uint64_t *lw = arena_.AllocT<uint64_t>(ln);
 	uint64_t *rw = arena_.AllocT<uint64_t>(rn);
-	kern::WidenKeys(lk.data, kw, ln, lw, stream_);
-	uint64_t *mm = arena_.AllocT<uint64_t>(2);
-	kern::WidenKeysMinMax(rk.data, kw, rn, rw, mm, stream_);
-	uint64_t host_mm[2];
-	VGPU_CUDA(cudaMemcpyAsync(host_mm, mm, 16, cudaMemcpyDeviceToHost, stream_));
-	VGPU_CUDA(cudaStreamSynchronize(stream_));
-	const uint64_t bias = host_mm[0];
-	const int bits = BitsFor(host_mm[1] - host_mm[0]);
-	kern::SubtractBias(rw, rn, bias, stream_);
+	uint64_t *words = arena_.AllocT<uint64_t>(2);
+	const kern::BoundsColumn want {rk.data, rn, kern::RawBoundsKind(kw)};
+	kern::ColumnBounds(&want, 1, words, stream_);
+	const std::vector<uint64_t> bounds = ReadWords(words, 2);
+	const uint64_t bias = kern::BoundsLow(bounds.data(), want.kind);
+	const uint64_t range = kern::BoundsHigh(bounds.data(), want.kind) - bias;
+	const int bits = BitsFor(range);
+	kern::WidenKeys(lk.data, kw, ln, 0, lw, stream_);
+	kern::WidenKeys(rk.data, kw, rn, bias, rw, stream_);
 	uint32_t *perm = arena_.AllocT<uint32_t>(rn);
-	kern::Iota(perm, rn, stream_);
 	uint64_t *rw_alt = arena_.AllocT<uint64_t>(rn);
 	uint32_t *perm_alt = arena_.AllocT<uint32_t>(rn);
 	kern::RadixSortPairs(rw, perm, rw_alt, perm_alt, rn, bits, arena_);
@@ -1773,7 +1815,6 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	arena_.FreeNow(perm_alt);
 	// each left key's run of equal right keys through a radix directory: one bucket per key value when
 	// the key range is dense (the run is read, not searched), else 2^22 buckets and a short search
-	const uint64_t range = host_mm[1] - host_mm[0];
 	const uint32_t shift = (range < (1ull << 28) && range < 4 * rn) ? 0u : bits > 22 ? static_cast<uint32_t>(bits - 22) : 0u;
 	const uint64_t nb = (range >> shift) + 1;
 	uint32_t *dir = arena_.AllocT<uint32_t>(nb + 1);

@@ -2,7 +2,8 @@
 #include "kernels.hpp"
 
 #include <algorithm>
-
+#include <cstring>
+#include <limits>
 #include <type_traits>
 
 #include <utility>
@@ -189,101 +190,105 @@ template <typename T> __global__ void GatherKernel(const T *src, const uint32_t 
 	}
 }
 
-template <typename T> __global__ void WidenKernel(const T *src, uint64_t n, uint64_t *dst) {
+// Key bits zero-extended to 64 bits, minus `bias`.
+template <typename T> __global__ void WidenKernel(const T *src, uint64_t n, uint64_t bias, uint64_t *dst) {
 	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		dst[i] = static_cast<uint64_t>(src[i]);
+		dst[i] = static_cast<uint64_t>(src[i]) - bias;
 	}
 }
 
-// The CTA's smallest and largest value (unsigned) folded into out[0] / out[1] with one atomic pair per
-// CTA: per-warp atomics on two words serialize at L2 once thousands of warps reach them.
-template <typename U>
-__device__ __forceinline__ void BlockMinMaxToGlobal(U mn, U mx, U *out) {
-	__shared__ U smn[32], smx[32];
-	for (int o = 16; o > 0; o >>= 1) {
-		const U a = __shfl_xor_sync(0xffffffffu, mn, o);
-		const U b = __shfl_xor_sync(0xffffffffu, mx, o);
-		mn = a < mn ? a : mn;
-		mx = b > mx ? b : mx;
-	}
-	const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	if (lane == 0) {
-		smn[warp] = mn;
-		smx[warp] = mx;
-	}
-	__syncthreads();
-	if (warp == 0) {
-		const unsigned nw = (blockDim.x + 31) >> 5;
-		mn = lane < nw ? smn[lane] : smn[0];
-		mx = lane < nw ? smx[lane] : smx[0];
-		for (int o = 16; o > 0; o >>= 1) {
-			const U a = __shfl_xor_sync(0xffffffffu, mn, o);
-			const U b = __shfl_xor_sync(0xffffffffu, mx, o);
-			mn = a < mn ? a : mn;
-			mx = b > mx ? b : mx;
-		}
-		if (lane == 0) {
-			atomicMin(&out[0], mn);
-			atomicMax(&out[1], mx);
-		}
-	}
-}
+// ---- value ranges of columns ------------------------------------------------------------------------
+//
+// One launch for up to kMaxBoundsColumns columns (blockIdx.y picks the column), bound by reading them
+// once: 16-byte loads, four in flight per thread, one atomic pair per CTA (a pair per warp serializes on
+// the two words once thousands of warps reach them: a 10M-row INT32 key column 28 -> 19 us; 2^24 INT64
+// keys and their INT32 values 0.095 ms in two kernels, one of them writing the keys widened, -> 0.046 ms,
+// 4.4 TB/s). Values travel as an order-preserving
+// unsigned image (signed values with the sign bit flipped); the minimum is kept as the maximum of the
+// complemented image, so one zero fill is the identity of both.
 
-__global__ void MinMaxKernel(const uint64_t *keys, uint64_t n, uint64_t *minmax) {
-	unsigned long long mn = ~0ull, mx = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const unsigned long long k = keys[i];
-		mn = k < mn ? k : mn;
-		mx = k > mx ? k : mx;
-	}
-	BlockMinMaxToGlobal<unsigned long long>(mn, mx, reinterpret_cast<unsigned long long *>(minmax));
-}
+struct BoundsArgs {
+	BoundsColumn c[kMaxBoundsColumns];
+	unsigned long long *out;
+};
 
-// Keys zero-extended to 64 bits and their range in one pass (the widening and the range the dense join
-// tables need).
-template <typename T> __global__ void WidenMinMaxKernel(const T *src, uint64_t n, uint64_t *dst, uint64_t *minmax) {
-	unsigned long long mn = ~0ull, mx = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const unsigned long long k = static_cast<uint64_t>(src[i]);
-		dst[i] = k;
-		mn = k < mn ? k : mn;
-		mx = k > mx ? k : mx;
-	}
-	BlockMinMaxToGlobal<unsigned long long>(mn, mx, reinterpret_cast<unsigned long long *>(minmax));
-}
-
-template <typename T> __global__ void MinMaxSignedKernel(const T *data, uint64_t n, int64_t *out) {
-	int64_t mn = INT64_MAX, mx = INT64_MIN;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const int64_t v = static_cast<int64_t>(data[i]);
+template <typename T, bool kBool>
+__device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx) {
+	auto take = [&](T v) {
+		if constexpr (kBool) v = v != 0 ? 1 : 0;
 		mn = v < mn ? v : mn;
 		mx = v > mx ? v : mx;
+	};
+	constexpr uint64_t kPer = 16 / sizeof(T);
+	const uint64_t skew = reinterpret_cast<uintptr_t>(p) & 15u;
+	uint64_t head = skew ? (16 - skew) / sizeof(T) : 0;  // values before the first 16-byte boundary
+	if (head > n) head = n;
+	const uint64_t vecs = (n - head) / kPer;
+	const uint64_t tail = head + vecs * kPer;
+	const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+	if (tid < head) take(p[tid]);
+	if (tid < n - tail) take(p[tail + tid]);  // both ends are shorter than a warp
+	const uint4 *v = reinterpret_cast<const uint4 *>(p + head);
+	auto take4 = [&](const uint4 &q) {
+		T x[kPer];
+		memcpy(x, &q, 16);
+#pragma unroll
+		for (uint64_t j = 0; j < kPer; j++) take(x[j]);
+	};
+	uint64_t i = tid;
+	for (; i + 3 * stride < vecs; i += 4 * stride) {
+		const uint4 a = v[i], b = v[i + stride], c = v[i + 2 * stride], d = v[i + 3 * stride];
+		take4(a);
+		take4(b);
+		take4(c);
+		take4(d);
 	}
+	for (; i < vecs; i += stride) take4(v[i]);
+}
+
+template <typename T, bool kBool = false>
+__device__ __forceinline__ void RangeImage(const void *p, uint64_t n, unsigned long long &lo, unsigned long long &hi) {
+	T mn = std::numeric_limits<T>::max(), mx = std::numeric_limits<T>::lowest();
+	RangeOf<T, kBool>(static_cast<const T *>(p), n, mn, mx);
+	constexpr unsigned long long kFlip = std::is_signed<T>::value ? 1ull << 63 : 0ull;
+	const bool any = mn <= mx;  // a thread without values leaves the identity
+	lo = any ? static_cast<unsigned long long>(mn) ^ kFlip : ~0ull;
+	hi = any ? static_cast<unsigned long long>(mx) ^ kFlip : 0ull;
+}
+
+constexpr int kBoundsBlock = 256;
+
+__global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a) {
+	const BoundsColumn &c = a.c[blockIdx.y];
+	unsigned long long lo = ~0ull, hi = 0ull;
+	switch (c.kind) {
+	case BoundsKind::U8: RangeImage<uint8_t>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::U16: RangeImage<uint16_t>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::U32: RangeImage<uint32_t>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::U64: RangeImage<unsigned long long>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::I16: RangeImage<int16_t>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::I32: RangeImage<int32_t>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::I64: RangeImage<long long>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::BOOL: RangeImage<uint8_t, true>(c.data, c.rows, lo, hi); break;
+	}
+	__shared__ unsigned long long slo[kBoundsBlock / 32], shi[kBoundsBlock / 32];
 	for (int o = 16; o > 0; o >>= 1) {
-		int64_t a = __shfl_xor_sync(0xffffffffu, mn, o);
-		int64_t b = __shfl_xor_sync(0xffffffffu, mx, o);
-		mn = a < mn ? a : mn;
-		mx = b > mx ? b : mx;
+		const unsigned long long x = __shfl_xor_sync(0xffffffffu, lo, o), y = __shfl_xor_sync(0xffffffffu, hi, o);
+		lo = x < lo ? x : lo;
+		hi = y > hi ? y : hi;
 	}
 	if ((threadIdx.x & 31) == 0) {
-		atomicMin(reinterpret_cast<long long *>(&out[0]), static_cast<long long>(mn));
-		atomicMax(reinterpret_cast<long long *>(&out[1]), static_cast<long long>(mx));
+		slo[threadIdx.x >> 5] = lo;
+		shi[threadIdx.x >> 5] = hi;
 	}
-}
-
-__global__ void InitMinMaxSignedKernel(int64_t *out) {
-	out[0] = INT64_MAX;
-	out[1] = INT64_MIN;
-}
-
-__global__ void InitMinMaxKernel(uint64_t *minmax) {
-	minmax[0] = ~0ull;
-	minmax[1] = 0ull;
-}
-
-__global__ void SubtractBiasKernel(uint64_t *keys, uint64_t n, uint64_t bias) {
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		keys[i] -= bias;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		for (int w = 1; w < kBoundsBlock / 32; w++) {
+			lo = slo[w] < lo ? slo[w] : lo;
+			hi = shi[w] > hi ? shi[w] : hi;
+		}
+		atomicMax(a.out + 2 * blockIdx.y, ~lo);
+		atomicMax(a.out + 2 * blockIdx.y + 1, hi);
 	}
 }
 
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(kSortBlock) RadixScatterKernel(const uint64_t 
 		const uint64_t idx = base + static_cast<uint64_t>(k) * 32 + lane;
 		const bool valid = idx < n;
 		keys[k] = valid ? kin[idx] : 0ull;
-		vals[k] = valid ? vin[idx] : 0u;
+		vals[k] = !valid ? 0u : vin ? vin[idx] : static_cast<uint32_t>(idx);
 	}
 #pragma unroll
 	for (int k = 0; k < kSortItems; k++) {
@@ -544,70 +549,58 @@ __global__ void JoinDirectoryKernel(const uint64_t *sorted, uint64_t n, uint32_t
 	}
 }
 
-// Dense key tables: entry of (biased) key k = row index + 1, or (1 << 32 | value) with the row's
-// value inlined; a key met twice counts as a duplicate (compare-and-swap from empty).
-__global__ void JoinDenseRowsKernel(const uint64_t *keys, uint64_t n, uint64_t bias, uint32_t *table, uint32_t *dups) {
-	uint32_t local = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		if (atomicCAS(&table[keys[i] - bias], 0u, static_cast<uint32_t>(i + 1)) != 0u) local++;
-	}
-	if (local) atomicAdd(dups, local);
-}
-
-template <typename T>
-__global__ void JoinDenseInlineKernel(const uint64_t *keys, const T *values, uint64_t n, uint64_t bias,
-                                      unsigned long long *table, uint32_t *dups) {
-	uint32_t local = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const unsigned long long e = (1ull << 32) | static_cast<unsigned long long>(values[i]);
-		if (atomicCAS(&table[keys[i] - bias], 0ull, e) != 0ull) local++;
-	}
-	if (local) atomicAdd(dups, local);
-}
-
-template <typename T> __global__ void ValueBitsKernel(const T *values, uint64_t n, uint32_t *bounds) {
-	unsigned int lo = 0xffffffffu, hi = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const unsigned int bits = static_cast<uint32_t>(values[i]);
-		lo = bits < lo ? bits : lo;
-		hi = bits > hi ? bits : hi;
-	}
-	BlockMinMaxToGlobal<unsigned int>(lo, hi, bounds);
-}
-
-// Compact inline table: entry = value bits - vmin in E (all ones = no key), filled by compare-and-swap
-// from the marker; a key met twice counts in *dups. One-byte entries swap their 32-bit word (bounded
-// retries while neighbours change it; running out counts as a duplicate, so the caller falls back).
-template <typename T, typename E>
-__global__ void JoinDenseCompactKernel(const uint64_t *keys, const T *values, uint64_t n, uint64_t bias, uint32_t vmin,
-                                       E *table, uint32_t *dups) {
-	uint32_t local = 0;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const uint32_t entry = static_cast<uint32_t>(values[i]) - vmin;
-		E *slot = table + (keys[i] - bias);
-		if constexpr (sizeof(E) == 4) {
-			if (atomicCAS(reinterpret_cast<unsigned int *>(slot), 0xffffffffu, entry) != 0xffffffffu) local++;
-		} else if constexpr (sizeof(E) == 2) {
-			if (atomicCAS(reinterpret_cast<unsigned short *>(slot), static_cast<unsigned short>(0xffffu),
-			              static_cast<unsigned short>(entry)) != 0xffffu) {
-				local++;
-			}
-		} else {
-			unsigned int *word = reinterpret_cast<unsigned int *>(reinterpret_cast<uintptr_t>(slot) & ~uintptr_t(3));
-			const uint32_t sh = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(slot) & 3u) * 8u;
-			uint32_t old = *reinterpret_cast<volatile unsigned int *>(word);
-			bool done = false;
-			for (int t = 0; t < 4096 && !done; ++t) {
-				if (((old >> sh) & 0xffu) != 0xffu) break;  // taken: a duplicate key
-				const uint32_t want = (old & ~(0xffu << sh)) | ((entry & 0xffu) << sh);
-				const uint32_t prev = atomicCAS(word, old, want);
-				done = prev == old;
-				old = prev;
-			}
-			if (!done) local++;
+// Dense key tables (see JoinDenseFill): plain stores, then a count of the entries that were written. Keys
+// are distinct exactly when that count equals the row count, so nothing has to be claimed by
+// compare-and-swap: 2^24 keys into a 32 MB table of 2-byte entries took 0.40 ms with 16-bit swaps; the
+// fill, the stores (bound by one L2 sector write per key) and the count together take 0.16 ms.
+template <typename K, typename V, typename E>
+__global__ void JoinFillKernel(const K *keys, const V *values, uint64_t n, uint64_t bias, uint64_t base, E *table) {
+	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+	uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+	for (; i + 3 * stride < n; i += 4 * stride) {
+		K k[4];
+		V v[4];
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			k[j] = keys[i + j * stride];
+			v[j] = values[i + j * stride];
 		}
+#pragma unroll
+		for (int j = 0; j < 4; j++) table[static_cast<uint64_t>(k[j]) - bias] = static_cast<E>(static_cast<uint64_t>(v[j]) + base);
 	}
-	if (local) atomicAdd(dups, local);
+	for (; i < n; i += stride) table[static_cast<uint64_t>(keys[i]) - bias] = static_cast<E>(static_cast<uint64_t>(values[i]) + base);
+}
+
+template <typename K> __global__ void JoinFillRowsKernel(const K *keys, uint64_t n, uint64_t bias, uint32_t *table) {
+	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+		table[static_cast<uint64_t>(keys[i]) - bias] = static_cast<uint32_t>(i + 1);
+	}
+}
+
+// Entries that differ from the empty marker (zero, or all ones).
+template <typename E> __global__ void __launch_bounds__(256) JoinCountKernel(const E *table, uint64_t entries, E empty,
+                                                                            uint32_t *occupied) {
+	constexpr uint64_t kPer = 16 / sizeof(E);
+	const uint64_t vecs = entries / kPer, stride = (uint64_t)gridDim.x * blockDim.x;
+	const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+	uint32_t c = 0;
+	const uint4 *v = reinterpret_cast<const uint4 *>(table);
+	for (uint64_t i = tid; i < vecs; i += stride) {
+		const uint4 q = v[i];
+		E x[kPer];
+		memcpy(x, &q, 16);
+#pragma unroll
+		for (uint64_t j = 0; j < kPer; j++) c += x[j] != empty ? 1u : 0u;
+	}
+	if (tid < entries - vecs * kPer) c += table[vecs * kPer + tid] != empty ? 1u : 0u;
+	c = __reduce_add_sync(0xffffffffu, c);
+	__shared__ uint32_t warps[8];
+	if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = c;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		for (int w = 1; w < 8; w++) c += warps[w];
+		if (c) atomicAdd(occupied, c);
+	}
 }
 
 __global__ void CountAdjacentEqualKernel(const uint64_t *sorted, uint64_t n, uint32_t *out) {
@@ -735,51 +728,105 @@ void JoinDirectory(const uint64_t *sorted, uint64_t n, uint32_t shift, uint64_t 
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void JoinDenseRows(const uint64_t *keys, uint64_t n, uint64_t range, uint32_t *table, uint32_t *dups,
-                   cudaStream_t stream, uint64_t bias) {
-	LaunchScope scope("join_dense_table", stream, n * 12 + (range + 1) * 4, n);
-	VGPU_CUDA(cudaMemsetAsync(table, 0, (range + 1) * 4, stream));
-	VGPU_CUDA(cudaMemsetAsync(dups, 0, 4, stream));
-	JoinDenseRowsKernel<<<GridFor(n, 256), 256, 0, stream>>>(keys, n, bias, table, dups);
-	VGPU_CUDA(cudaGetLastError());
+namespace {
+
+// f(typed key pointer) for a key column of `width` bytes, read as unsigned.
+template <typename F> void WithKeys(const void *keys, size_t width, F &&f) {
+	switch (width) {
+	case 1: return f(static_cast<const uint8_t *>(keys));
+	case 2: return f(static_cast<const uint16_t *>(keys));
+	case 4: return f(static_cast<const uint32_t *>(keys));
+	case 8: return f(static_cast<const uint64_t *>(keys));
+	default: Fail(VGPU_ERR_INTERNAL, "join keys: width must be 1, 2, 4 or 8 bytes");
+	}
 }
 
-void JoinDenseInline(const uint64_t *keys, const void *values, size_t width, uint64_t n, uint64_t range,
-                     uint64_t *table, uint32_t *dups, cudaStream_t stream, uint64_t bias) {
-	LaunchScope scope("join_dense_table", stream, n * (8 + width) + (range + 1) * 8, n);
-	VGPU_CUDA(cudaMemsetAsync(table, 0, (range + 1) * 8, stream));
-	VGPU_CUDA(cudaMemsetAsync(dups, 0, 4, stream));
-	auto *t = reinterpret_cast<unsigned long long *>(table);
-	const unsigned grid = GridFor(n, 256);
+template <typename F> void WithValues(const void *values, size_t width, F &&f) {
 	switch (width) {
-	case 1:
-		JoinDenseInlineKernel<uint8_t><<<grid, 256, 0, stream>>>(keys, static_cast<const uint8_t *>(values), n, bias, t, dups);
-		break;
-	case 2:
-		JoinDenseInlineKernel<uint16_t><<<grid, 256, 0, stream>>>(keys, static_cast<const uint16_t *>(values), n, bias, t, dups);
-		break;
-	case 4:
-		JoinDenseInlineKernel<uint32_t><<<grid, 256, 0, stream>>>(keys, static_cast<const uint32_t *>(values), n, bias, t, dups);
-		break;
-	default:
-		Fail(VGPU_ERR_INTERNAL, "dense inline join table: value width must be 1, 2 or 4 bytes");
+	case 1: return f(static_cast<const uint8_t *>(values));
+	case 2: return f(static_cast<const uint16_t *>(values));
+	case 4: return f(static_cast<const uint32_t *>(values));
+	default: Fail(VGPU_ERR_INTERNAL, "join table: value width must be 1, 2 or 4 bytes");
+	}
+}
+
+template <typename E> void LaunchCount(const E *table, uint64_t entries, E empty, uint32_t *occupied, cudaStream_t stream) {
+	const unsigned grid = std::min<unsigned>(GridFor(entries * sizeof(E) / 16 + 1, 256), Runtime::Get().props().sm_count * 8);
+	JoinCountKernel<E><<<grid, 256, 0, stream>>>(table, entries, empty, occupied);
+}
+
+} // namespace
+
+void JoinDenseFill(const void *keys, size_t kwidth, const void *values, size_t vwidth, uint64_t n, uint64_t bias,
+                   uint64_t range, uint32_t vmin, void *table, size_t width, uint32_t *occupied, cudaStream_t stream) {
+	LaunchScope scope("join_dense_table", stream, n * (kwidth + vwidth) + (range + 1) * width, n);
+	// 8-byte entries and row numbers mark an empty key with 0, narrower values with all ones
+	const bool ones = values != nullptr && width != 8;
+	VGPU_CUDA(cudaMemsetAsync(table, ones ? 0xff : 0, (range + 1) * width, stream));
+	VGPU_CUDA(cudaMemsetAsync(occupied, 0, 4, stream));
+	const unsigned grid = GridFor((n + 3) / 4, 256);
+	WithKeys(keys, kwidth, [&](auto *k) {
+		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
+		if (!values) {
+			JoinFillRowsKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, bias, static_cast<uint32_t *>(table));
+			return;
+		}
+		WithValues(values, vwidth, [&](auto *v) {
+			using V = std::remove_const_t<std::remove_pointer_t<decltype(v)>>;
+			const uint64_t base = width == 8 ? 1ull << 32 : 0ull - vmin;
+			switch (width) {
+			case 1: JoinFillKernel<K, V, uint8_t><<<grid, 256, 0, stream>>>(k, v, n, bias, base, static_cast<uint8_t *>(table)); break;
+			case 2: JoinFillKernel<K, V, uint16_t><<<grid, 256, 0, stream>>>(k, v, n, bias, base, static_cast<uint16_t *>(table)); break;
+			case 4: JoinFillKernel<K, V, uint32_t><<<grid, 256, 0, stream>>>(k, v, n, bias, base, static_cast<uint32_t *>(table)); break;
+			case 8: JoinFillKernel<K, V, uint64_t><<<grid, 256, 0, stream>>>(k, v, n, bias, base, static_cast<uint64_t *>(table)); break;
+			default: Fail(VGPU_ERR_INTERNAL, "join table: entry width must be 1, 2, 4 or 8 bytes");
+			}
+		});
+	});
+	VGPU_CUDA(cudaGetLastError());
+	switch (width) {
+	case 1: LaunchCount<uint8_t>(static_cast<uint8_t *>(table), range + 1, 0xffu, occupied, stream); break;
+	case 2: LaunchCount<uint16_t>(static_cast<uint16_t *>(table), range + 1, 0xffffu, occupied, stream); break;
+	case 4: LaunchCount<uint32_t>(static_cast<uint32_t *>(table), range + 1, ones ? 0xffffffffu : 0u, occupied, stream); break;
+	default: LaunchCount<uint64_t>(static_cast<uint64_t *>(table), range + 1, 0ull, occupied, stream); break;
 	}
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void ValueBits(const void *values, size_t width, uint64_t n, uint32_t *bounds, cudaStream_t stream) {
-	VGPU_CUDA(cudaMemsetAsync(bounds, 0xff, 4, stream));
-	VGPU_CUDA(cudaMemsetAsync(bounds + 1, 0, 4, stream));
-	if (n == 0) return;
-	LaunchScope scope("value_bits", stream, n * width, n);
-	const unsigned grid = std::min<unsigned>(GridFor(n, 256), 1184);
-	switch (width) {
-	case 1: ValueBitsKernel<uint8_t><<<grid, 256, 0, stream>>>(static_cast<const uint8_t *>(values), n, bounds); break;
-	case 2: ValueBitsKernel<uint16_t><<<grid, 256, 0, stream>>>(static_cast<const uint16_t *>(values), n, bounds); break;
-	case 4: ValueBitsKernel<uint32_t><<<grid, 256, 0, stream>>>(static_cast<const uint32_t *>(values), n, bounds); break;
-	default: Fail(VGPU_ERR_INTERNAL, "value bits: width must be 1, 2 or 4 bytes");
+void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream) {
+	if (n <= 0) return;
+	VGPU_CUDA(cudaMemsetAsync(out, 0, static_cast<size_t>(n) * 16, stream));
+	for (int first = 0; first < n; first += kMaxBoundsColumns) {
+		BoundsArgs a;
+		const int count = std::min(n - first, kMaxBoundsColumns);
+		uint64_t bytes = 0, rows = 0, widest = 0;
+		for (int j = 0; j < count; j++) {
+			a.c[j] = cols[first + j];
+			const uint64_t b = a.c[j].rows * BoundsWidth(a.c[j].kind);
+			bytes += b;
+			rows += a.c[j].rows;
+			widest = std::max(widest, b);
+		}
+		if (widest == 0) continue;
+		a.out = reinterpret_cast<unsigned long long *>(out + 2 * first);
+		LaunchScope scope("column_bounds", stream, bytes, rows);
+		// four 16-byte loads per thread, at most eight CTAs per SM over all columns
+		const uint64_t cap = std::max<uint64_t>(1, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8 / count);
+		const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(cap, (widest + kBoundsBlock * 64 - 1) / (kBoundsBlock * 64)));
+		ColumnBoundsKernel<<<dim3(grid, static_cast<unsigned>(count)), kBoundsBlock, 0, stream>>>(a);
+		VGPU_CUDA(cudaGetLastError());
 	}
-	VGPU_CUDA(cudaGetLastError());
+}
+
+BoundsKind SignedBoundsKind(ValueType t) {
+	switch (t) {
+	case ValueType::INT16: return BoundsKind::I16;
+	case ValueType::INT32:
+	case ValueType::DICTIONARY_STRING: return BoundsKind::I32;
+	case ValueType::INT64: return BoundsKind::I64;
+	case ValueType::BOOLEAN: return BoundsKind::BOOL;
+	default: Fail(VGPU_ERR_INTERNAL, "min/max statistics need an integer column");
+	}
 }
 
 // Multi-match inline table: entry[k] = the key's match count in the low `cbits` bits, then one
@@ -787,13 +834,13 @@ void ValueBits(const void *values, size_t width, uint64_t n, uint32_t *bounds, c
 // A match reserves its slot by adding 1 to the count and then ORs its value into that slot; a key
 // with more than rmax matches (rmax < 2^cbits, so the count never wraps before it is seen) counts in
 // *overflow and the table is not valid.
-template <typename T, typename E>
-__global__ void JoinDenseMultiKernel(const uint64_t *keys, const T *values, uint64_t n, uint64_t bias, uint32_t vmin,
+template <typename K, typename T, typename E>
+__global__ void JoinDenseMultiKernel(const K *keys, const T *values, uint64_t n, uint64_t bias, uint32_t vmin,
                                      uint32_t vbits, uint32_t cbits, uint32_t rmax, E *table, uint32_t *overflow) {
 	const E cmask = (E(1) << cbits) - 1;
 	uint32_t local = 0;
 	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		E *slot = table + (keys[i] - bias);
+		E *slot = table + (static_cast<uint64_t>(keys[i]) - bias);
 		const E old = atomicAdd(slot, E(1));
 		const uint32_t j = static_cast<uint32_t>(old & cmask);
 		if (j >= rmax) {
@@ -806,79 +853,30 @@ __global__ void JoinDenseMultiKernel(const uint64_t *keys, const T *values, uint
 	if (local) atomicAdd(overflow, local);
 }
 
-namespace {
-template <typename E>
-void LaunchDenseCompact(const uint64_t *keys, const void *values, size_t vwidth, uint64_t n, uint64_t bias, uint32_t vmin,
-                        E *table, uint32_t *dups, cudaStream_t stream) {
-	const unsigned grid = GridFor(n, 256);
-	switch (vwidth) {
-	case 1:
-		JoinDenseCompactKernel<uint8_t, E><<<grid, 256, 0, stream>>>(keys, static_cast<const uint8_t *>(values), n, bias,
-		                                                             vmin, table, dups);
-		break;
-	case 2:
-		JoinDenseCompactKernel<uint16_t, E><<<grid, 256, 0, stream>>>(keys, static_cast<const uint16_t *>(values), n,
-		                                                              bias, vmin, table, dups);
-		break;
-	case 4:
-		JoinDenseCompactKernel<uint32_t, E><<<grid, 256, 0, stream>>>(keys, static_cast<const uint32_t *>(values), n,
-		                                                              bias, vmin, table, dups);
-		break;
-	default:
-		Fail(VGPU_ERR_INTERNAL, "compact join table: value width must be 1, 2 or 4 bytes");
-	}
-}
-} // namespace
-
-void JoinDenseCompact(const uint64_t *keys, const void *values, size_t vwidth, uint64_t n, uint64_t range,
-                      uint32_t vmin, void *table, size_t width, uint32_t *dups, cudaStream_t stream, uint64_t bias) {
-	LaunchScope scope("join_dense_table", stream, n * (8 + vwidth) + (range + 1) * width, n);
-	VGPU_CUDA(cudaMemsetAsync(table, 0xff, (range + 1) * width, stream));
-	VGPU_CUDA(cudaMemsetAsync(dups, 0, 4, stream));
-	switch (width) {
-	case 1: LaunchDenseCompact(keys, values, vwidth, n, bias, vmin, static_cast<uint8_t *>(table), dups, stream); break;
-	case 2: LaunchDenseCompact(keys, values, vwidth, n, bias, vmin, static_cast<uint16_t *>(table), dups, stream); break;
-	case 4: LaunchDenseCompact(keys, values, vwidth, n, bias, vmin, static_cast<uint32_t *>(table), dups, stream); break;
-	default: Fail(VGPU_ERR_INTERNAL, "compact join table: width must be 1, 2 or 4 bytes");
-	}
-	VGPU_CUDA(cudaGetLastError());
-}
-
-void JoinDenseMulti(const uint64_t *keys, const void *values, size_t vwidth, uint64_t n, uint64_t range, uint32_t vmin,
-                    uint32_t vbits, uint32_t cbits, uint32_t rmax, void *table, bool wide, uint32_t *overflow,
-                    cudaStream_t stream, uint64_t bias) {
+void JoinDenseMulti(const void *keys, size_t kwidth, const void *values, size_t vwidth, uint64_t n, uint64_t bias,
+                    uint64_t range, uint32_t vmin, uint32_t vbits, uint32_t cbits, uint32_t rmax, void *table, bool wide,
+                    uint32_t *overflow, cudaStream_t stream) {
 	const size_t ew = wide ? 8 : 4;
 	if (cbits < 1 || cbits > 3 || rmax >= (1u << cbits) || cbits + rmax * vbits > ew * 8) {
 		Fail(VGPU_ERR_INTERNAL, "multi-match join table: slots do not fit the entry");
 	}
-	LaunchScope scope("join_dense_multi", stream, n * (8 + vwidth) + (range + 1) * ew, n);
+	LaunchScope scope("join_dense_multi", stream, n * (kwidth + vwidth) + (range + 1) * ew, n);
 	VGPU_CUDA(cudaMemsetAsync(table, 0, (range + 1) * ew, stream));
 	VGPU_CUDA(cudaMemsetAsync(overflow, 0, 4, stream));
 	const unsigned grid = GridFor(n, 256);
-	auto launch = [&](auto *tab) {
-		using E = std::remove_pointer_t<decltype(tab)>;
-		switch (vwidth) {
-		case 1:
-			JoinDenseMultiKernel<uint8_t, E><<<grid, 256, 0, stream>>>(keys, static_cast<const uint8_t *>(values), n, bias,
-			                                                           vmin, vbits, cbits, rmax, tab, overflow);
-			break;
-		case 2:
-			JoinDenseMultiKernel<uint16_t, E><<<grid, 256, 0, stream>>>(keys, static_cast<const uint16_t *>(values), n,
-			                                                            bias, vmin, vbits, cbits, rmax, tab, overflow);
-			break;
-		case 4:
-			JoinDenseMultiKernel<uint32_t, E><<<grid, 256, 0, stream>>>(keys, static_cast<const uint32_t *>(values), n,
-			                                                            bias, vmin, vbits, cbits, rmax, tab, overflow);
-			break;
-		default:
-			Fail(VGPU_ERR_INTERNAL, "multi-match join table: value width must be 1, 2 or 4 bytes");
-		}
-	};
-	if (wide) {
-		launch(static_cast<unsigned long long *>(table));
-	} else {
-		launch(static_cast<unsigned int *>(table));
-	}
+	WithKeys(keys, kwidth, [&](auto *k) {
+		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
+		WithValues(values, vwidth, [&](auto *v) {
+			using V = std::remove_const_t<std::remove_pointer_t<decltype(v)>>;
+			if (wide) {
+				JoinDenseMultiKernel<K, V, unsigned long long><<<grid, 256, 0, stream>>>(
+				    k, v, n, bias, vmin, vbits, cbits, rmax, static_cast<unsigned long long *>(table), overflow);
+			} else {
+				JoinDenseMultiKernel<K, V, unsigned int><<<grid, 256, 0, stream>>>(
+				    k, v, n, bias, vmin, vbits, cbits, rmax, static_cast<unsigned int *>(table), overflow);
+			}
+		});
+	});
 	VGPU_CUDA(cudaGetLastError());
 }
 
@@ -1084,103 +1082,38 @@ void Gather(const void *src, size_t width, const uint32_t *idx, uint64_t n, void
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void WidenKeys(const void *src, size_t width, uint64_t n, uint64_t *dst, cudaStream_t stream) {
+void WidenKeys(const void *src, size_t width, uint64_t n, uint64_t bias, uint64_t *dst, cudaStream_t stream) {
 	if (n == 0) return;
 	LaunchScope scope("widen_keys", stream, n * (width + 8), n);
-	const unsigned grid = GridFor(n, 256);
-	switch (width) {
-	case 1:
-		WidenKernel<uint8_t><<<grid, 256, 0, stream>>>(static_cast<const uint8_t *>(src), n, dst);
-		break;
-	case 2:
-		WidenKernel<uint16_t><<<grid, 256, 0, stream>>>(static_cast<const uint16_t *>(src), n, dst);
-		break;
-	case 4:
-		WidenKernel<uint32_t><<<grid, 256, 0, stream>>>(static_cast<const uint32_t *>(src), n, dst);
-		break;
-	case 8:
-		WidenKernel<uint64_t><<<grid, 256, 0, stream>>>(static_cast<const uint64_t *>(src), n, dst);
-		break;
-	default:
-		Fail(VGPU_ERR_INTERNAL, "widen: unsupported width");
-	}
+	WithKeys(src, width, [&](auto *k) {
+		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
+		WidenKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, bias, dst);
+	});
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void MinMaxU64(const uint64_t *keys, uint64_t n, uint64_t *minmax, cudaStream_t stream) {
-	LaunchScope scope("minmax", stream, n * 8, n);
-	InitMinMaxKernel<<<1, 1, 0, stream>>>(minmax);
-	if (n > 0) {
-		const unsigned grid = std::min<unsigned>(GridFor(n, 256), Runtime::Get().props().sm_count * 8);
-		MinMaxKernel<<<grid, 256, 0, stream>>>(keys, n, minmax);
-	}
-	VGPU_CUDA(cudaGetLastError());
-}
-
-void WidenKeysMinMax(const void *src, size_t width, uint64_t n, uint64_t *dst, uint64_t *minmax, cudaStream_t stream) {
-	InitMinMaxKernel<<<1, 1, 0, stream>>>(minmax);
-	if (n == 0) {
-		VGPU_CUDA(cudaGetLastError());
-		return;
-	}
-	LaunchScope scope("widen_keys", stream, n * (width + 8), n);
-	const unsigned grid = std::min<unsigned>(GridFor(n, 256), Runtime::Get().props().sm_count * 8);
-	switch (width) {
-	case 1:
-		WidenMinMaxKernel<uint8_t><<<grid, 256, 0, stream>>>(static_cast<const uint8_t *>(src), n, dst, minmax);
-		break;
-	case 2:
-		WidenMinMaxKernel<uint16_t><<<grid, 256, 0, stream>>>(static_cast<const uint16_t *>(src), n, dst, minmax);
-		break;
-	case 4:
-		WidenMinMaxKernel<uint32_t><<<grid, 256, 0, stream>>>(static_cast<const uint32_t *>(src), n, dst, minmax);
-		break;
-	case 8:
-		WidenMinMaxKernel<uint64_t><<<grid, 256, 0, stream>>>(static_cast<const uint64_t *>(src), n, dst, minmax);
-		break;
-	default:
-		Fail(VGPU_ERR_INTERNAL, "widen: unsupported width");
-	}
-	VGPU_CUDA(cudaGetLastError());
-}
-
-void MinMaxSigned(const void *data, int type, uint64_t n, int64_t *out, cudaStream_t stream) {
-	LaunchScope scope("minmax_signed", stream, n * 8, n);
-	InitMinMaxSignedKernel<<<1, 1, 0, stream>>>(out);
-	if (n > 0) {
-		const unsigned grid = GridFor(n, 256);
-		switch (static_cast<ValueType>(type)) {
-		case ValueType::INT16:
-			MinMaxSignedKernel<int16_t><<<grid, 256, 0, stream>>>(static_cast<const int16_t *>(data), n, out);
-			break;
-		case ValueType::INT32:
-		case ValueType::DICTIONARY_STRING:
-			MinMaxSignedKernel<int32_t><<<grid, 256, 0, stream>>>(static_cast<const int32_t *>(data), n, out);
-			break;
-		case ValueType::INT64:
-			MinMaxSignedKernel<int64_t><<<grid, 256, 0, stream>>>(static_cast<const int64_t *>(data), n, out);
-			break;
-		case ValueType::BOOLEAN:
-			MinMaxSignedKernel<uint8_t><<<grid, 256, 0, stream>>>(static_cast<const uint8_t *>(data), n, out);
-			break;
-		default:
-			Fail(VGPU_ERR_INTERNAL, "min/max statistics need an integer column");
-		}
-	}
+void Iota(uint32_t *out, uint64_t n, cudaStream_t stream) {
+	if (n == 0) return;
+	LaunchScope scope("iota", stream, n * 4, n);
+	IotaKernel<<<GridFor(n, 256), 256, 0, stream>>>(out, n);
 	VGPU_CUDA(cudaGetLastError());
 }
 
 void RadixSortPairs(uint64_t *keys, uint32_t *values, uint64_t *keys_alt, uint32_t *values_alt, uint64_t n, int bits,
                     Arena &arena) {
-	if (n <= 1 || bits <= 0) return;
 	cudaStream_t s = arena.stream();
+	if (n <= 1 || bits <= 0) {
+		Iota(values, n, s);
+		return;
+	}
 	const uint64_t ntiles64 = (n + kSortTile - 1) / kSortTile;
 	if (ntiles64 > 0xffffffffull) Fail(VGPU_ERR_UNSUPPORTED, "radix sort: too many rows");
 	const uint32_t ntiles = static_cast<uint32_t>(ntiles64);
 	uint32_t *hist = arena.AllocT<uint32_t>(static_cast<size_t>(ntiles) * 256);
 	uint32_t *total = arena.AllocT<uint32_t>(1);
 	uint64_t *kin = keys, *kout = keys_alt;
-	uint32_t *vin = values, *vout = values_alt;
+	const uint32_t *vin = nullptr;  // the first pass takes each key's position
+	uint32_t *vout = values_alt, *vspare = values;
 	const int passes = (bits + 7) / 8;
 	for (int p = 0; p < passes; p++) {
 		const int shift = 8 * p;
@@ -1195,26 +1128,13 @@ void RadixSortPairs(uint64_t *keys, uint32_t *values, uint64_t *keys_alt, uint32
 		}
 		VGPU_CUDA(cudaGetLastError());
 		std::swap(kin, kout);
-		std::swap(vin, vout);
+		vin = vout;
+		std::swap(vout, vspare);
 	}
 	if (kin != keys) {
 		VGPU_CUDA(cudaMemcpyAsync(keys, kin, n * 8, cudaMemcpyDeviceToDevice, s));
 		VGPU_CUDA(cudaMemcpyAsync(values, vin, n * 4, cudaMemcpyDeviceToDevice, s));
 	}
-}
-
-void SubtractBias(uint64_t *keys, uint64_t n, uint64_t bias, cudaStream_t stream) {
-	if (n == 0 || bias == 0) return;
-	LaunchScope scope("subtract_bias", stream, n * 16, n);
-	SubtractBiasKernel<<<GridFor(n, 256), 256, 0, stream>>>(keys, n, bias);
-	VGPU_CUDA(cudaGetLastError());
-}
-
-void Iota(uint32_t *out, uint64_t n, cudaStream_t stream) {
-	if (n == 0) return;
-	LaunchScope scope("iota", stream, n * 4, n);
-	IotaKernel<<<GridFor(n, 256), 256, 0, stream>>>(out, n);
-	VGPU_CUDA(cudaGetLastError());
 }
 
 void JoinExpand(const uint64_t *offsets, const uint64_t *lower, uint64_t n_left, const uint32_t *sorted_perm,

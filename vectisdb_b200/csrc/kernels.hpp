@@ -30,22 +30,47 @@ void PackValidity(const uint8_t *bytes, uint8_t *bitmap, uint64_t n, cudaStream_
 void Gather(const void *src, size_t width, const uint32_t *idx, uint64_t n, void *dst, cudaStream_t stream);
 
 //! Raw key bits zero-extended to 64 bits (the reference's WidenKeyKernel semantics,
-//! cuda_engine/src/operators/gpu_groupby.cu:76-94), plus the range of the widened values.
-void WidenKeys(const void *src, size_t width, uint64_t n, uint64_t *dst, cudaStream_t stream);
-void MinMaxU64(const uint64_t *keys, uint64_t n, uint64_t *minmax /* device [2] */, cudaStream_t stream);
-//! WidenKeys and MinMaxU64 of the widened keys in one pass.
-void WidenKeysMinMax(const void *src, size_t width, uint64_t n, uint64_t *dst, uint64_t *minmax, cudaStream_t stream);
+//! cuda_engine/src/operators/gpu_groupby.cu:76-94), minus `bias`.
+void WidenKeys(const void *src, size_t width, uint64_t n, uint64_t bias, uint64_t *dst, cudaStream_t stream);
 
-//! Signed range of an integer/boolean column: out[0] = min, out[1] = max (device i64[2]).
-void MinMaxSigned(const void *data, int type /* ValueType */, uint64_t n, int64_t *out, cudaStream_t stream);
+//! How a column's values are read for ColumnBounds (BOOL: one byte, zero or not).
+enum class BoundsKind : int { U8, U16, U32, U64, I16, I32, I64, BOOL };
+constexpr int kMaxBoundsColumns = 8;
+struct BoundsColumn {
+	const void *data;
+	uint64_t rows;
+	BoundsKind kind;
+};
+inline size_t BoundsWidth(BoundsKind k) {
+	return k == BoundsKind::U8 || k == BoundsKind::BOOL ? 1 : k == BoundsKind::U16 || k == BoundsKind::I16 ? 2
+	       : k == BoundsKind::U32 || k == BoundsKind::I32 ? 4 : 8;
+}
+//! The unsigned kind of a `width`-byte column's raw bits, zero-extended.
+inline BoundsKind RawBoundsKind(size_t width) {
+	return width == 1 ? BoundsKind::U8 : width == 2 ? BoundsKind::U16 : width == 4 ? BoundsKind::U32 : BoundsKind::U64;
+}
+//! The kind of an integer, boolean or dictionary column's values.
+BoundsKind SignedBoundsKind(ValueType t);
+//! Smallest and largest value of each of `n` columns, one launch per kMaxBoundsColumns of them: two words
+//! per column in `out` (device, 2n words), read back with BoundsLow / BoundsHigh. A column without rows
+//! gives the largest value of its 64-bit kind as the smallest and the other way round.
+void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream);
+inline bool BoundsSigned(BoundsKind k) {
+	return k == BoundsKind::I16 || k == BoundsKind::I32 || k == BoundsKind::I64;
+}
+//! The column's bounds as the 64-bit pattern of its value (two's complement for the signed kinds).
+inline uint64_t BoundsLow(const uint64_t *words, BoundsKind k) {
+	return ~words[0] ^ (BoundsSigned(k) ? 1ull << 63 : 0ull);
+}
+inline uint64_t BoundsHigh(const uint64_t *words, BoundsKind k) {
+	return words[1] ^ (BoundsSigned(k) ? 1ull << 63 : 0ull);
+}
 
-//! Stable LSD radix sort of (key, value) pairs over the low `bits` bits of the keys (8-bit digits).
-//! Results end in (keys, values); (keys_alt, values_alt) are the ping-pong buffers.
+//! Stable LSD radix sort of keys over their low `bits` bits (8-bit digits), `values` becoming the sorted
+//! keys' positions in the input. Results end in (keys, values); (keys_alt, values_alt) are the ping-pong buffers.
 void RadixSortPairs(uint64_t *keys, uint32_t *values, uint64_t *keys_alt, uint32_t *values_alt, uint64_t n, int bits,
                     Arena &arena);
 
-//! keys[i] -= bias (normalizes a key range to start at zero before sorting).
-void SubtractBias(uint64_t *keys, uint64_t n, uint64_t bias, cudaStream_t stream);
 void Iota(uint32_t *out, uint64_t n, cudaStream_t stream);
 
 //! Left row i owns outputs [offsets[i], offsets[i + 1]) (offsets ascending, offsets[0] = 0): output o
@@ -61,29 +86,22 @@ void JoinRuns(const uint64_t *probe, uint64_t n_probe, const uint64_t *sorted, c
 //! Radix directory of a sorted (biased) key array: dir[b] = first position whose key >> shift >= b,
 //! for b in [0, nb]; dir needs nb + 1 entries and nb must exceed every key >> shift.
 void JoinDirectory(const uint64_t *sorted, uint64_t n, uint32_t shift, uint64_t nb, uint32_t *dir, cudaStream_t stream);
-//! Dense join tables over keys - bias all <= range (`bias`: the keys' minimum, subtracted on the fly;
-//! 0 for keys already biased), range + 1 entries, built without sorting:
-//! table[k] = row index + 1 of key k (0 = none), or (1 << 32 | value) with a <= 4-byte value of that
-//! row inlined. *dups = keys met more than once (then the table is not a valid lookup).
-void JoinDenseRows(const uint64_t *keys, uint64_t n, uint64_t range, uint32_t *table, uint32_t *dups,
-                   cudaStream_t stream, uint64_t bias = 0);
-void JoinDenseInline(const uint64_t *keys, const void *values, size_t width, uint64_t n, uint64_t range,
-                     uint64_t *table, uint32_t *dups, cudaStream_t stream, uint64_t bias = 0);
-//! Smallest and largest raw bits (zero-extended to 32) of a 1-, 2- or 4-byte column: bounds[0], bounds[1].
-void ValueBits(const void *values, size_t width, uint64_t n, uint32_t *bounds, cudaStream_t stream);
-//! The inline table in `width` (1, 2 or 4) bytes per key: table[k] = value bits - vmin, all ones = no
-//! key (every value's offset must stay below that marker). *dups = keys met more than once.
-void JoinDenseCompact(const uint64_t *keys, const void *values, size_t vwidth, uint64_t n, uint64_t range,
-                      uint32_t vmin, void *table, size_t width, uint32_t *dups, cudaStream_t stream,
-                      uint64_t bias = 0);
-//! Dense multi-match table over (biased) keys <= range, built without sorting, for a join that contributes
+//! Dense join table over the raw keys (`kwidth` bytes, zero-extended) minus `bias` (their minimum), all <=
+//! `range`: range + 1 entries of `width` bytes, built without sorting. Without values (width 4): row index
+//! + 1 of the key's row, 0 = no key. With a 1-, 2- or 4-byte value column: width 8 holds (1 << 32 | value
+//! bits), 0 = no key; width 1, 2 or 4 holds value bits - vmin, all ones = no key (every value's offset must
+//! stay below that marker). *occupied = entries written: below n when a key repeats, and the table is then
+//! not a valid lookup.
+void JoinDenseFill(const void *keys, size_t kwidth, const void *values, size_t vwidth, uint64_t n, uint64_t bias,
+                   uint64_t range, uint32_t vmin, void *table, size_t width, uint32_t *occupied, cudaStream_t stream);
+//! Dense multi-match table over the same keys, built without sorting, for a join that contributes
 //! one right column of at most 4 bytes: entry[k] (4 bytes, or 8 when `wide`) holds k's match count in its
 //! low `cbits` bits (1..3) and one `vbits`-bit slot per match above them, each the value bits - vmin. A key
 //! with more than `rmax` matches (rmax < 2^cbits, cbits + rmax * vbits within the entry) counts in
 //! *overflow, and the table is then not valid.
-void JoinDenseMulti(const uint64_t *keys, const void *values, size_t vwidth, uint64_t n, uint64_t range, uint32_t vmin,
-                    uint32_t vbits, uint32_t cbits, uint32_t rmax, void *table, bool wide, uint32_t *overflow,
-                    cudaStream_t stream, uint64_t bias = 0);
+void JoinDenseMulti(const void *keys, size_t kwidth, const void *values, size_t vwidth, uint64_t n, uint64_t bias,
+                    uint64_t range, uint32_t vmin, uint32_t vbits, uint32_t cbits, uint32_t rmax, void *table, bool wide,
+                    uint32_t *overflow, cudaStream_t stream);
 //! *out = number of positions i > 0 with sorted[i] == sorted[i - 1].
 void CountAdjacentEqual(const uint64_t *sorted, uint64_t n, uint32_t *out, cudaStream_t stream);
 //! *out = the length of the longest run of equal keys in `sorted` (saturating at 2^32 - 1).
