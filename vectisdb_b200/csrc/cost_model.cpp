@@ -43,7 +43,19 @@ struct Walker {
 	const std::vector<uint32_t> *scan_widths;
 	const std::vector<bool> *scan_resident;
 	size_t scan_index = 0;
+	bool from_cache = false;  // scans are served from the column cache, which knows their columns' ranges
 	vgpu_working_set ws {};
+
+	// A right side whose cached key is dense enough for a table indexed by the key.
+	bool DenseRightKey(const PlanNode &join) const {
+		if (!from_cache || join.children.size() != 2 || join.children[1]->op != OpType::SCAN || join.probe_keys.size() != 1) {
+			return false;
+		}
+		DevColumn c;
+		if (!ColumnCache::Get().GetWhole(join.children[1]->table, join.probe_keys[0], c) || !c.has_stats) return false;
+		const uint64_t range = static_cast<uint64_t>(c.max) - static_cast<uint64_t>(c.min);
+		return range < (1ull << 28) && range < 4 * c.rows;
+	}
 
 	void Charge(const char *op, uint64_t bytes) {
 		ws.total_bytes = SatAdd(ws.total_bytes, bytes);
@@ -135,9 +147,9 @@ struct Walker {
 			const uint64_t out_width = 8 * std::max<size_t>(1, n.output_columns.size());
 			uint64_t bytes;
 			if (!materialize) {
-				// the join as a pipeline source: right keys widened, their range, a dense table (at most
-				// 8 bytes per key of the range) or sorted keys with a radix directory
-				bytes = SatMul(r.rows, 32);
+				// the join as a pipeline source: a dense table (1 to 8 bytes per key of the range, which is under
+				// four times the rows), or widened keys, sorted with their positions, and a radix directory
+				bytes = SatMul(r.rows, DenseRightKey(n) ? 8 : 32);
 				e.rows = n.estimated_rows ? Capped(n.estimated_rows) : l.rows;
 			} else {
 				// materializing: both sides' keys widened, the right side sorted with a permutation and
@@ -170,8 +182,9 @@ struct Walker {
 vgpu_working_set EstimateWorkingSet(const PlanNode &plan, uint64_t max_chunk_rows,
                                     const std::vector<uint64_t> *scan_rows,
                                     const std::vector<uint32_t> *scan_widths,
-                                    const std::vector<bool> *scan_resident) {
+                                    const std::vector<bool> *scan_resident, bool from_cache) {
 	Walker w;
+	w.from_cache = from_cache;
 	w.cap = IsRowIndependent(plan) ? max_chunk_rows : 0;
 	w.scan_rows = scan_rows;
 	w.scan_widths = scan_widths;
@@ -211,7 +224,7 @@ vgpu_working_set EstimateWorkingSetFor(const PlanNode &plan, const std::vector<v
 		widths.push_back(w);
 		resident.push_back(res);
 	}
-	return EstimateWorkingSet(plan, 0, &rows, &widths, &resident);
+	return EstimateWorkingSet(plan, 0, &rows, &widths, &resident, serve_from_cache);
 }
 
 namespace {

@@ -18,7 +18,7 @@ namespace vgpu {
 vgpu_working_set EstimateWorkingSet(const PlanNode &plan, uint64_t max_chunk_rows,
                                     const std::vector<uint64_t> *scan_rows = nullptr,
                                     const std::vector<uint32_t> *scan_widths = nullptr,
-                                    const std::vector<bool> *scan_resident = nullptr);
+                                    const std::vector<bool> *scan_resident = nullptr, bool from_cache = false);
 
 //! The estimate for one execution with its actual inputs and options: rows and widths from the
 //! inputs (or the cached columns a cache-served scan reads), SCANs over cache-served or device-memory
