@@ -255,7 +255,8 @@ def algorithmic_bytes(name: str, wl, kernel: str, passing: int, groups: int) -> 
     if name == "c0":
         return {"vgpu_gb_direct": 20 * n}.get(kernel, 0)
     if name == "cp":  # the count pass reads the predicate columns, the write pass all three + the output
-        return {"vgpu_mat_count": 16 * n, "vgpu_mat_write": 20 * n + 20 * passing}.get(kernel, 0)
+        return {"vgpu_mat_count": 16 * n, "vgpu_mat_write": 20 * n + 20 * passing,
+                "vgpu_mat_onepass": 20 * n + 20 * passing}.get(kernel, 0)
     if name in ("c2", "c2dup"):
         build = wl.params["build_n"]
         return {"vgpu_gb_direct": 16 * n, "join_dense_table": 12 * build}.get(kernel, 0)

@@ -563,6 +563,10 @@ void ResolveRows(const vgpu_result *result) {
 	} else {
 		std::memcpy(&rows, word.get(), sizeof(rows));
 	}
+	for (auto &c : r->exec.columns) {
+		// the columns were sized for the most rows there could be; more marks a pass that gave up waiting
+		if (rows > c.rows) Fail(VGPU_ERR_CUDA, "the result's rows were not completed on the device");
+	}
 	for (auto &c : r->exec.columns) c.rows = rows;
 	r->exec.pending_rows = nullptr;  // its buffer is freed with the result
 }

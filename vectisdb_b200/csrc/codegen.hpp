@@ -104,6 +104,10 @@ public:
 	//! then per output column c: data @+1+2c, byte-validity @+2+2c). Without a filter only
 	//! vgpu_mat_write exists and writes row-aligned.
 	std::string EmitMaterialize(const std::vector<int> &out_columns, const Geometry &g) const;
+	//! The form that reads its inputs once (a row filter, no multi-match join): kernel vgpu_mat_onepass, with
+	//! 2 * tile rows * OnePassRowBytes of dynamic shared memory.
+	std::string EmitMaterializeOnePass(const std::vector<int> &out_columns, const Geometry &g) const;
+	uint64_t OnePassRowBytes(const std::vector<int> &out_columns) const;
 
 	//! vgpu_stats: per column c, atomic min/max of the (integer) value over every row < n into
 	//! i64 mins @+2c and maxs @+2c+1 (pointers to device i64). Ignores predicates (a superset bound).
@@ -209,7 +213,8 @@ private:
 	void Resolve();
 	std::string EmitExpression(const Expr &expr, const std::vector<PipeColumn> &cols, int index);
 	std::string Prologue() const;
-	std::string LoadBlock(const Geometry &g, const std::vector<bool> &needed, bool chunked) const;
+	std::string LoadDecls(const Geometry &g, const std::vector<bool> &needed) const;
+	std::string LoadBlock(const Geometry &g, const std::vector<bool> &needed, bool declare = true) const;
 	//! Opens the per-item loop of a tile: `row`, `keep` and (for a multi-match join source) the loop over
 	//! the row's matches with the needed right columns loaded at each; ItemClose closes what it opened.
 	std::string ItemOpen(const Geometry &g, const std::vector<bool> &needed) const;

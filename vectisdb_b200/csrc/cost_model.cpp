@@ -407,7 +407,9 @@ std::string GenerateSourceText(const PlanNode &plan, const std::vector<vgpu_colu
 	if (!gb) {
 		std::vector<int> outs;
 		for (size_t i = 0; i < cg.visible().size(); i++) outs.push_back(static_cast<int>(i));
-		return cg.EmitMaterialize(outs, g);
+		std::string text = cg.EmitMaterialize(outs, g);
+		if (cg.has_filter()) text += "\n//@@VGPU_TU@@\n" + cg.EmitMaterializeOnePass(outs, g);
+		return text;
 	}
 	PipelineCodegen::GroupBySpec spec_gb;
 	int shift = 0;

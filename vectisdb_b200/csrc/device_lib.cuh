@@ -256,6 +256,17 @@ __device__ __forceinline__ void load_valid(const u8 *__restrict__ base, u64 row0
 		for (int r = 0; r < R; ++r) out[r] = true;
 		return;
 	}
+	if constexpr (R % 4 == 0) {
+		if (row0 + R <= n && ((u64)(base + row0) & 3ull) == 0) {
+#pragma unroll
+			for (int q = 0; q < R / 4; ++q) {
+				const u32 w = ld_stream_u32(base + row0 + 4 * q);
+#pragma unroll
+				for (int r = 0; r < 4; ++r) out[4 * q + r] = ((w >> (8 * r)) & 0xffu) != 0;
+			}
+			return;
+		}
+	}
 #pragma unroll
 	for (int r = 0; r < R; ++r) out[r] = (row0 + r < n) ? (base[row0 + r] != 0) : false;
 }
@@ -292,6 +303,95 @@ __device__ __forceinline__ u32 block_exclusive_scan(u32 v, u32 *scratch, u32 *to
 	*total = scratch[32];
 	__syncthreads();
 	return result;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Starts of consecutive tiles in one launch: every tile publishes its row count, one CTA turns the counts
+// into starts in tile order, and a tile waits for its own start only. (Each tile adding up the tiles before
+// it instead, with look-back, keeps a thousand warps polling the same few sectors: a filter + projection of
+// 2^24 rows took 0.29 ms with 32 states per look and 0.97 ms with 256, against 0.10 ms this way.) CTAs take work from a counter whose first ticket is the scanning
+// CTA, so when a tile waits, the scanner and every tile before it are running or done.
+// counts[t] = rows of tile t + 1, starts[t] = start of tile t + 1; both zero at launch. A word carries all
+// that its reader needs, so relaxed accesses suffice.
+
+__device__ __forceinline__ u64 ld_relaxed(const u64 *p) {
+	u64 v;
+	asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ u32 ld_relaxed(const u32 *p) {
+	u32 v;
+	asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ void st_relaxed(u64 *p, u64 v) {
+	asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed(u32 *p, u32 v) {
+	asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// A bounded wait's clock: true once about two seconds (or 2^26 polls) have passed since the first call.
+struct PollLimit {
+	u32 polls = 0;
+	u64 t0 = 0;
+	__device__ __forceinline__ bool Expired() {
+		if ((++polls & 255u) != 0) return false;
+		const u64 now = global_ns();
+		if (t0 == 0) t0 = now;
+		return now - t0 > 2000000000ull || polls >= (1u << 26);
+	}
+};
+
+// One thread: the start of a tile, or ~0 when the wait ran out.
+__device__ __forceinline__ u64 tile_wait(const u64 *start) {
+	PollLimit limit;
+	for (;;) {
+		const u64 v = ld_relaxed(start);
+		if (v != 0) return v - 1;
+		if (limit.Expired()) return ~0ull;
+	}
+}
+
+// The scanning CTA (blockDim.x a multiple of 32; `scratch` 33 words and `bound` one word of shared memory):
+// up to four tiles per thread and step, as far as their counts are published without a gap. Returns the
+// total, or ~0 when the tiles stopped making progress.
+__device__ __forceinline__ u64 tile_scanner(const u32 *counts, u64 *starts, u64 ntiles, u32 *scratch, u32 *bound) {
+	constexpr u32 kEach = 4;
+	u64 carry = 0, first = 0;
+	PollLimit limit;
+	while (first < ntiles) {
+		u32 c[kEach];
+		u32 ready = 0;  // leading published counts of this thread's tiles
+		const u64 mine = first + (u64)threadIdx.x * kEach;
+#pragma unroll
+		for (u32 i = 0; i < kEach; ++i) c[i] = mine + i < ntiles ? ld_relaxed(counts + mine + i) : 0u;
+#pragma unroll
+		for (u32 i = 0; i < kEach; ++i) ready += ready == i && c[i] != 0 ? 1u : 0u;
+		if (threadIdx.x == 0) *bound = kEach * blockDim.x;
+		__syncthreads();
+		if (ready < kEach) atomicMin(bound, threadIdx.x * kEach + ready);
+		__syncthreads();
+		const u32 n = *bound;  // tiles first .. first + n - 1 are published
+		u32 sum = 0;
+#pragma unroll
+		for (u32 i = 0; i < kEach; ++i) {
+			c[i] = threadIdx.x * kEach + i < n ? c[i] - 1u : 0u;
+			sum += c[i];
+		}
+		u32 total;
+		u64 run = carry + block_exclusive_scan(sum, scratch, &total);
+#pragma unroll
+		for (u32 i = 0; i < kEach; ++i) {
+			if (threadIdx.x * kEach + i < n) st_relaxed(starts + mine + i, run + 1);
+			run += c[i];
+		}
+		carry += total;
+		first += n;
+		if (n != 0) limit = PollLimit();
+		if (__syncthreads_or(n == 0 && limit.Expired())) return ~0ull;
+	}
+	return carry;
 }
 
 // ---------------------------------------------------------------------------------------------

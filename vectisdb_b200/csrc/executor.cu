@@ -526,23 +526,97 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
                                const std::vector<std::string> &names, bool at_root) {
 	auto cgp = CodegenFor(pin.spec);
 	const PipelineCodegen &cg = *cgp;
+	const uint64_t n = pin.rows;
+	const uint64_t row_bytes = cg.OnePassRowBytes(out_cols);
+	bool null_outs = false;
+	for (int c : out_cols) null_outs = null_outs || cg.visible()[c].nullable;
+	// One pass or two. One pass needs room for a row per input row before it knows how many are kept: taken
+	// while that is at most 8 GiB and within the budget, and unless the plan's own estimate says that under
+	// two rows in five survive (what the admission estimate charges for the outputs then stays near what
+	// they take). Its two staged tiles of 512 rows allow 96 bytes a row (96 KB a CTA, two CTAs per SM).
+	// VGPU_MAT_PASSES=2: always two (testing).
+	bool one_pass = cg.has_filter() && n > 0 && !pin.spec.join_multi && row_bytes > 0 && row_bytes <= 96 &&
+	                n <= (8ull << 30) / row_bytes &&
+	                Runtime::Get().allocator().HasHeadroom(n * row_bytes);
+	for (const PlanNode *node : pin.spec.chain) {
+		if (node->op == OpType::FILTER && node->estimated_rows && 5 * node->estimated_rows < 2 * n) one_pass = false;
+	}
+	if (const char *env = std::getenv("VGPU_MAT_PASSES")) one_pass = one_pass && std::strcmp(env, "2") != 0;
 	Geometry g;
 	g.block = 256;
 	g.items = 4;
+	if (one_pass) g.block = 128;
+	const size_t smem = one_pass ? static_cast<size_t>(2 * g.tile() * row_bytes) : 0;
 	std::string mkey = "mat|" + SpecKey(pin.spec) + "|outs:";
 	for (int c : out_cols) mkey += std::to_string(c) + ",";
-	mkey += "|g:" + std::to_string(g.block) + "x" + std::to_string(g.items);
-	auto module = Runtime::Get().modules().GetOrCompileMemo(mkey, [&] { return cg.EmitMaterialize(out_cols, g); });
-	const uint64_t n = pin.rows;
+	mkey += "|g:" + std::to_string(g.block) + "x" + std::to_string(g.items) + (one_pass ? "o" : "");
+	auto module = Runtime::Get().modules().GetOrCompileMemo(mkey, [&] {
+		return one_pass ? cg.EmitMaterializeOnePass(out_cols, g) : cg.EmitMaterialize(out_cols, g);
+	});
 	const uint64_t ntiles = (n + g.tile() - 1) / g.tile();
 	const int sms = Runtime::Get().props().sm_count;
 	const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(sms) * 8)));
 	const int cb = cg.ConsumerBase();
 	uint64_t out_rows = n;
 	void *tile_offsets = nullptr;
+	uint64_t in_bytes = 0;
+	for (auto &s : pin.sources) in_bytes += s.rows * TypeSize(s.type);
+	Relation out;
+	auto add_columns = [&](KArgsHost &a, uint64_t rows) {
+		for (size_t c = 0; c < out_cols.size(); c++) {
+			const auto &vc = cg.visible()[out_cols[c]];
+			DevColumn col;
+			col.name = names[c];
+			col.type = vc.type;
+			col.rows = rows;
+			col.data = arena_.Alloc(rows * TypeSize(vc.type));
+			if (vc.nullable) {
+				col.valid = arena_.AllocT<uint8_t>(rows);
+			}
+			if (vc.source >= 0 && pin.sources[vc.source].has_stats) {
+				col.has_stats = true;
+				col.min = pin.sources[vc.source].min;
+				col.max = pin.sources[vc.source].max;
+			}
+			a.SetPtr(cb + 1 + 2 * static_cast<int>(c), col.data);
+			a.SetPtr(cb + 2 + 2 * static_cast<int>(c), col.valid);
+			out.push_back(col);
+		}
+	};
+	if (one_pass) {
+		const uint64_t words = 2 + (ntiles + 1) / 2 + ntiles;  // total, ticket, tile counts, tile starts
+		uint64_t *chain = arena_.AllocT<uint64_t>(words);
+		VGPU_CUDA(cudaMemsetAsync(chain, 0, words * 8, stream_));
+		KArgsHost a;
+		FillArgs(pin, a);
+		a.SetPtr(cb, chain);
+		add_columns(a, n);
+		CUfunction f = module->Get("vgpu_mat_onepass");
+		const int occ = std::max(1, Runtime::Get().MaxActiveBlocks(f, g.block, smem));
+		LaunchGenerated(*module, "vgpu_mat_onepass",
+		                static_cast<unsigned>(std::min<uint64_t>(ntiles + 1, uint64_t(sms) * occ)), g.block, smem, stream_, a,
+		                in_bytes, n);
+		// at the root, outputs without NULL masks may leave the count on the device
+		if (at_root && !null_outs && DeferRows(chain, 8, 0)) return out;
+		out_rows = ReadU64(chain);
+		if (out_rows > n) Fail(VGPU_ERR_CUDA, "gpu_executor: a row filter's tiles were not completed within two seconds");
+		for (auto &col : out) {
+			col.rows = out_rows;
+			// a result that keeps few of many rows does not hold on to the room for all of them
+			if (n * row_bytes > (64ull << 20) && out_rows < n / 4) {
+				auto shrink = [&](void *p, size_t width) {
+					void *q = arena_.Alloc(out_rows * width);
+					if (out_rows) VGPU_CUDA(cudaMemcpyAsync(q, p, out_rows * width, cudaMemcpyDeviceToDevice, stream_));
+					arena_.FreeNow(p);
+					return q;
+				};
+				col.data = shrink(col.data, TypeSize(col.type));
+				if (col.valid) col.valid = static_cast<uint8_t *>(shrink(col.valid, 1));
+			}
+		}
+		return out;
+	}
 	if (cg.has_filter() && n > 0) {
-		uint64_t in_bytes = 0;
-		for (auto &s : pin.sources) in_bytes += s.rows * TypeSize(s.type);
 		KArgsHost a;
 		FillArgs(pin, a);
 		if (pin.spec.join_multi) {  // 64-bit tile counts: the matches can outnumber the rows
@@ -565,13 +639,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 			kern::ExclusiveScanU32(tile_counts, tile_counts, ntiles, total, arena_);
 			// at the root, outputs without NULL masks may take a row per input row and leave the count
 			// on the device
-			bool defer = at_root;
-			uint64_t row_bytes = 0;
-			for (int c : out_cols) {
-				defer = defer && !cg.visible()[c].nullable;
-				row_bytes += TypeSize(cg.visible()[c].type);
-			}
-			if (defer && DeferRows(total, 4, n * row_bytes)) {
+			if (at_root && !null_outs && DeferRows(total, 4, n * row_bytes)) {
 				out_rows = n;
 			} else {
 				out_rows = ReadU32(total);
@@ -579,29 +647,10 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 			tile_offsets = tile_counts;
 		}
 	}
-	Relation out;
 	KArgsHost a;
 	FillArgs(pin, a);
 	a.SetPtr(cb, tile_offsets);
-	for (size_t c = 0; c < out_cols.size(); c++) {
-		const auto &vc = cg.visible()[out_cols[c]];
-		DevColumn col;
-		col.name = names[c];
-		col.type = vc.type;
-		col.rows = out_rows;
-		col.data = arena_.Alloc(out_rows * TypeSize(vc.type));
-		if (vc.nullable) {
-			col.valid = arena_.AllocT<uint8_t>(out_rows);
-		}
-		if (vc.source >= 0 && pin.sources[vc.source].has_stats) {
-			col.has_stats = true;
-			col.min = pin.sources[vc.source].min;
-			col.max = pin.sources[vc.source].max;
-		}
-		a.SetPtr(cb + 1 + 2 * static_cast<int>(c), col.data);
-		a.SetPtr(cb + 2 + 2 * static_cast<int>(c), col.valid);
-		out.push_back(col);
-	}
+	add_columns(a, out_rows);
 	if (n > 0 && (out_rows > 0 || !cg.has_filter())) {
 		LaunchGenerated(*module, "vgpu_mat_write", grid, g.block, 0, stream_, a, 0, n);
 	}
