@@ -13,6 +13,7 @@
 #pragma once
 
 #include <memory>
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -127,6 +128,8 @@ public:
 		// One-pass group-by, MIN/MAX: >= 0 keeps the shared-memory state as a 32-bit offset from the
 		// value in this argument word (the input's minimum; its range spans less than 2^32).
 		int narrow_word = -1;
+		// L2 table: an integer SUM or AVG whose total over all rows cannot leave 64 bits keeps one word.
+		bool sum64 = false;
 	};
 	struct GroupBySpec {
 		std::vector<GroupKey> keys;
@@ -174,6 +177,17 @@ public:
 	//!  direct-partitioned: vgpu_gb_part_count, vgpu_gb_part_scatter, vgpu_gb_dtab_init, vgpu_gb_dbucket
 	std::string EmitGroupBy(const GroupBySpec &gb, bool partitioned, const Geometry &g) const;
 
+	//! One-pass group-by into one table of the whole key space in global memory, which L2 holds:
+	//! vgpu_gb_l2_init, vgpu_gb_l2 (kL2HotSlots * StateWords words of dynamic shared memory), vgpu_gb_l2_final.
+	static constexpr uint64_t kL2TableBytes = 64ull << 20;
+	static constexpr int kL2HotSlots = 512, kL2SampleRows = 2048, kL2FinalTile = 1024;
+	std::string EmitGroupByL2(const GroupBySpec &gb, const Geometry &g) const;
+	//! Argument word of its compaction chain (total, ticket, tile counts and starts); the next one takes
+	//! the hot keys' tags (kL2HotSlots u32).
+	int L2ChainWord(const GroupBySpec &gb) const {
+		return ConsumerBase() + 1 + StateWords(gb) + static_cast<int>(gb.keys.size() + gb.aggs.size());
+	}
+
 	//! Word offsets inside one query's row of a batch query table (see EmitBatchGroupBy).
 	struct BatchLayout {
 		int qwords = 0;
@@ -214,7 +228,8 @@ private:
 	std::string EmitExpression(const Expr &expr, const std::vector<PipeColumn> &cols, int index);
 	std::string Prologue() const;
 	std::string LoadDecls(const Geometry &g, const std::vector<bool> &needed) const;
-	std::string LoadBlock(const Geometry &g, const std::vector<bool> &needed, bool declare = true) const;
+	std::string LoadBlock(const Geometry &g, const std::vector<bool> &needed, bool declare = true,
+	                      const std::string &first_row = std::string()) const;
 	//! Opens the per-item loop of a tile: `row`, `keep` and (for a multi-match join source) the loop over
 	//! the row's matches with the needed right columns loaded at each; ItemClose closes what it opened.
 	std::string ItemOpen(const Geometry &g, const std::vector<bool> &needed) const;

@@ -125,6 +125,9 @@ struct Walker {
 			if (SatMul(groups, fields * 8) <= 96 * 1024) {
 				// one pass: per-CTA shared tables, one global table over the key domain, outputs
 				bytes = SatAdd(SatMul(groups, fields * 8 + out_width), 64);
+			} else if (n.estimated_rows && SatMul(groups, fields * 8) <= PipelineCodegen::kL2TableBytes / 4) {
+				// one pass into a table over the key domain (dense keys: up to twice the groups), outputs
+				bytes = SatMul(groups, 2 * fields * 8 + out_width);
 			} else {
 				// partitioned: one record per passing row (packed key + carried values, 32-byte aligned),
 				// outputs per group, per-(partition, CTA) offsets, tables of split partitions
@@ -472,13 +475,15 @@ std::string GenerateSourceText(const PlanNode &plan, const std::vector<vgpu_colu
 	gst.staged = true;
 	// Separate translation units, separated by a marker line: direct, partitioned, key statistics,
 	// direct-partitioned, direct-partitioned with heavy keys, the last two staged, the plain bucket pass,
-	// and the direct one with narrow counts and MIN/MAX.
+	// the direct one with narrow counts and MIN/MAX, and the table held in L2.
+	Geometry gl = g;
+	gl.items = 4;
 	return cg.EmitGroupBy(spec_gb, false, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_gb, true, g) +
 	       "\n//@@VGPU_TU@@\n" + cg.EmitStats(key_columns, gs) + "\n//@@VGPU_TU@@\n" +
 	       cg.EmitGroupBy(spec_dp, true, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_hv, true, g) +
 	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_dp, true, gst) + "\n//@@VGPU_TU@@\n" +
 	       cg.EmitGroupBy(spec_hv, true, gst) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_plain, true, g) +
-	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_nc, false, g);
+	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_nc, false, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupByL2(spec_gb, gl);
 }
 
 } // namespace vgpu
