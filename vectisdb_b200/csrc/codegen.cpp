@@ -2583,22 +2583,41 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 }
 
 std::string SpecKey(const PipelineSpec &spec) {
-	std::ostringstream o;
-	o << "src:";
+	std::string k = "src:";
+	auto num = [&](long long v, char end) {
+		k += std::to_string(v);
+		k += end;
+	};
 	for (auto &sc : spec.sources) {
-		o << sc.name << '/' << static_cast<int>(sc.type) << '/' << sc.nullable << '/' << sc.side << ';';
+		k += sc.name;
+		k += '/';
+		num(static_cast<int>(sc.type), '/');
+		num(sc.nullable, '/');
+		num(sc.side, ';');
 	}
-	o << "|cross:" << spec.cross << "|join:" << spec.join << '/' << spec.join_key << '/' << spec.join_inline << '/' << spec.join_multi << '/' << spec.join_minline << "|chain:";
+	k += "|cross:";
+	num(spec.cross, '/');
+	num(spec.join, '/');
+	num(spec.join_key, '/');
+	num(spec.join_inline, '/');
+	num(spec.join_multi, '/');
+	num(spec.join_minline, '|');
 	for (const PlanNode *n : spec.chain) {
-		o << static_cast<int>(n->op) << '{';
+		num(static_cast<int>(n->op), '{');
 		for (auto &e : n->expressions) {
-			o << static_cast<int>(e.output_type) << ':' << e.source.size() << ':' << e.source << '(';
-			for (auto &in : e.input_columns) o << in << ',';
-			o << ')';
+			num(static_cast<int>(e.output_type), ':');
+			num(static_cast<long long>(e.source.size()), ':');
+			k += e.source;
+			k += '(';
+			for (auto &in : e.input_columns) {
+				k += in;
+				k += ',';
+			}
+			k += ')';
 		}
-		o << '}';
+		k += '}';
 	}
-	return o.str();
+	return k;
 }
 
 std::string GroupByKey(const PipelineCodegen::GroupBySpec &gb, bool partitioned) {
@@ -2615,9 +2634,12 @@ std::string GroupByKey(const PipelineCodegen::GroupBySpec &gb, bool partitioned)
 }
 
 std::shared_ptr<const PipelineCodegen> CodegenFor(const PipelineSpec &spec) {
+	return CodegenFor(spec, SpecKey(spec));
+}
+
+std::shared_ptr<const PipelineCodegen> CodegenFor(const PipelineSpec &spec, const std::string &key) {
 	static std::mutex mu;
 	static std::map<std::string, std::shared_ptr<const PipelineCodegen>> memo;
-	const std::string key = SpecKey(spec);
 	{
 		std::lock_guard<std::mutex> lock(mu);
 		auto it = memo.find(key);

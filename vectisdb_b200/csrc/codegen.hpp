@@ -253,6 +253,8 @@ std::string GroupByKey(const PipelineCodegen::GroupBySpec &gb, bool partitioned)
 //! A code generator for `spec`, shared by every pipeline with the same SpecKey (the chain's nodes are
 //! read only while it is built).
 std::shared_ptr<const PipelineCodegen> CodegenFor(const PipelineSpec &spec);
+//! ... with the pipeline's SpecKey already at hand.
+std::shared_ptr<const PipelineCodegen> CodegenFor(const PipelineSpec &spec, const std::string &key);
 
 //! Registers the reference access forms of an expression source: returns the rewritten statement or
 //! throws Error(VGPU_ERR_UNSUPPORTED) when the source uses inputs/out/row/idx any other way.

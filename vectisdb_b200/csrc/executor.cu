@@ -215,6 +215,14 @@ private:
 		uint64_t rows = 0;              // pairs for CROSS
 		uint64_t right_rows = 0;
 		uint64_t join_words[4] = {0, 0, 0, 0};  // join source: sorted keys, directory, bias, shift | nb << 8
+		//! SpecKey(spec), built once the spec is complete.
+		const std::string &Key() {
+			if (key.empty()) key = SpecKey(spec);
+			return key;
+		}
+
+	private:
+		std::string key;
 	};
 
 	Relation Scan(const PlanNode &node);
@@ -524,7 +532,7 @@ Executor::PipelineInput Executor::PipelineOver(const Relation &rel) {
 
 Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_cols,
                                const std::vector<std::string> &names, bool at_root) {
-	auto cgp = CodegenFor(pin.spec);
+	auto cgp = CodegenFor(pin.spec, pin.Key());
 	const PipelineCodegen &cg = *cgp;
 	const uint64_t n = pin.rows;
 	const uint64_t row_bytes = cg.OnePassRowBytes(out_cols);
@@ -547,7 +555,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 	g.items = 4;
 	if (one_pass) g.block = 128;
 	const size_t smem = one_pass ? static_cast<size_t>(2 * g.tile() * row_bytes) : 0;
-	std::string mkey = "mat|" + SpecKey(pin.spec) + "|outs:";
+	std::string mkey = "mat|" + pin.Key() + "|outs:";
 	for (int c : out_cols) mkey += std::to_string(c) + ",";
 	mkey += "|g:" + std::to_string(g.block) + "x" + std::to_string(g.items) + (one_pass ? "o" : "");
 	auto module = Runtime::Get().modules().GetOrCompileMemo(mkey, [&] {
@@ -670,7 +678,7 @@ Relation Executor::RunChain(const PlanNode &node) {
 		cur = cur->children[0].get();
 	}
 	PipelineInput pin = BuildPipeline(*cur, chain, true);
-	auto probe_cg = CodegenFor(pin.spec);
+	auto probe_cg = CodegenFor(pin.spec, pin.Key());
 	const PipelineCodegen &probe = *probe_cg;
 	std::vector<int> outs;
 	std::vector<std::string> names;
@@ -731,7 +739,7 @@ void Executor::ComputeStats(PipelineInput &pin, const PipelineCodegen &cg, const
 	Geometry g;
 	g.block = 256;
 	g.items = 4;
-	std::string skey = "stats|" + SpecKey(pin.spec) + "|cols:";
+	std::string skey = "stats|" + pin.Key() + "|cols:";
 	for (int c : missing) skey += std::to_string(c) + ",";
 	auto module = Runtime::Get().modules().GetOrCompileMemo(skey, [&] { return cg.EmitStats(missing, g); });
 	int64_t *mm = arena_.AllocT<int64_t>(2 * missing.size());
@@ -863,7 +871,7 @@ Relation Executor::GroupBy(const PlanNode &node) {
 }
 
 Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
-	auto cgp = CodegenFor(pin.spec);
+	auto cgp = CodegenFor(pin.spec, pin.Key());
 	const PipelineCodegen &cg = *cgp;
 	if (cg.visible().empty()) {
 		Fail(VGPU_ERR_INVALID_ARGUMENT, "gpu_groupby: input operator produced no columns to group");
@@ -967,14 +975,16 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	const int out_words = key_words + static_cast<int>(gb.aggs.size());
 	gb.domain = domain;
 
-	// Output columns, sized for the largest possible group count.
+	// Output columns, sized for the largest possible group count. The few groups of a shared-memory table that
+	// are the query's result on the host go straight to page-locked memory, the count in front: the last
+	// kernel's writes cross the link as it runs, and one wait replaces the count's read-back, a copy per column
+	// and a second wait (4096 rows into 16 groups 0.069 -> 0.031 ms per call, 2^24 rows into 1024 groups 0.132 -> 0.100 ms).
 	const uint64_t cap_rows = direct || pin.spec.join_multi ? domain : std::min<uint64_t>(domain, n);
 	Relation out;
 	for (size_t i = 0; i < key_cols.size(); i++) {
 		DevColumn c;
 		c.name = node.group_keys[i];
 		c.type = cg.visible()[key_cols[i]].type;
-		c.data = arena_.Alloc(cap_rows * TypeSize(c.type));
 		c.has_stats = true;
 		c.min = ranges[i].first;
 		c.max = ranges[i].second;
@@ -984,8 +994,21 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		DevColumn c;
 		c.name = "agg_" + std::to_string(i);
 		c.type = node.aggregates[i].output_type;
-		c.data = arena_.Alloc(cap_rows * TypeSize(c.type));
 		out.push_back(c);
+	}
+	uint64_t host_bytes = 16;
+	for (auto &c : out) host_bytes += (cap_rows * TypeSize(c.type) + 15) / 16 * 16;
+	std::shared_ptr<uint8_t> host;  // [0] the count, then the columns
+	if (direct && &node == root_ && !options_.output_on_device && host_bytes <= 256 * 1024) {
+		host = PinnedPool::Get().Acquire(host_bytes);
+		uint64_t off = 16;
+		for (auto &c : out) {
+			c.host = std::shared_ptr<uint8_t>(host, host.get() + off);
+			c.data = c.host.get();
+			off += (cap_rows * TypeSize(c.type) + 15) / 16 * 16;
+		}
+	} else {
+		for (auto &c : out) c.data = arena_.Alloc(cap_rows * TypeSize(c.type));
 	}
 	uint64_t in_bytes = 0;
 	for (auto &s : pin.sources) in_bytes += s.rows * TypeSize(s.type);
@@ -1037,11 +1060,13 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		if (const char *env = std::getenv("VGPU_GB_DIRECT_BLOCK")) {  // tuning override (whole warps)
 			g.block = std::max(64, std::min(1024, std::atoi(env))) / 32 * 32;
 		}
-		const std::string gkey = SpecKey(pin.spec) + "|" + GroupByKey(gb, false) + "|g:" + std::to_string(g.block) + "x" +
+		const std::string gkey = pin.Key() + "|" + GroupByKey(gb, false) + "|g:" + std::to_string(g.block) + "x" +
 		                         std::to_string(g.items);
 		auto module = Runtime::Get().modules().GetOrCompileMemo(gkey, [&] { return cg.EmitGroupBy(gb, false, g); });
-		uint64_t *fields = arena_.AllocT<uint64_t>(domain * F);
-		uint64_t *count = arena_.AllocT<uint64_t>(1);
+		// the tables, the finished-CTA ticket and, unless the result may take it over, the count
+		uint64_t *fields = arena_.AllocT<uint64_t>(domain * F + 2);
+		uint64_t *count = host ? reinterpret_cast<uint64_t *>(host.get())
+		                  : options_.no_sync ? arena_.AllocT<uint64_t>(1) : fields + domain * F + 1;
 		KArgsHost a;
 		FillArgs(pin, a);
 		SetKeyWords(a, gb);
@@ -1050,7 +1075,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		for (int w = 0; w < out_words; w++) a.SetPtr(cb + 1 + F + w, out[w].data);
 		a.SetPtr(cb + 1 + F + out_words, count);
 		const bool fused_final = cg.DirectFinalFused(gb);
-		if (fused_final) a.SetPtr(cb + 3 + F + out_words, arena_.AllocT<uint32_t>(1));  // finished-CTA ticket
+		if (fused_final) a.SetPtr(cb + 3 + F + out_words, fields + domain * F);
 		for (auto &na : narrow_args) a.Set(na.first, static_cast<uint64_t>(na.second));
 		const unsigned init_grid = static_cast<unsigned>(std::min<uint64_t>((domain + 255) / 256, 1024));
 		LaunchGenerated(*module, "vgpu_gb_direct_init", init_grid, 256, 0, stream_, a, domain * F * 8, domain);
@@ -1063,7 +1088,10 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		if (direct_l2) a.SetPtr(cb + 2 + F + out_words, arena_.AllocT<uint64_t>(uint64_t(grid) * direct_f64 * domain));
 		LaunchGenerated(*module, "vgpu_gb_direct", grid, g.block, smem, stream_, a, in_bytes, n);
 		if (!fused_final) LaunchGenerated(*module, "vgpu_gb_direct_final", 1, 1024, 0, stream_, a, domain * F * 8, domain);
-		if (&node == root_ && !node.group_keys.empty() && DeferRows(count, 8, 0)) {
+		if (host) {
+			VGPU_CUDA(cudaStreamSynchronize(stream_));
+			std::memcpy(&groups, host.get(), sizeof(groups));
+		} else if (&node == root_ && !node.group_keys.empty() && DeferRows(count, 8, 0)) {
 			groups = domain;  // the columns already hold a slot per key value
 		} else {
 			groups = ReadU64(count);
@@ -1073,7 +1101,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		Geometry g;
 		g.block = 512;
 		g.items = 4;
-		const std::string gkey = SpecKey(pin.spec) + "|" + GroupByKey(gb, false) + "|l2";
+		const std::string gkey = pin.Key() + "|" + GroupByKey(gb, false) + "|l2";
 		auto module = Runtime::Get().modules().GetOrCompileMemo(gkey, [&] { return cg.EmitGroupByL2(gb, g); });
 		const uint64_t final_tiles = domain / PipelineCodegen::kL2FinalTile;
 		uint64_t *fields = arena_.AllocT<uint64_t>(domain * F);
@@ -1217,7 +1245,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		}
 		g.staged = staged;
 		auto compile = [&](const PipelineCodegen::GroupBySpec &spec) {
-			const std::string gkey = SpecKey(pin.spec) + "|" + GroupByKey(spec, true) + "|g:" + std::to_string(g.block) +
+			const std::string gkey = pin.Key() + "|" + GroupByKey(spec, true) + "|g:" + std::to_string(g.block) +
 			                         "x" + std::to_string(g.items) + (g.staged ? "s" : "") + "m" + std::to_string(g.min_blocks);
 			return Runtime::Get().modules().GetOrCompileMemo(gkey, [&] { return cg.EmitGroupBy(spec, true, g); });
 		};
@@ -1986,6 +2014,7 @@ ExecResult ExecutePlan(const PlanNode &plan, const std::vector<vgpu_column> &inp
 	Relation rel = ex.Exec(plan);
 	ExecResult result;
 	result.stream = stream;
+	bool copies = false;
 	if (void *rows = ex.deferred_rows()) {
 		result.pending_rows = rows;
 		result.pending_rows_bytes = ex.deferred_rows_bytes();
@@ -2018,11 +2047,15 @@ ExecResult ExecutePlan(const PlanNode &plan, const std::vector<vgpu_column> &inp
 				o.device_validity = bm;
 			}
 		} else {
-			if (bytes) {
+			if (bytes && c.host) {
+				o.host = c.host;
+			} else if (bytes) {
+				copies = true;
 				o.host = PinnedPool::Get().Acquire(bytes);
 				VGPU_CUDA(cudaMemcpyAsync(o.host.get(), c.data, bytes, cudaMemcpyDeviceToHost, stream));
 			}
 			if (c.valid && c.rows > 0) {
+				copies = true;
 				const size_t vb = (c.rows + 7) / 8;
 				uint8_t *bm = ex.arena().AllocT<uint8_t>(vb);
 				kern::PackValidity(c.valid, bm, c.rows, stream);
@@ -2032,7 +2065,8 @@ ExecResult ExecutePlan(const PlanNode &plan, const std::vector<vgpu_column> &inp
 		}
 		result.columns.push_back(std::move(o));
 	}
-	if (!(options.output_on_device && options.no_sync)) {
+	// (a result written straight to the host has been waited for)
+	if (options.output_on_device ? !options.no_sync : copies || rel.empty() || !rel.front().host) {
 		VGPU_CUDA(cudaStreamSynchronize(stream));
 	}
 	return result;
