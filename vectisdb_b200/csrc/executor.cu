@@ -1933,8 +1933,6 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	}
 	if (ln >= (1ull << 32) || rn >= (1ull << 32)) Fail(VGPU_ERR_UNSUPPORTED, "gpu_hash_join: side too large");
 	const size_t kw = TypeSize(lk.type);
-	uint64_t *lw = arena_.AllocT<uint64_t>(ln);
-	uint64_t *rw = arena_.AllocT<uint64_t>(rn);
 	uint64_t *words = arena_.AllocT<uint64_t>(2);
 	const kern::BoundsColumn want {rk.data, rn, kern::RawBoundsKind(kw)};
 	kern::ColumnBounds(&want, 1, words, stream_);
@@ -1942,7 +1940,49 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	const uint64_t bias = kern::BoundsLow(bounds.data(), want.kind);
 	const uint64_t range = kern::BoundsHigh(bounds.data(), want.kind) - bias;
 	const int bits = BitsFor(range);
-	kern::WidenKeys(lk.data, kw, ln, 0, lw, stream_);
+	const bool dense = range < (1ull << 28) && range < 4 * rn;
+	auto too_large = [](uint64_t rows) {
+		Fail(VGPU_ERR_UNSUPPORTED, "gpu_hash_join: join result of " + std::to_string(rows) +
+		                               " rows is too large for GPU execution");
+	};
+	// Matches written by tiles of left rows: for up to 16 output columns, while no tile of 1024 left rows has over
+	// 2^16 matches (one CTA writes a tile: at 64 matches a row the longest one still takes microseconds; past
+	// that the expansion below spreads a row's matches over many CTAs). Dense right keys need no sort.
+	const bool tiled = sources.size() <= static_cast<size_t>(kern::kMaxJoinOuts);
+	// two words for JoinDenseRuns' info, then the chain of the count: read back together
+	uint64_t *info = tiled ? arena_.AllocT<uint64_t>(2 + kern::JoinChainWords(ln)) : nullptr;
+	uint64_t *chain = info + 2;
+	auto emit_tiles = [&](const kern::JoinRunsView &view, const uint32_t *rows, Relation &out) {
+		kern::JoinCountMatches(lk.data, kw, ln, view, chain, stream_);
+		const std::vector<uint64_t> head = ReadWords(info, 4);
+		if (view.entries && (head[0] >> 32) > kern::kJoinRunLimit) return false;  // a run not in row order
+		if ((head[2] >> 62) != 0 || (head[3] >> 32) > (1u << 16)) return false;
+		const uint64_t total = head[2];
+		if (total > kMaxOutputRows) too_large(total);
+		out = make_out(total);
+		if (total == 0) return true;
+		kern::JoinOuts outs;
+		for (size_t i = 0; i < sources.size(); i++) {
+			outs.c[outs.n++] = {sources[i]->data, out[i].data, static_cast<int>(TypeSize(sources[i]->type)), !from_left[i]};
+		}
+		kern::JoinEmit(lk.data, kw, ln, view, chain, rows, outs, total, stream_);
+		return true;
+	};
+	if (tiled && dense) {
+		uint64_t *entries = arena_.AllocT<uint64_t>(range + 1);
+		uint32_t *rows = arena_.AllocT<uint32_t>(rn);
+		uint32_t *list = arena_.AllocT<uint32_t>(rn / 17 + 1);
+		kern::JoinDenseRuns(rk.data, kw, rn, bias, range, entries, rows, list, reinterpret_cast<uint32_t *>(info), stream_);
+		kern::JoinRunsView view;
+		view.entries = entries;
+		view.nb = range + 1;
+		view.bias = bias;
+		Relation out;
+		if (emit_tiles(view, rows, out)) return out;
+		arena_.FreeNow(entries);
+		arena_.FreeNow(rows);
+	}
+	uint64_t *rw = arena_.AllocT<uint64_t>(rn);
 	kern::WidenKeys(rk.data, kw, rn, bias, rw, stream_);
 	uint32_t *perm = arena_.AllocT<uint32_t>(rn);
 	uint64_t *rw_alt = arena_.AllocT<uint64_t>(rn);
@@ -1952,20 +1992,29 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	arena_.FreeNow(perm_alt);
 	// each left key's run of equal right keys through a radix directory: one bucket per key value when
 	// the key range is dense (the run is read, not searched), else 2^22 buckets and a short search
-	const uint32_t shift = (range < (1ull << 28) && range < 4 * rn) ? 0u : bits > 22 ? static_cast<uint32_t>(bits - 22) : 0u;
+	const uint32_t shift = dense ? 0u : bits > 22 ? static_cast<uint32_t>(bits - 22) : 0u;
 	const uint64_t nb = (range >> shift) + 1;
 	uint32_t *dir = arena_.AllocT<uint32_t>(nb + 1);
 	kern::JoinDirectory(rw, rn, shift, nb, dir, stream_);
+	if (tiled && !dense) {
+		kern::JoinRunsView view;
+		view.sorted = rw;
+		view.dir = dir;
+		view.nb = nb;
+		view.bias = bias;
+		view.shift = shift;
+		Relation out;
+		if (emit_tiles(view, perm, out)) return out;
+	}
+	uint64_t *lw = arena_.AllocT<uint64_t>(ln);
+	kern::WidenKeys(lk.data, kw, ln, 0, lw, stream_);
 	uint64_t *lower = arena_.AllocT<uint64_t>(ln);
 	uint64_t *counts = arena_.AllocT<uint64_t>(ln);
 	kern::JoinRuns(lw, ln, rw, dir, nb, shift, bias, lower, counts, stream_);
 	uint64_t *total = arena_.AllocT<uint64_t>(1);
 	kern::ExclusiveScanU64(counts, counts, ln, total, arena_);
 	const uint64_t total_rows = ReadU64(total);
-	if (total_rows > kMaxOutputRows) {
-		Fail(VGPU_ERR_UNSUPPORTED, "gpu_hash_join: join result of " + std::to_string(total_rows) +
-		                               " rows is too large for GPU execution");
-	}
+	if (total_rows > kMaxOutputRows) too_large(total_rows);
 	Relation out = make_out(total_rows);
 	if (total_rows == 0) return out;
 	uint32_t *out_left = arena_.AllocT<uint32_t>(total_rows);

@@ -83,6 +83,43 @@ void JoinExpand(const uint64_t *offsets, const uint64_t *lower, uint64_t n_left,
 void JoinRuns(const uint64_t *probe, uint64_t n_probe, const uint64_t *sorted, const uint32_t *dir, uint64_t nb,
               uint32_t shift, uint64_t bias, uint64_t *lower, uint64_t *count, cudaStream_t stream);
 
+//! Where a left key's right rows are: dense keys by an entry per key value (JoinDenseRuns), else a sorted key
+//! array with its radix directory (`entries` null).
+struct JoinRunsView {
+	const uint64_t *entries = nullptr;
+	const uint64_t *sorted = nullptr;
+	const uint32_t *dir = nullptr;
+	uint64_t nb = 0;  // entries, or directory buckets
+	uint64_t bias = 0;
+	uint32_t shift = 0;
+};
+//! Longest run JoinDenseRuns puts in row order.
+constexpr uint32_t kJoinRunLimit = 4096;
+//! The rows of each key value contiguous in `rows` [n], in row order, and an entry per value of the range (range
+//! + 1 words of `entries`), without sorting the keys. `list` [n / 17 + 1] and `info` [3] are scratch; info[1]
+//! becomes the longest run's length: past kJoinRunLimit that run is not in order, and the caller sorts instead.
+void JoinDenseRuns(const void *keys, size_t kwidth, uint64_t n, uint64_t bias, uint64_t range, uint64_t *entries,
+                   uint32_t *rows, uint32_t *list, uint32_t *info, cudaStream_t stream);
+//! Matches of the left rows (raw keys): chain [JoinChainWords] = the total (bits 62 and 63 set when a tile has 2^31
+//! or a wait ran out), [1] >> 32 = the most matches of one tile of left rows, then the tiles' starts for JoinEmit.
+uint64_t JoinChainWords(uint64_t n_left);
+void JoinCountMatches(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, uint64_t *chain,
+                      cudaStream_t stream);
+struct JoinOut {
+	const void *src;
+	void *dst;
+	int width;   // 1, 2, 4, 8 or 16
+	bool right;  // a column of the right side
+};
+constexpr int kMaxJoinOuts = 16;
+struct JoinOuts {
+	JoinOut c[kMaxJoinOuts];
+	int n = 0;
+};
+//! Every output column of the matches, left rows in order and each one's matches in the order of `rows`.
+void JoinEmit(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, const uint64_t *chain,
+              const uint32_t *rows, const JoinOuts &outs, uint64_t total, cudaStream_t stream);
+
 //! Radix directory of a sorted (biased) key array: dir[b] = first position whose key >> shift >= b,
 //! for b in [0, nb]; dir needs nb + 1 entries and nb must exceed every key >> shift.
 void JoinDirectory(const uint64_t *sorted, uint64_t n, uint32_t shift, uint64_t nb, uint32_t *dir, cudaStream_t stream);
