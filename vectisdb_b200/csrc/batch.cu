@@ -185,7 +185,7 @@ struct BatchEntry {
 		auto &al = Runtime::Get().allocator();
 		if (graph) cudaGraphExecDestroy(graph);
 		graph = nullptr;
-		for (void *p : {static_cast<void *>(qtab), static_cast<void *>(acc), static_cast<void *>(counts),
+		for (void *p : {static_cast<void *>(qtab), static_cast<void *>(acc), static_cast<void *>(pinned ? nullptr : counts),
 		                static_cast<void *>(outp), static_cast<void *>(work), tiles}) {
 			if (p) al.Free(p, stream);
 		}
@@ -469,16 +469,17 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 		e->qtab = static_cast<uint64_t *>(al.Alloc(qt.size() * 8, stream));
 		e->tiles = al.Alloc(std::max<size_t>(8, tl.size() * 4), stream);
 		e->acc = static_cast<uint64_t *>(al.Alloc(e->acc_words * F * 8, stream));
-		e->counts = static_cast<uint64_t *>(al.Alloc(qs.size() * 8, stream));
 		e->outp = static_cast<uint64_t *>(al.Alloc(out_words * 8, stream));
 		e->work = static_cast<uint32_t *>(al.Alloc(16, stream));
 		if (transient) {
 			e->pinned = false;
 			e->host_stage.assign(qs.size() + out_words, 0);
+			e->counts = static_cast<uint64_t *>(al.Alloc(qs.size() * 8, stream));
 			e->counts_host = e->host_stage.data();
 			e->outp_host = e->host_stage.data() + qs.size();
 		} else {
 			VGPU_CUDA(cudaMallocHost(&e->counts_host, qs.size() * 8));
+			e->counts = e->counts_host;  // written there by the finalize kernel
 			VGPU_CUDA(cudaMallocHost(&e->outp_host, out_words * 8));
 		}
 		VGPU_CUDA(cudaMemcpyAsync(e->qtab, qt.data(), qt.size() * 8, cudaMemcpyHostToDevice, stream));
@@ -588,9 +589,27 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 		out_types.push_back(root.aggregates[i].output_type);
 		out_names.push_back("agg_" + std::to_string(i));
 	}
-	for (size_t w = 0; w < out_words; w++) {
-		holder->ptrs.push_back(Runtime::Get().allocator().Alloc(std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]), stream));
-		e.outp_host[w] = reinterpret_cast<uint64_t>(holder->ptrs[w]);
+	// Host results of moderate size go straight to page-locked memory, which each query's columns then share:
+	// only the groups there are cross the link, as the finalize kernel finds them. (Copies of the whole
+	// capacity into pageable memory and out of it again took four fifths of a call: 20 queries with 1.6e5 groups
+	// 0.85 -> 0.27 ms in the engine.) Past 32 MB of capacity the memory held would outweigh that.
+	uint64_t capacity = 0;
+	for (size_t w = 0; w < out_words; w++) capacity += (std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]) + 255) / 256 * 256;
+	std::shared_ptr<uint8_t> host;
+	std::vector<uint64_t> host_off(out_words, 0);
+	if (!options.output_on_device && capacity <= (32ull << 20)) {
+		host = PinnedPool::Get().Acquire(capacity);
+		uint64_t off = 0;
+		for (size_t w = 0; w < out_words; w++) {
+			host_off[w] = off;
+			e.outp_host[w] = reinterpret_cast<uint64_t>(host.get() + off);
+			off += (std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]) + 255) / 256 * 256;
+		}
+	} else {
+		for (size_t w = 0; w < out_words; w++) {
+			holder->ptrs.push_back(Runtime::Get().allocator().Alloc(std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]), stream));
+			e.outp_host[w] = reinterpret_cast<uint64_t>(holder->ptrs[w]);
+		}
 	}
 	VGPU_CUDA(cudaMemcpyAsync(e.outp, e.outp_host, out_words * 8, cudaMemcpyHostToDevice, stream));
 	init_if_needed(e);
@@ -622,9 +641,9 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 	} else {
 		enqueue(e, true);
 	}
-	VGPU_CUDA(cudaMemcpyAsync(e.counts_host, e.counts, e.nq * 8, cudaMemcpyDeviceToHost, stream));
+	if (!e.pinned) VGPU_CUDA(cudaMemcpyAsync(e.counts_host, e.counts, e.nq * 8, cudaMemcpyDeviceToHost, stream));
 	std::vector<std::vector<uint8_t>> host_out;
-	if (!options.output_on_device) {
+	if (!options.output_on_device && !host) {
 		host_out.resize(out_words);
 		for (size_t w = 0; w < out_words; w++) {
 			host_out[w].resize(e.out_rows * TypeSize(out_types[w]));
@@ -646,6 +665,8 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 			const size_t width = TypeSize(out_types[w]);
 			if (options.output_on_device) {
 				c.device_data = static_cast<char *>(holder->ptrs[w]) + e.out_base[qi] * width;
+			} else if (host) {
+				if (cnt) c.host = std::shared_ptr<uint8_t>(host, host.get() + host_off[w] + e.out_base[qi] * width);
 			} else {
 				const uint8_t *src = host_out[w].data() + e.out_base[qi] * width;
 				c.data.assign(src, src + cnt * width);

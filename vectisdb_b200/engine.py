@@ -584,14 +584,16 @@ class GpuEngine:
         else:
             results = []
             for i in range(n):
+                # zero-copy views of the result's own memory, freed with the last view (or with `owner`, should
+                # the reading fail)
                 h = C.c_void_p(handles[i])
+                owner = _ResultOwner(h)
                 try:
-                    columns = _read_result(h, None)
+                    columns = _read_result(h, owner)
                 except Exception:
-                    for j in range(i, n):
+                    for j in range(i + 1, n):
                         self.lib.vgpu_result_free(C.c_void_p(handles[j]))
                     raise
-                self.lib.vgpu_result_free(h)
                 results.append(GpuExecutionResult(True, "", abi.OK, columns))
         stats = {k: getattr(st, k) for k, _ in abi.vgpu_batch_stats._fields_}
         return results, stats
