@@ -207,6 +207,8 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 	if (it == staging_.end()) return;
 	cudaStream_t s = Runtime::Get().default_stream();
 	auto &alloc = Runtime::Get().allocator();
+	std::vector<std::pair<std::string, Entry>> done;
+	std::vector<kern::BoundsColumn> ranged;
 	for (auto &kv : it->second) {
 		Staged &st = kv.second;
 		if (st.failed || st.rows != scanned_rows) {
@@ -252,20 +254,32 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		}
 		e.bytes = st.bytes;
 		if (IsIntegerKeyType(st.type) || st.type == ValueType::DICTIONARY_STRING) {
-			uint64_t *mm = static_cast<uint64_t *>(alloc.Alloc(16, s));
-			const kern::BoundsColumn bc {e.column.data, st.rows, kern::SignedBoundsKind(st.type)};
-			kern::ColumnBounds(&bc, 1, mm, s);
-			uint64_t host[2];
-			VGPU_CUDA(cudaMemcpyAsync(host, mm, 16, cudaMemcpyDeviceToHost, s));
-			VGPU_CUDA(cudaStreamSynchronize(s));
-			alloc.Free(mm, s);
-			if (st.rows > 0) {
+			ranged.push_back({e.column.data, st.rows, kern::SignedBoundsKind(st.type)});
+		}
+		done.emplace_back(kv.first, std::move(e));
+	}
+	// the integer columns' ranges: one launch and one read-back for the table
+	std::vector<uint64_t> bounds(2 * ranged.size());
+	if (!ranged.empty()) {
+		uint64_t *mm = static_cast<uint64_t *>(alloc.Alloc(bounds.size() * 8, s));
+		kern::ColumnBounds(ranged.data(), static_cast<int>(ranged.size()), mm, s);
+		VGPU_CUDA(cudaMemcpyAsync(bounds.data(), mm, bounds.size() * 8, cudaMemcpyDeviceToHost, s));
+		VGPU_CUDA(cudaStreamSynchronize(s));
+		alloc.Free(mm, s);
+	}
+	size_t next = 0;
+	for (auto &named : done) {
+		Entry &e = named.second;
+		if (IsIntegerKeyType(e.column.type) || e.column.type == ValueType::DICTIONARY_STRING) {
+			const uint64_t *words = &bounds[2 * next];
+			const kern::BoundsKind kind = ranged[next++].kind;
+			if (e.column.rows > 0) {
 				e.column.has_stats = true;
-				e.column.min = static_cast<int64_t>(kern::BoundsLow(host, bc.kind));
-				e.column.max = static_cast<int64_t>(kern::BoundsHigh(host, bc.kind));
+				e.column.min = static_cast<int64_t>(kern::BoundsLow(words, kind));
+				e.column.max = static_cast<int64_t>(kern::BoundsHigh(words, kind));
 			}
 		}
-		const std::string key = Key(table, kv.first);
+		const std::string key = Key(table, named.first);
 		const bool replaced = entries_.count(key) != 0;
 		if (replaced) EvictLocked(key);  // the column staged again: the new contents replace the old entry
 		e.table_key = tk;
@@ -274,7 +288,7 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		committed_ += e.bytes;
 		entries_[key] = std::move(e);
 		auto &cols = table_columns_[tk];
-		if (std::find(cols.begin(), cols.end(), kv.first) == cols.end()) cols.push_back(kv.first);
+		if (std::find(cols.begin(), cols.end(), named.first) == cols.end()) cols.push_back(named.first);
 	}
 	VGPU_CUDA(cudaStreamSynchronize(s));
 	staging_.erase(it);
