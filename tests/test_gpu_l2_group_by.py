@@ -97,9 +97,10 @@ def test_cached_integer_sums_on_either_side_of_64_bits(limit):
     assert dict(zip(got[0].data.tolist(), hugeint_to_int(got[1].data))) == exp
 
 
-@pytest.mark.parametrize("span,taken", [(12_288, False), (12_289, True), (1 << 23, True), ((1 << 23) + 1, False)])
+@pytest.mark.parametrize("span,taken", [(12_288, False), (12_289, True), (1 << 23, True), ((1 << 23) + 1, True)])
 def test_range_of_key_spaces(span, taken):
-    """COUNT(*) alone: one state word per slot, so 2^13 slots still fit shared memory and 2^23 make 64 MB."""
+    """COUNT(*) alone: one state word per slot, so 2^13 slots still fit shared memory and 2^23 make 64 MB;
+    past that few rows of many key values are hashed."""
     span = {12_288: 8192, 12_289: 16_384}.get(span, span)
     rng = np.random.default_rng(span)
     k = rng.integers(0, span, 300_000).astype(np.int32)
@@ -171,3 +172,55 @@ def test_over_a_join_with_one_and_several_matches(repeat):
     assert np.array_equal(got[0].data, keys)
     assert hugeint_to_int(got[1].data) == np.bincount(inv, weights=lv[left]).astype(np.int64).tolist()
     assert np.array_equal(got[2].data, np.bincount(inv))
+
+
+@pytest.mark.parametrize("n,distinct,bits", [(2, 2, 62), (1000, 1000, 40), (8192, 3000, 63), (300_007, 60_000, 50),
+                                             (1_000_003, 1_000_003, 60), (2_000_003, 700_001, 55)])
+def test_sparse_keys_in_a_hashed_table(n, distinct, bits):
+    rng = np.random.default_rng(n)
+    ids = np.unique(np.concatenate([[0, (1 << bits) - 1], rng.integers(0, 1 << bits, distinct, dtype=np.int64)]))
+    pick = rng.integers(0, len(ids), n) if distinct < n else rng.permutation(np.arange(n) % len(ids))
+    hot = rng.random(n) < 0.3
+    pick[hot & (distinct < n)] = 1  # a frequent key
+    pick[:2] = [0, len(ids) - 1]
+    k = ids[pick] - (1 << 40)
+    v = rng.integers(-(1 << 62), 1 << 62, n, dtype=np.int64)
+    x = rng.integers(-1000, 1000, n).astype(np.float64)
+    plan = make_group_by(["k"], [make_aggregate(A.SUM, "x", T.FLOAT64), make_aggregate(A.MIN, "v", T.INT64),
+                                 make_aggregate(A.COUNT_STAR, "", T.INT64)], make_scan(["k", "x", "v"]))
+    got = _run(plan, [make_column("k", T.INT64, k), make_column("x", T.FLOAT64, x), make_column("v", T.INT64, v)])
+    keys, inv = np.unique(k, return_inverse=True)
+    order = np.argsort(got[0].data)
+    assert np.array_equal(got[0].data[order], keys)
+    assert np.array_equal(got[1].data[order], np.bincount(inv, weights=x))
+    lo = np.full(len(keys), np.iinfo(np.int64).max)
+    np.minimum.at(lo, inv, v)
+    assert np.array_equal(got[2].data[order], lo) and np.array_equal(got[3].data[order], np.bincount(inv))
+
+
+@pytest.mark.parametrize("keys,estimate,tried", [("pairs", 0, True), ("pairs", 600_000, True), ("pairs", 700_000, False),
+                                                 ("one", 0, False)])
+def test_more_sparse_keys_than_the_hashed_table_holds(keys, estimate, tried):
+    """Seven state words and the key make 2^20 slots of 64 MB. 1.5M pairs of two keys with some 1200 values each
+    end the pass, and the partitions do it; the plan's estimate, or one key's own distinct count, says so before."""
+    rng = np.random.default_rng(3)
+    n = 1_500_001
+    order = rng.permutation(n).astype(np.int64)
+    a, b = (order // 1225 * 1001, order % 1225 * 997) if keys == "pairs" else (order * 1_000_003, np.zeros(n, np.int64))
+    cols = [make_column("a", T.INT64, a), make_column("b", T.INT64, b)]
+    cols += [make_column(f"x{i}", T.INT64, np.roll(order, i + 1)) for i in range(6)]
+    plan = make_group_by(["a", "b"], [make_aggregate(A.MAX, f"x{i}", T.INT64) for i in range(6)],
+                         make_scan([c.name for c in cols]))
+    plan.estimated_rows = estimate
+    profile_drain()
+    profile_enable(True)
+    try:
+        r = GpuEngine.instance().execute_plan(plan, cols)
+        names = [rec[0] for rec in profile_drain()]
+    finally:
+        profile_enable(False)
+    assert r.success and (KERNEL in names) == tried and "vgpu_gb_bucket" in names, names
+    got, want = np.lexsort((r.columns[1].data, r.columns[0].data)), np.lexsort((b, a))
+    assert np.array_equal(r.columns[0].data[got], a[want]) and np.array_equal(r.columns[1].data[got], b[want])
+    for i in range(6):
+        assert np.array_equal(r.columns[2 + i].data[got], cols[2 + i].data[want])

@@ -2261,9 +2261,12 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 // up. 20M rows, 2^20 keys, SUM and COUNT, whole query: uniform keys 0.36 ms, one key in every row 0.19,
 // Zipf(1.1) 0.46, Zipf(2.0) 0.28 (partitioned: 0.94, 0.90, 0.96, 0.85). The per-CTA tables in global memory
 // instead took 0.61 ms for Zipf(1.1), and with a fence to read them back in the same launch 0.74 ms.
-// Arguments: cb = D, field arrays, outputs, the compaction's chain (see EmitMaterializeOnePass), the hot keys'
-// tags (u32 [kL2HotSlots]: slot + 1, or 0).
-std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry &g) const {
+//
+// `hashed`, for keys too sparse to be places: the same over a table of D key words with double hashing (one more
+// read of a random word per row, 280 G/s). More keys than fit raise a flag beside the ticket that ends the pass.
+// Arguments: cb = D, field arrays, outputs, the compaction's chain (see EmitMaterializeOnePass; the flag in the
+// ticket's word), the hot keys' tags ([kL2HotSlots] u32, u64 when hashed: key + 1, or 0), hashed: the keys.
+std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry &g, bool hashed) const {
 	std::ostringstream o;
 	o << Prologue();
 	const int cb = ConsumerBase();
@@ -2286,7 +2289,11 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	for (auto &a : gb.aggs) values.push_back(a.column >= 0 ? visible_[a.column].value : "0");
 	const int chain_word = L2ChainWord(gb);
 	const int H = kL2HotSlots;
-	const std::string hash = "((u32)slot * 0x9e3779b1u) >> " + std::to_string(32 - BitLength(H - 1));
+	// `slot` is the packed key in both forms: the place in a dense table follows from it, in a hashed one it is
+	// looked up (and entered); frequent keys are told by 32 or 64 bits
+	const std::string kt = hashed ? "u64" : "u32";
+	const std::string fold = hashed ? "(u32)(slot ^ (slot >> 32))" : "(u32)slot";
+	const std::string hash = "(" + fold + " * 0x9e3779b1u) >> " + std::to_string(32 - BitLength(H - 1));
 	// neighbouring keys a 64th of the table apart: skewed keys are often small numbers, whose slots would
 	// otherwise share a few cache lines (20M rows of Zipf(1.1) keys: 0.57 -> 0.48 ms; 2^27 skewed rows 3.0 -> 2.1 ms)
 	const std::string place = "(slot & 63u) * D64 + (slot >> 6)";
@@ -2294,7 +2301,24 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	const std::string chain_decl = "\tu64 *chain = (u64*)a.w[" + std::to_string(chain_word) + "];\n\tconst u64 ntiles = D / " +
 	                               fin_tile + ";\n";
 
-	const std::string tags = "((u32*)a.w[" + std::to_string(chain_word + 1) + "])";
+	const std::string tags = "((" + kt + "*)a.w[" + std::to_string(chain_word + 1) + "])";
+	const std::string table = "(u64*)a.w[" + std::to_string(chain_word + 2) + "]";  // hashed: the keys, ~0 = free
+	// adds `code` (which updates place `at`) for the key `slot`; a key that finds no place raises the flag beside
+	// the ticket
+	auto placed = [&](const std::string &code) {
+		if (!hashed) return "\t\tconst u64 at = " + place + ";\n" + code;
+		return "\t\tconst i64 at = vgpu_l2_place(K, D, slot);\n\t\tif (at < 0) { *vgpu_full = 1u; } else {\n" + code + "\t\t}\n";
+	};
+	if (hashed) {
+		// double hashing, 32 places at most: enough up to three fifths full (2^20 keys in 2^21 places leave none
+		// out), and a table that overflows says so after short waits
+		o << "__device__ __forceinline__ i64 vgpu_l2_place(u64 *K, u64 D, u64 key) {\n\tconst u64 h = mix64(key);\n"
+		  << "\tu64 s = h & (D - 1);\n\tconst u64 step = (h >> 32) | 1ull;\n"
+		  << "\t#pragma unroll 1\n\tfor (int i = 0; i < 32; ++i) {\n"
+		  << "\t\tconst u64 cur = ld_relaxed(K + s);\n\t\tif (cur == key) return (i64)s;\n"
+		  << "\t\tif (cur == ~0ull) {\n\t\t\tconst u64 prev = atomicCAS((unsigned long long*)(K + s), ~0ull, key);\n"
+		  << "\t\t\tif (prev == ~0ull || prev == key) return (i64)s;\n\t\t}\n\t\ts = (s + step) & (D - 1);\n\t}\n\treturn -1;\n}\n\n";
+	}
 	o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_gb_l2_init(KArgs a) {\n" << kKernelHead
 	  << "\tconst u64 D = a.w[" << cb << "];\n\t{\n" << chain_decl
 	  << "\tconst u64 t0 = blockIdx.x * (u64)blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;\n"
@@ -2304,28 +2328,30 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 		o << "\t\t((ulonglong2*)a.w[" << cb + 1 + f << "])[s] = make_ulonglong2(" << InitValue(fields[f]) << ", "
 		  << InitValue(fields[f]) << ");\n";
 	}
+	if (hashed) o << "\t\t((ulonglong2*)" << table << ")[s] = make_ulonglong2(~0ull, ~0ull);\n";
 	// the last CTA samples: groups of consecutive rows spread over the input, counted in a small hash table
 	o << "\t}\n\t}\n\tif (blockIdx.x != gridDim.x - 1) return;\n"
-	  << "\t__shared__ u64 claim[" << H << "];\n\t__shared__ u32 skey[" << kL2SampleRows << "], scount[" << kL2SampleRows << "];\n"
+	  << "\t__shared__ u64 claim[" << H << "];\n\t__shared__ " << kt << " skey[" << kL2SampleRows << "];\n\t__shared__ u32 scount[" << kL2SampleRows << "];\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") claim[i] = 0ull;\n"
-	  << "\tfor (u32 i = threadIdx.x; i < " << kL2SampleRows << "u; i += " << g.block << ") { skey[i] = ~0u; scount[i] = 0u; }\n"
+	  << "\tfor (u32 i = threadIdx.x; i < " << kL2SampleRows << "u; i += " << g.block << ") { skey[i] = ~(" << kt << ")0; scount[i] = 0u; }\n"
 	  << "\t__syncthreads();\n"
 	  << "\tif (n >= " << kL2SampleRows * 4 << "ull && threadIdx.x < " << kL2SampleRows / g.items << "u) {\n"
 	  << LoadBlock(g, needed, true,
 	               "(u64)threadIdx.x * (n / " + std::to_string(g.items) + ") / " + std::to_string(kL2SampleRows / g.items) + " * " +
 	                   std::to_string(g.items))
-	  << ItemOpen(g, needed) << chain_code_ << "\t\tif (keep) {\n\t\t\tconst u32 slot = (u32)" << pack.str() << ";\n"
-	  << "\t\t\tu32 p = (slot * 0x85ebca6bu) >> " << 32 - BitLength(kL2SampleRows - 1) << ";\n"
+	  << ItemOpen(g, needed) << chain_code_ << "\t\tif (keep) {\n\t\t\tconst " << kt << " slot = (" << kt << ")" << pack.str() << ";\n"
+	  << "\t\t\tu32 p = (" << fold << " * 0x85ebca6bu) >> " << 32 - BitLength(kL2SampleRows - 1) << ";\n"
 	  << "\t\t\t#pragma unroll 1\n\t\t\tfor (int i = 0; i < 8; ++i) {\n"
-	  << "\t\t\t\tconst u32 prev = atomicCAS(&skey[p], ~0u, slot);\n"
-	  << "\t\t\t\tif (prev == ~0u || prev == slot) { atomicAdd(&scount[p], 1u); break; }\n"
+	  << "\t\t\t\tconst " << kt << " prev = atomicCAS(&skey[p], ~(" << kt << ")0, slot);\n"
+	  << "\t\t\t\tif (prev == ~(" << kt << ")0 || prev == slot) { atomicAdd(&scount[p], 1u); break; }\n"
 	  << "\t\t\t\tp = (p + 1) & " << kL2SampleRows - 1 << "u;\n\t\t\t}\n\t\t}\n"
 	  << ItemClose() << "\t}\n\t__syncthreads();\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << kL2SampleRows << "u; i += " << g.block << ") {\n"
-	  << "\t\tconst u32 slot = skey[i];\n"
-	  << "\t\tif (scount[i] >= 2u) atomicMax((unsigned long long*)&claim[" << hash << "], ((u64)scount[i] << 32) | (slot + 1u));\n"
+	  << "\t\tconst " << kt << " slot = skey[i];\n"
+	  << "\t\tif (scount[i] >= 2u) atomicMax((unsigned long long*)&claim[" << hash << "], ((u64)scount[i] << 32) | (i + 1u));\n"
 	  << "\t}\n\t__syncthreads();\n"
-	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") " << tags << "[i] = (u32)claim[i];\n}\n\n";
+	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") " << tags
+	  << "[i] = (u32)claim[i] ? skey[(u32)claim[i] - 1u] + 1u : 0u;\n}\n\n";
 
 	o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_gb_l2(KArgs a) {\n" << kKernelHead
 	  << "\textern __shared__ __align__(16) u64 vgpu_smem[];\n";
@@ -2333,17 +2359,22 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 		o << "\tu64 *G" << f << " = (u64*)a.w[" << cb + 1 + f << "];\n"
 		  << "\tu64 *T" << f << " = vgpu_smem + " << f * H << ";\n";
 	}
-	o << "\t__shared__ u32 tag[" << H << "];\n\tconst u32 lane = threadIdx.x & 31; (void)lane;\n"
+	if (hashed) {
+		o << "\tu64 *K = " << table << ";\n\tconst u64 D = a.w[" << cb << "];\n\tvolatile u32 *vgpu_full = (volatile u32*)(" << "(u64*)a.w["
+		  << chain_word << "] + 1) + 1;\n";
+	}
+	o << "\t__shared__ " << kt << " tag[" << H << "];\n\tconst u32 lane = threadIdx.x & 31; (void)lane;\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") {\n"
-	  << "\t\ttag[i] = " << tags << "[i];\n\t\tif (tag[i] != 0u) {\n";
+	  << "\t\ttag[i] = " << tags << "[i];\n\t\tif (tag[i] != 0) {\n";
 	for (int f = 0; f < F; f++) o << "\t\t\tT" << f << "[i] = " << InitValue(fields[f]) << ";\n";
 	o << "\t\t}\n\t}\n\t__syncthreads();\n"
 	  << "\tconst u64 ntiles = (n + " << g.tile() - 1 << ") / " << g.tile() << ";\n"
-	  << "\tconst u64 D64 = a.w[" << cb << "] / 64;\n"
+	  << "\tconst u64 D64 = a.w[" << cb << "] / 64; (void)D64;\n"
 	  << "\tfor (u64 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {\n"
+	  << (hashed ? "\t\tif (__any_sync(0xffffffffu, *vgpu_full != 0u)) break;  // the caller takes another way\n" : "")
 	  << LoadBlock(g, needed) << ItemOpen(g, needed) << chain_code_ << "\t\tconst u64 slot = " << pack.str() << ";\n"
 	  << "\t\tconst u32 hp = " << hash << ";\n"
-	  << "\t\tconst bool hot = keep && tag[hp] == (u32)slot + 1u;\n";
+	  << "\t\tconst bool hot = keep && tag[hp] == (" << kt << ")slot + 1u;\n";
 	// one row's values, or the totals of a combined group
 	std::ostringstream own, tdecl, txor, ttake, upd;
 	own << "\t\tu32 gc = 1u;\n";
@@ -2386,7 +2417,8 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	o << own.str() << "\t\tbool lead = hot;\n";
 	if (!spec_.join_multi) {  // (a match list's items come lane by lane: nothing to combine)
 		o << "\t\tif (__popc(__ballot_sync(0xffffffffu, hot)) >= 8) {\n"
-		  << "\t\t\tconst u32 peers = __match_any_sync(0xffffffffu, hot ? (u32)slot : 0x80000000u | lane);\n"
+		  << "\t\t\tconst u32 peers = __match_any_sync(0xffffffffu, hot ? (" << kt << ")slot : "
+		  << (hashed ? "(1ull << 63)" : "0x80000000u") << " | lane);\n"
 		  << "\t\t\tfor (u32 todo = __ballot_sync(0xffffffffu, hot && __popc(peers) >= 4); todo;) {\n"
 		  << "\t\t\t\tconst u32 src_ = __ffs(todo) - 1;\n"
 		  << "\t\t\t\tconst u32 gmask = __shfl_sync(0xffffffffu, peers, src_);\n"
@@ -2396,17 +2428,18 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 		  << "\t\t\t\ttodo &= ~gmask;\n\t\t\t}\n\t\t}\n";
 	}
 	o << "\t\tif (hot) {\n\t\t\tif (lead) {\n" << upd.str() << "\t\t\t}\n\t\t} else if (keep) {\n"
-	  << "\t\tconst u64 at = " << place << ";\n" << UpdateCode(fields, "G", "at", values, false) << "\t\t}\n" << ItemClose() << "\t}\n"
+	  << placed(UpdateCode(fields, "G", "at", values, false)) << "\t\t}\n" << ItemClose() << "\t}\n"
 	  << "\t__syncthreads();\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") {\n"
-	  << "\t\tif (tag[i] != 0u && T0[i] != 0ull) {\n\t\t\tconst u64 slot = tag[i] - 1u, at = " << place << ";\n"
-	  << MergeCode(fields, "T", "i", "G", "at") << "\t\t}\n\t}\n}\n\n";
+	  << "\t\tif (tag[i] != 0 && T0[i] != 0ull) {\n\t\t\tconst u64 slot = tag[i] - 1u;\n"
+	  << placed(MergeCode(fields, "T", "i", "G", "at")) << "\t\t}\n\t}\n}\n\n";
 
 	// live slots in key order, finalized: tiles of kL2FinalTile slots, four per thread a quarter tile apart, so
 	// that the rows written are consecutive over a warp (2^22 slots of two words, SUM and COUNT: four consecutive
 	// slots per thread 0.093 ms, this 0.046 ms before the slots were spread)
 	static_assert(kL2FinalTile == 4 * 256, "the compaction's 32 (quarter, warp) counts fill one warp");
 	constexpr int quarter = kL2FinalTile / 4;
+	const int apart = hashed ? quarter : quarter / 64;  // places of one thread's four slots
 	o << "extern \"C\" __global__ void __launch_bounds__(" << kL2FinalTile / 4 << ") vgpu_gb_l2_final(KArgs a) {\n"
 	  << "\tconst u64 D = a.w[" << cb << "];\n" << chain_decl
 	  << "\tu32 *counts = (u32*)(chain + 2);\n\tu64 *starts = chain + 2 + (ntiles + 1) / 2;\n";
@@ -2420,9 +2453,10 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	  << "\t\tif (threadIdx.x == 0) atomicAdd(chain, t_ == ~0ull ? 1ull << 63 : t_);\n\t\treturn;\n\t}\n"
 	  << "\tfor (u64 tile = (u64)vgpu_next - 1; tile < ntiles;) {\n"
 	  << "\t\tconst u64 s0 = tile * " << fin_tile << "ull + threadIdx.x;\n"
-	  << "\t\t// slot s0 + 256 r is at p0 + 4 r (see above)\n\t\tconst u64 p0 = (s0 & 63u) * (D / 64) + (s0 >> 6);\n"
+	  << (hashed ? "\t\tconst u64 p0 = s0;\n"
+	             : "\t\t// slot s0 + 256 r is at p0 + 4 r (see above)\n\t\tconst u64 p0 = (s0 & 63u) * (D / 64) + (s0 >> 6);\n")
 	  << "\t\tu32 live[4];  // the warp's live lanes in each quarter\n"
-	  << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < 4; ++r) live[r] = __ballot_sync(0xffffffffu, G0[p0 + " << quarter / 64
+	  << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < 4; ++r) live[r] = __ballot_sync(0xffffffffu, G0[p0 + " << apart
 	  << " * r] != 0ull);\n"
 	  << "\t\tif (lane < 4u) vgpu_warps[lane * " << quarter / 32 << " + (threadIdx.x >> 5)] = __popc(lane == 0 ? live[0] : lane == 1 ? live[1] "
 	     ": lane == 2 ? live[2] : live[3]);\n"
@@ -2437,7 +2471,8 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	  << "\t\t\t\tif (b_ == ~0ull) atomicOr(chain, 1ull << 63);\n\t\t\t\tvgpu_base = b_;\n\t\t\t\tvgpu_next = next_;\n\t\t\t}\n\t\t}\n"
 	  << "\t\t__syncthreads();\n\t\tif (vgpu_base == ~0ull) return;\n"
 	  << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < 4; ++r) {\n\t\t\tif (!((live[r] >> lane) & 1u)) continue;\n"
-	  << "\t\t\tconst u64 key = s0 + " << quarter << "ull * r, at = p0 + " << quarter / 64 << "ull * r;\n"
+	  << "\t\t\tconst u64 at = p0 + " << apart << "ull * r;\n\t\t\tconst u64 key = "
+	  << (hashed ? "(" + table + ")[at]" : "s0 + " + std::to_string(quarter) + "ull * r") << ";\n"
 	  << "\t\t\tconst u64 pos = vgpu_base + vgpu_warps[r * " << quarter / 32 << " + (threadIdx.x >> 5)] + __popc(live[r] & ((1u << lane) - 1u));\n"
 	  << FinalizeCode(gb, fields, visible_, "G", "at", "key", "pos", cb + 1 + F)
 	  << "\t\t}\n\t\tconst u64 after_ = (u64)vgpu_next - 1;\n\t\t__syncthreads();  // the shared words have been read\n"

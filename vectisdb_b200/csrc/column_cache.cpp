@@ -258,11 +258,12 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		}
 		done.emplace_back(kv.first, std::move(e));
 	}
-	// the integer columns' ranges: one launch and one read-back for the table
-	std::vector<uint64_t> bounds(2 * ranged.size());
+	// the integer columns' ranges and distinct counts: one launch and one read-back for the table
+	const int columns = static_cast<int>(ranged.size());
+	std::vector<uint64_t> bounds(kern::BoundsWords(columns, true));
 	if (!ranged.empty()) {
 		uint64_t *mm = static_cast<uint64_t *>(alloc.Alloc(bounds.size() * 8, s));
-		kern::ColumnBounds(ranged.data(), static_cast<int>(ranged.size()), mm, s);
+		kern::ColumnBounds(ranged.data(), columns, mm, s, true);
 		VGPU_CUDA(cudaMemcpyAsync(bounds.data(), mm, bounds.size() * 8, cudaMemcpyDeviceToHost, s));
 		VGPU_CUDA(cudaStreamSynchronize(s));
 		alloc.Free(mm, s);
@@ -272,12 +273,14 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		Entry &e = named.second;
 		if (IsIntegerKeyType(e.column.type) || e.column.type == ValueType::DICTIONARY_STRING) {
 			const uint64_t *words = &bounds[2 * next];
-			const kern::BoundsKind kind = ranged[next++].kind;
+			const kern::BoundsKind kind = ranged[next].kind;
 			if (e.column.rows > 0) {
+				e.column.distinct = kern::DistinctEstimate(bounds.data(), columns, static_cast<int>(next), kind);
 				e.column.has_stats = true;
 				e.column.min = static_cast<int64_t>(kern::BoundsLow(words, kind));
 				e.column.max = static_cast<int64_t>(kern::BoundsHigh(words, kind));
 			}
+			next++;
 		}
 		const std::string key = Key(table, named.first);
 		const bool replaced = entries_.count(key) != 0;

@@ -2,6 +2,7 @@
 #include "kernels.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <limits>
 #include <type_traits>
@@ -207,17 +208,38 @@ template <typename T> __global__ void WidenKernel(const T *src, uint64_t n, uint
 // unsigned image (signed values with the sign bit flipped); the minimum is kept as the maximum of the
 // complemented image, so one zero fill is the identity of both.
 
+//
+// With `ranks`, also an estimate of each column's distinct values (HyperLogLog: of the hashes that share their
+// low 8 bits, the most leading zeros in the rest) over one value in 1024, as a cheap hash picks them: a
+// multiplication per value, and the rest for one warp step in thirty (8M INT64 values 0.028 -> 0.029 ms; every value
+// taken, or one in eight, which is nearly every step of a warp: 0.041 ms).
+constexpr int kDistinctShift = 10;
+
 struct BoundsArgs {
 	BoundsColumn c[kMaxBoundsColumns];
 	unsigned long long *out;
+	unsigned int *ranks;  // kDistinctRanks per column, or null
 };
 
+// Out of line: few values come here, and the kernel's eight unrolled readers stay small.
+__device__ __noinline__ void NoteValue(u64 v, uint32_t *ranks) {
+	const u64 h = mix64(v);
+	const uint32_t rank = static_cast<uint32_t>(__clzll(static_cast<long long>(h | (kDistinctRanks - 1)))) + 1u;
+	uint32_t *r = ranks + (h & (kDistinctRanks - 1));
+	if (*reinterpret_cast<volatile uint32_t *>(r) < rank) atomicMax(r, rank);
+}
+
 template <typename T, bool kBool>
-__device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx) {
+__device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx, uint32_t *ranks) {
 	auto take = [&](T v) {
 		if constexpr (kBool) v = v != 0 ? 1 : 0;
 		mn = v < mn ? v : mn;
 		mx = v > mx ? v : mx;
+		if constexpr (sizeof(T) >= 4) {
+			u32 w = static_cast<u32>(v);
+			if constexpr (sizeof(T) == 8) w ^= static_cast<u32>(static_cast<u64>(v) >> 32);
+			if (w * 0x9e3779b1u < (1u << (32 - kDistinctShift)) && ranks) NoteValue(static_cast<u64>(v), ranks);
+		}
 	};
 	constexpr uint64_t kPer = 16 / sizeof(T);
 	const uint64_t skew = reinterpret_cast<uintptr_t>(p) & 15u;
@@ -247,9 +269,10 @@ __device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx) {
 }
 
 template <typename T, bool kBool = false>
-__device__ __forceinline__ void RangeImage(const void *p, uint64_t n, unsigned long long &lo, unsigned long long &hi) {
+__device__ __forceinline__ void RangeImage(const void *p, uint64_t n, unsigned long long &lo, unsigned long long &hi,
+                                           uint32_t *ranks) {
 	T mn = std::numeric_limits<T>::max(), mx = std::numeric_limits<T>::lowest();
-	RangeOf<T, kBool>(static_cast<const T *>(p), n, mn, mx);
+	RangeOf<T, kBool>(static_cast<const T *>(p), n, mn, mx, ranks);
 	constexpr unsigned long long kFlip = std::is_signed<T>::value ? 1ull << 63 : 0ull;
 	const bool any = mn <= mx;  // a thread without values leaves the identity
 	lo = any ? static_cast<unsigned long long>(mn) ^ kFlip : ~0ull;
@@ -261,15 +284,20 @@ constexpr int kBoundsBlock = 256;
 __global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a) {
 	const BoundsColumn &c = a.c[blockIdx.y];
 	unsigned long long lo = ~0ull, hi = 0ull;
+	__shared__ uint32_t shared_ranks[kDistinctRanks];
+	static_assert(kDistinctRanks == kBoundsBlock, "one rank per thread");
+	shared_ranks[threadIdx.x] = 0;
+	uint32_t *ranks = a.ranks ? shared_ranks : nullptr;
+	__syncthreads();
 	switch (c.kind) {
-	case BoundsKind::U8: RangeImage<uint8_t>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::U16: RangeImage<uint16_t>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::U32: RangeImage<uint32_t>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::U64: RangeImage<unsigned long long>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::I16: RangeImage<int16_t>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::I32: RangeImage<int32_t>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::I64: RangeImage<long long>(c.data, c.rows, lo, hi); break;
-	case BoundsKind::BOOL: RangeImage<uint8_t, true>(c.data, c.rows, lo, hi); break;
+	case BoundsKind::U8: RangeImage<uint8_t>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::U16: RangeImage<uint16_t>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::U32: RangeImage<uint32_t>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::U64: RangeImage<unsigned long long>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::I16: RangeImage<int16_t>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::I32: RangeImage<int32_t>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::I64: RangeImage<long long>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::BOOL: RangeImage<uint8_t, true>(c.data, c.rows, lo, hi, ranks); break;
 	}
 	__shared__ unsigned long long slo[kBoundsBlock / 32], shi[kBoundsBlock / 32];
 	for (int o = 16; o > 0; o >>= 1) {
@@ -289,6 +317,13 @@ __global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a)
 		}
 		atomicMax(a.out + 2 * blockIdx.y, ~lo);
 		atomicMax(a.out + 2 * blockIdx.y + 1, hi);
+	}
+	if (a.ranks) {  // (the values were all taken before the barrier above)
+		// few CTAs raise a rank the others have raised before: looked at first (a thousand CTAs' atomics on the
+		// same eight lines took 20 us)
+		unsigned int *to = a.ranks + blockIdx.y * kDistinctRanks + threadIdx.x;
+		const uint32_t r = shared_ranks[threadIdx.x];
+		if (r != 0 && r > __ldcg(to)) atomicMax(to, r);
 	}
 }
 
@@ -1020,9 +1055,10 @@ void JoinDenseFill(const void *keys, size_t kwidth, const void *values, size_t v
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream) {
+void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream, bool distinct) {
 	if (n <= 0) return;
-	VGPU_CUDA(cudaMemsetAsync(out, 0, static_cast<size_t>(n) * 16, stream));
+	VGPU_CUDA(cudaMemsetAsync(out, 0, BoundsWords(n, distinct) * 8, stream));
+	unsigned int *ranks = distinct ? reinterpret_cast<unsigned int *>(out + 2 * n) : nullptr;
 	for (int first = 0; first < n; first += kMaxBoundsColumns) {
 		BoundsArgs a;
 		const int count = std::min(n - first, kMaxBoundsColumns);
@@ -1036,6 +1072,7 @@ void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t s
 		}
 		if (widest == 0) continue;
 		a.out = reinterpret_cast<unsigned long long *>(out + 2 * first);
+		a.ranks = ranks ? ranks + static_cast<size_t>(first) * kDistinctRanks : nullptr;
 		LaunchScope scope("column_bounds", stream, bytes, rows);
 		// four 16-byte loads per thread, at most eight CTAs per SM over all columns
 		const uint64_t cap = std::max<uint64_t>(1, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8 / count);
@@ -1043,6 +1080,20 @@ void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t s
 		ColumnBoundsKernel<<<dim3(grid, static_cast<unsigned>(count)), kBoundsBlock, 0, stream>>>(a);
 		VGPU_CUDA(cudaGetLastError());
 	}
+}
+
+uint64_t DistinctEstimate(const uint64_t *words, int n, int column, BoundsKind kind) {
+	if (BoundsWidth(kind) < 4) return 0;
+	const uint32_t *ranks = reinterpret_cast<const uint32_t *>(words + 2 * n) + static_cast<size_t>(column) * kDistinctRanks;
+	double sum = 0;
+	int empty = 0;
+	for (int i = 0; i < kDistinctRanks; i++) {
+		sum += std::ldexp(1.0, -static_cast<int>(ranks[i]));
+		empty += ranks[i] == 0;
+	}
+	const double m = kDistinctRanks, raw = 0.7213 / (1 + 1.079 / m) * m * m / sum;
+	const double picked = raw <= 2.5 * m && empty ? m * std::log(m / empty) : raw;
+	return static_cast<uint64_t>(picked * (1 << kDistinctShift)) + 1;
 }
 
 BoundsKind SignedBoundsKind(ValueType t) {

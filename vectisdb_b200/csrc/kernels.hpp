@@ -54,7 +54,15 @@ BoundsKind SignedBoundsKind(ValueType t);
 //! Smallest and largest value of each of `n` columns, one launch per kMaxBoundsColumns of them: two words
 //! per column in `out` (device, 2n words), read back with BoundsLow / BoundsHigh. A column without rows
 //! gives the largest value of its 64-bit kind as the smallest and the other way round.
-void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream);
+//! With `distinct`, kDistinctRanks 32-bit ranks per column follow in `out` (BoundsWords in all), from which
+//! DistinctEstimate (on the words read back) gives about how many distinct values a 4- or 8-byte column has
+//! (within some 7%; 0 for narrower ones).
+void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream, bool distinct = false);
+constexpr int kDistinctRanks = 256;
+inline size_t BoundsWords(int n, bool distinct) {
+	return static_cast<size_t>(n) * (2 + (distinct ? kDistinctRanks / 2 : 0));
+}
+uint64_t DistinctEstimate(const uint64_t *words, int n, int column, BoundsKind kind);
 inline bool BoundsSigned(BoundsKind k) {
 	return k == BoundsKind::I16 || k == BoundsKind::I32 || k == BoundsKind::I64;
 }
