@@ -794,6 +794,8 @@ struct Field {
 	// One-pass group-by, MIN/MAX in shared memory: >= 0 keeps the value as a 32-bit offset from the
 	// minimum in argument word `narrow_word` (the low word of the slot, updated by native 32-bit atomics).
 	int narrow_word = -1;
+	// One-pass group-by, an FP64 sum in shared memory that stands for the count too (see f64_presence).
+	bool presence = false;
 };
 
 std::vector<Field> StateFields(const PipelineCodegen::GroupBySpec &gb) {
@@ -838,6 +840,9 @@ int FieldIndex(const std::vector<Field> &fields, const std::string &kind, int ag
 }
 
 std::string InitValue(const Field &f) {
+	if (f.presence) {
+		return "0x8000000000000000ull";  // -0.0
+	}
 	if (f.narrow_word >= 0) {
 		return f.kind == "min" ? "0xffffffffull" : "0ull";
 	}
@@ -859,9 +864,16 @@ std::string UpdateCode(const std::vector<Field> &fields, const std::string &tab,
                        const std::vector<std::string> &agg_values, bool shared, bool narrow_count = false,
                        bool count_as_flag = false) {
 	std::ostringstream o;
+	bool presence = false;
+	for (auto &f : fields) presence = presence || f.presence;
 	for (size_t i = 0; i < fields.size(); i++) {
 		auto &f = fields[i];
 		std::string p = tab + std::to_string(i) + " + " + slot;
+		if (f.kind == "cnt" && presence) continue;
+		if (f.presence) {
+			o << "\t\t\tatomicAdd((double*)(" << p << "), (double)(" << agg_values[f.agg] << ") + 0.0);\n";
+			continue;
+		}
 		if ((f.kind == "min" || f.kind == "max") && shared && f.narrow_word >= 0) {
 			o << "\t\t\tatomic" << (f.kind == "min" ? "Min" : "Max") << "((u32*)(" << p << "), (u32)((i64)("
 			  << agg_values[f.agg] << ") - (i64)a.w[" << f.narrow_word << "]));\n";
@@ -895,9 +907,12 @@ std::string UpdateCode(const std::vector<Field> &fields, const std::string &tab,
 std::string MergeCode(const std::vector<Field> &fields, const std::string &src, const std::string &ss,
                       const std::string &dst, const std::string &ds, bool l2_src = false) {
 	std::ostringstream o;
+	bool presence = false;
+	for (auto &f : fields) presence = presence || f.presence;
 	for (size_t i = 0; i < fields.size(); i++) {
 		auto &f = fields[i];
 		std::string ps = src + std::to_string(i) + "[" + ss + "]";
+		if (f.kind == "cnt" && presence) ps = "1ull";
 		if (l2_src && f.kind == "f64") ps = "__ldcg(&" + ps + ")";
 		std::string pd = dst + std::to_string(i) + " + " + ds;
 		if (f.kind == "cnt" || f.kind == "s64") {
@@ -1005,6 +1020,7 @@ int PipelineCodegen::DirectSlotBytes(const GroupBySpec &gb) {
 uint64_t PipelineCodegen::DirectSmemBytes(const GroupBySpec &gb, uint64_t domain) {
 	const int F = static_cast<int>(StateFields(gb).size());
 	const int shared64 = F - 1 - (gb.f64_l2 ? F64Fields(gb) : 0);
+	if (gb.f64_presence) return domain * static_cast<uint64_t>(shared64) * 8;
 	const bool c32 = gb.count32 && (gb.narrow_count || gb.count_as_flag);
 	return domain * (static_cast<uint64_t>(shared64) * 8 + (c32 ? 4 : 8));
 }
@@ -1124,6 +1140,12 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		for (auto &f : dfields) {
 			if (f.kind == "min" || f.kind == "max") f.narrow_word = gb.aggs[f.agg].narrow_word;
 		}
+		int marker = 0;  // the field that says whether a slot has rows
+		if (gb.f64_presence) {
+			while (marker < F && dfields[marker].kind != "f64") marker++;
+			if (marker == F || gb.f64_l2 || !gb.count_as_flag) Fail(VGPU_ERR_INTERNAL, "no FP64 sum to mark groups with");
+			dfields[marker].presence = true;
+		}
 		o << "extern \"C\" __global__ void vgpu_gb_direct_init(KArgs a) {\n"
 		  << "\tconst u64 D = a.w[" << cb << "];\n";
 		if (fused) o << "\tif (blockIdx.x == 0 && threadIdx.x == 0) *(u32*)a.w[" << ticket << "] = 0u;\n";
@@ -1139,29 +1161,35 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		const int nl2 = l2 ? F64Fields(gb) : 0;
 		o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_gb_direct(KArgs a) {\n"
 		  << kKernelHead << "\textern __shared__ __align__(16) u64 vgpu_smem[];\n"
-		  << "\tconst u64 D = a.w[" << cb << "];\n";
+		  << "\tconst u64 D = a.w[" << cb << "];\n"
+		  // Copies of every slot, side by side, that the lanes of a warp share out among themselves: rows of one
+		  // group that meet in a warp then update different words (64M rows into 50 groups 0.312 -> 0.220 ms, 5.8 TB/s;
+		  // into 300 groups 0.249 -> 0.236).
+		  << "\tconst u32 copies = (u32)a.w[" << kCopiesWord << "], copies_log = 31u - __clz(copies);\n"
+		  << "\tconst u32 copy = threadIdx.x & (copies - 1u);\n\tconst u64 DC = D * copies;\n";
 		// A count that never carries (fewer than 2^32 rows) or only marks presence needs 32 bits: with
 		// count32 its array goes after the 64-bit ones, in 4 bytes per slot (DirectSmemBytes sizes the
 		// launch alike).
 		const bool c32 = gb.count32 && (gb.narrow_count || gb.count_as_flag);
 		int sh = 0;
 		for (int f = 0, gl = 0; f < F; f++) {
+			if (f == 0 && marker != 0) continue;  // no count table
 			if (l2 && fields[f].kind == "f64") {
 				o << "\tu64 *T" << f << " = (u64*)a.w[" << cb + 2 + F + out_words << "] + ((u64)blockIdx.x * " << nl2
-				  << " + " << gl++ << ") * D;\n";
+				  << " + " << gl++ << ") * DC;\n";
 			} else if (!(c32 && f == 0)) {
-				o << "\tu64 *T" << f << " = vgpu_smem + " << sh++ << " * D;\n";
+				o << "\tu64 *T" << f << " = vgpu_smem + " << sh++ << " * DC;\n";
 			}
 		}
-		if (c32) o << "\tu32 *T0 = (u32*)(vgpu_smem + " << sh << " * D);\n";
-		o << "\tfor (u64 s = threadIdx.x; s < D; s += " << g.block << ") {\n";
-		for (int f = 0; f < F; f++) {
+		if (c32 && marker == 0) o << "\tu32 *T0 = (u32*)(vgpu_smem + " << sh << " * DC);\n";
+		o << "\tfor (u64 s = threadIdx.x; s < DC; s += " << g.block << ") {\n";
+		for (int f = marker != 0 ? 1 : 0; f < F; f++) {
 			o << "\t\tT" << f << "[s] = " << InitValue(dfields[f]) << ";\n";
 		}
 		o << "\t}\n\t__syncthreads();\n" << tile_loop_head
 		  << "\tfor (u64 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {\n"
 		  << LoadBlock(g, needed) << ItemOpen(g, needed) << chain_code_ << "\t\tif (keep) {\n"
-		  << "\t\t\tconst u64 slot = " << pack.str() << ";\n"
+		  << "\t\t\tconst u64 slot = ((" << pack.str() << ") << copies_log) + copy;\n"
 		  << UpdateCode(dfields, "T", "slot", pipe_values, true, gb.narrow_count, gb.count_as_flag) << "\t\t}\n" << ItemClose()
 		  << "\t}\n"
 		  << (l2 ? "\t__threadfence();  // this thread's reductions are performed before the sums are read\n" : "")
@@ -1169,8 +1197,33 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		for (int f = 0; f < F; f++) {
 			o << "\tu64 *G" << f << " = (u64*)a.w[" << cb + 1 + f << "];\n";
 		}
-		o << "\tfor (u64 s = threadIdx.x; s < D; s += " << g.block << ") {\n\t\tif (T0[s] != 0) {\n"
-		  << MergeCode(dfields, "T", "s", "G", "s", l2) << "\t\t}\n\t}\n";
+		// a slot's copies are added up here, so the global tables see one update per CTA and group
+		o << "\tfor (u64 s = threadIdx.x; s < D; s += " << g.block << ") {\n";
+		for (int f = marker != 0 ? 1 : 0; f < F; f++) {
+			const std::string t = "T" + std::to_string(f) + "[(s << copies_log)]";
+			o << "\t\tu64 S" << f << "[1] = {" << (l2 && fields[f].kind == "f64" ? "__ldcg(&" + t + ")" : t) << "};\n";
+		}
+		o << "\t\tfor (u32 c = 1; c < copies; ++c) {\n\t\t\tconst u64 sc = (s << copies_log) + c;\n";
+		for (int f = marker != 0 ? 1 : 0; f < F; f++) {
+			const auto &fd = dfields[f];
+			const std::string S = "S" + std::to_string(f) + "[0]", T = "T" + std::to_string(f) + "[sc]";
+			if (fd.kind == "cnt") {
+				// a presence flag or 32-bit counts that cannot carry (copies are only taken then)
+				o << "\t\t\t" << S << " += " << T << ";\n";
+			} else if (fd.kind == "f64") {
+				o << "\t\t\t" << S << " = (u64)__double_as_longlong(__longlong_as_double((i64)" << S << ") + __longlong_as_double((i64)"
+				  << T << "));\n";
+			} else if (fd.kind == "lo") {
+				const std::string S1 = "S" + std::to_string(f + 1) + "[0]", T1 = "T" + std::to_string(f + 1) + "[sc]";
+				o << "\t\t\t" << S << " += " << T << "; " << S1 << " += " << T1 << " + (" << S << " < " << T << " ? 1ull : 0ull);\n";
+			} else if (fd.kind == "min" || fd.kind == "max") {
+				const char *op = fd.kind == "min" ? "<" : ">";
+				const std::string as = fd.narrow_word >= 0 ? "(u32)" : "(i64)";
+				o << "\t\t\tif (" << as << T << " " << op << " " << as << S << ") " << S << " = " << T << ";\n";
+			}
+		}
+		o << "\t\t}\n\t\tif (S" << marker << "[0] != " << (marker ? InitValue(dfields[marker]) : "0") << ") {\n"
+		  << MergeCode(dfields, "S", "0", "G", "s") << "\t\t}\n\t}\n";
 		// final: one CTA compacts the non-empty groups in key order. Fused, it is the CTA whose merge
 		// finished last: every thread fences its merge atomics before the CTA takes a ticket, and the
 		// last CTA fences again before reading the global tables (which no CTA has loaded through L1:
@@ -1190,14 +1243,27 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 				o << "\tconst u64 *G" << f << " = (const u64*)a.w[" << cb + 1 + f << "];\n";
 			}
 		}
-		o << "\tu64 base = 0;\n"
-		  << "\tfor (u64 c0 = 0; c0 < D; c0 += blockDim.x) {\n"
-		  << "\t\tconst u64 s = c0 + threadIdx.x;\n"
+		// Two passes over the slots without a barrier in either, so that their loads overlap (one scan per
+		// blockDim slots between loads and writes instead: 2M probe rows into 4096 groups 0.040 ms, this 0.037): live slots per warp and chunk, a scan
+		// of those counts, the rows.
+		o << "\t__shared__ u32 vgpu_wc[512];  // at most 2^13 * 1.5 slots: a count per 32 of them, rounded up to whole chunks\n"
+		  << "\tconst u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;\n"
+		  << "\tconst u32 chunks = (u32)((D + blockDim.x - 1) / blockDim.x), ncounts = chunks * nw;\n"
+		  << "\t#pragma unroll 4\n\tfor (u32 c = 0; c < chunks; ++c) {\n"
+		  << "\t\tconst u64 s = (u64)c * blockDim.x + threadIdx.x;\n"
+		  << "\t\tconst u32 b = __ballot_sync(0xffffffffu, s < D && G0[s] != 0);\n"
+		  << "\t\tif (lane == 0) vgpu_wc[c * nw + warp] = __popc(b);\n\t}\n\t__syncthreads();\n"
+		  << "\tu32 base = 0;\n"
+		  << "\tfor (u32 c0 = 0; c0 < ncounts; c0 += blockDim.x) {\n"
+		  << "\t\tconst u32 i = c0 + threadIdx.x;\n"
+		  << "\t\tu32 total; const u32 before = block_exclusive_scan(i < ncounts ? vgpu_wc[i] : 0u, scan_scratch, &total);\n"
+		  << "\t\tif (i < ncounts) vgpu_wc[i] = base + before;\n\t\tbase += total;\n\t}\n\t__syncthreads();\n"
+		  << "\t#pragma unroll 2\n\tfor (u32 c = 0; c < chunks; ++c) {\n"
+		  << "\t\tconst u64 s = (u64)c * blockDim.x + threadIdx.x;\n"
 		  << "\t\tconst bool live = s < D && G0[s] != 0;\n"
-		  << "\t\tu32 total; const u32 off = block_exclusive_scan(live ? 1u : 0u, scan_scratch, &total);\n"
-		  << "\t\tif (live) {\n\t\t\tconst u64 pos = base + off;\n\t\t\tconst u64 key = s;\n"
-		  << FinalizeCode(gb, fields, visible_, "G", "s", "key", "pos", cb + 1 + F) << "\t\t}\n"
-		  << "\t\tbase += total;\n\t}\n"
+		  << "\t\tconst u32 b = __ballot_sync(0xffffffffu, live);\n"
+		  << "\t\tif (live) {\n\t\t\tconst u64 pos = vgpu_wc[c * nw + warp] + __popc(b & ((1u << lane) - 1u));\n\t\t\tconst u64 key = s;\n"
+		  << FinalizeCode(gb, fields, visible_, "G", "s", "key", "pos", cb + 1 + F) << "\t\t}\n\t}\n"
 		  << "\tif (threadIdx.x == 0) *(u64*)a.w[" << cb + 1 + F + out_words << "] = base;\n}\n";
 		return o.str();
 	}
@@ -2664,7 +2730,7 @@ std::string GroupByKey(const PipelineCodegen::GroupBySpec &gb, bool partitioned)
 		o << static_cast<int>(a.kind) << '/' << a.column << '/' << static_cast<int>(a.input_type) << '/'
 		  << static_cast<int>(a.output_type) << '/' << a.narrow_word << '/' << a.sum64 << ';';
 	}
-	o << "|db:" << gb.direct_bits << "|bt:" << gb.bucket_threads << "|hv:" << gb.heavy_slots << "|f64l2:" << gb.f64_l2 << "|hw:" << gb.heavy_warp << "|bp:" << gb.bucket_plain << "|nc:" << gb.narrow_count << "|cf:" << gb.count_as_flag << "|c32:" << gb.count32;
+	o << "|db:" << gb.direct_bits << "|bt:" << gb.bucket_threads << "|hv:" << gb.heavy_slots << "|f64l2:" << gb.f64_l2 << "|hw:" << gb.heavy_warp << "|bp:" << gb.bucket_plain << "|nc:" << gb.narrow_count << "|cf:" << gb.count_as_flag << "|c32:" << gb.count32 << "|fp:" << gb.f64_presence;
 	return o.str();
 }
 

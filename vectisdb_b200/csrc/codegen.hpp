@@ -78,6 +78,8 @@ struct Geometry {
 constexpr int kKeyWord = 96;
 constexpr int kMaxPackedKeys = 8;
 constexpr int kMixWord = 120;
+// One-pass group-by (which does not mix): copies of every shared-memory slot, a power of two.
+constexpr int kCopiesWord = kMixWord;
 // Join-source words: [kJoinWord] sorted right keys (u64, biased), [+1] radix directory (u32),
 // [+2] bias (the right minimum), [+3] shift | bucket count << 8.
 constexpr int kJoinWord = 123;
@@ -166,6 +168,9 @@ public:
 		// One-pass group-by: no aggregate reads the row count (no COUNT, no AVG), so the count word only
 		// marks a group as present -- a plain store of 1, not an atomic add.
 		bool count_as_flag = false;
+		// One-pass group-by without a count to keep (count_as_flag) but with an FP64 sum in shared memory: the
+		// first such sum marks the group as present by not being -0.0, which no sum of values with +0.0 added is.
+		bool f64_presence = false;
 		// One-pass group-by: the count (narrow or a flag) takes 4 bytes per slot in shared memory instead
 		// of 8 (the tables shrink, more CTAs fit on an SM).
 		bool count32 = false;

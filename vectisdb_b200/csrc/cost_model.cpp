@@ -473,9 +473,12 @@ std::string GenerateSourceText(const PlanNode &plan, const std::vector<vgpu_colu
 	Geometry gst = g;
 	gst.items = 4;
 	gst.staged = true;
+	PipelineCodegen::GroupBySpec spec_fp = spec_gb;  // ... and an FP64 sum that marks its groups
+	spec_fp.count_as_flag = true;
+	spec_fp.f64_presence = PipelineCodegen::F64Fields(spec_fp) > 0;
 	// Separate translation units, separated by a marker line: direct, partitioned, key statistics,
 	// direct-partitioned, direct-partitioned with heavy keys, the last two staged, the plain bucket pass,
-	// the direct one with narrow counts and MIN/MAX, and the table held in L2, dense and hashed.
+	// the direct one with narrow counts and MIN/MAX and with groups marked by a sum, and the table held in L2, dense and hashed.
 	Geometry gl = g;
 	gl.items = 4;
 	return cg.EmitGroupBy(spec_gb, false, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_gb, true, g) +
@@ -483,7 +486,7 @@ std::string GenerateSourceText(const PlanNode &plan, const std::vector<vgpu_colu
 	       cg.EmitGroupBy(spec_dp, true, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_hv, true, g) +
 	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_dp, true, gst) + "\n//@@VGPU_TU@@\n" +
 	       cg.EmitGroupBy(spec_hv, true, gst) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_plain, true, g) +
-	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_nc, false, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupByL2(spec_gb, gl) +
+	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_nc, false, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupBy(spec_fp, false, g) + "\n//@@VGPU_TU@@\n" + cg.EmitGroupByL2(spec_gb, gl) +
 	       "\n//@@VGPU_TU@@\n" + cg.EmitGroupByL2(spec_gb, gl, true);
 }
 

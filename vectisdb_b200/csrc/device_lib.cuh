@@ -102,29 +102,35 @@ __device__ __forceinline__ void load_rows(const T *__restrict__ base, u64 row0, 
 	constexpr int BYTES = (int)sizeof(T) * R;
 	const T *p = base + row0;
 	const u64 addr = (u64)p;
-	if (row0 + R <= n && (BYTES % 16 == 0) && (addr & 15ull) == 0) {
-		u32 words[BYTES / 4];
+	if constexpr (BYTES % 4 == 0) {
+		// the widest access that the rows' bytes fill: 16, 8 or 4
+		constexpr int W = BYTES % 16 == 0 ? 16 : BYTES % 8 == 0 ? 8 : 4;
+		if (row0 + R <= n && (addr & (W - 1)) == 0) {
+			u32 words[BYTES / 4];
 #pragma unroll
-		for (int q = 0; q < BYTES / 16; ++q) {
-			uint4 v = ld_stream_v4(reinterpret_cast<const char *>(p) + 16 * q);
-			words[4 * q + 0] = v.x;
-			words[4 * q + 1] = v.y;
-			words[4 * q + 2] = v.z;
-			words[4 * q + 3] = v.w;
+			for (int q = 0; q < BYTES / W; ++q) {
+				const char *at = reinterpret_cast<const char *>(p) + W * q;
+				if constexpr (W == 16) {
+					const uint4 v = ld_stream_v4(at);
+					words[4 * q + 0] = v.x;
+					words[4 * q + 1] = v.y;
+					words[4 * q + 2] = v.z;
+					words[4 * q + 3] = v.w;
+				} else if constexpr (W == 8) {
+					const uint2 v = ld_stream_v2(at);
+					words[2 * q + 0] = v.x;
+					words[2 * q + 1] = v.y;
+				} else {
+					words[q] = ld_stream_u32(at);
+				}
+			}
+#pragma unroll
+			for (int r = 0; r < R; ++r) out[r] = word_element<T>(words, r);
+			return;
 		}
-#pragma unroll
-		for (int r = 0; r < R; ++r) out[r] = word_element<T>(words, r);
-	} else if (row0 + R <= n && BYTES == 8 && (addr & 7ull) == 0) {
-		u32 words[2];
-		uint2 v = ld_stream_v2(p);
-		words[0] = v.x;
-		words[1] = v.y;
-#pragma unroll
-		for (int r = 0; r < R; ++r) out[r] = word_element<T>(words, r);
-	} else {
-#pragma unroll
-		for (int r = 0; r < R; ++r) out[r] = (row0 + r < n) ? ld_scalar(p + r) : T();
 	}
+#pragma unroll
+	for (int r = 0; r < R; ++r) out[r] = (row0 + r < n) ? ld_scalar(p + r) : T();
 }
 
 // ---------------------------------------------------------------------------------------------

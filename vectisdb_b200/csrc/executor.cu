@@ -1054,6 +1054,9 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		// cost more than they hide (a 2^28-row probe into 4096 groups: 1.45 -> 1.51 ms)
 		gb.count32 = pin.spec.join_multi;
 		gb.f64_l2 = direct_l2;
+		// A sum of doubles tells a group with rows from one without by itself: no store per row for that, and tables
+		// of half the size over 4096 groups, so the threads of an SM are all in use (2^28 probe rows 1.47 -> 1.45 ms by itself).
+		gb.f64_presence = gb.count_as_flag && !direct_l2 && direct_f64 > 0;
 		// MIN/MAX over a cached integer column whose values span less than 2^32: the shared tables hold
 		// 32-bit offsets from the column's minimum (native 32-bit atomics on the slot's low word instead
 		// of 64-bit ones), the minimum in an argument word after the compaction ticket.
@@ -1080,7 +1083,12 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		}
 		Geometry g;
 		g.block = 512;
-		g.items = 4;  // also for a join source (a fused 2^28-row probe: 4 rows per thread 1.68 ms, 8 1.71 ms)
+		// a join's probe keeps fewer rows per thread, and so more of its random table reads apart from the shared
+		// updates that follow them (a fused 2^28-row probe: 1 row per thread 1.17 ms, 2 1.11, 4 1.45, 8 1.60)
+		g.items = pin.spec.join ? 2 : 4;
+		// ... and the largest CTAs, whose threads share one table to add to the global one at the end (20M probe
+		// rows into 4096 groups: 512 threads 0.118 ms, 1024 0.109)
+		if (pin.spec.join) g.block = 1024;
 		if (const char *env = std::getenv("VGPU_GB_DIRECT_ITEMS")) {  // tuning override
 			g.items = std::max(1, std::min(32, std::atoi(env)));
 		}
@@ -1106,12 +1114,22 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 		for (auto &na : narrow_args) a.Set(na.first, static_cast<uint64_t>(na.second));
 		const unsigned init_grid = static_cast<unsigned>(std::min<uint64_t>((domain + 255) / 256, 1024));
 		LaunchGenerated(*module, "vgpu_gb_direct_init", init_grid, 256, 0, stream_, a, domain * F * 8, domain);
-		const size_t smem = static_cast<size_t>(PipelineCodegen::DirectSmemBytes(gb, domain));
+		// copies of small tables, up to one per lane and 40 KB in all, which still leaves room for four CTAs per SM
+		const uint64_t table_bytes = PipelineCodegen::DirectSmemBytes(gb, domain);
+		uint64_t copies = 1;
+		if (!direct_l2 && (gb.narrow_count || gb.count_as_flag)) {
+			while (copies < 32 && 2 * copies * table_bytes <= 40 * 1024) copies *= 2;
+		}
+		a.SetWord(kCopiesWord, copies);
+		const size_t smem = static_cast<size_t>(copies * table_bytes);
 		CUfunction f = module->Get("vgpu_gb_direct");
 		int occ = std::max(1, Runtime::Get().MaxActiveBlocks(f, g.block, smem));
 		const uint64_t ntiles = (n + g.tile() - 1) / g.tile();
-		const unsigned grid =
-		    static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(props.sm_count) * occ)));
+		// Every CTA adds its table to the global one, so past one CTA per SM there are only as many as have four
+		// rows per slot (1M rows into 2048 groups, five state words: 490 CTAs 0.028 ms, 148 0.024).
+		const uint64_t sms = static_cast<uint64_t>(props.sm_count);
+		const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
+		    1, std::min<uint64_t>({ntiles, sms * occ, std::max<uint64_t>(sms, n / (4 * domain))})));
 		if (direct_l2) a.SetPtr(cb + 2 + F + out_words, arena_.AllocT<uint64_t>(uint64_t(grid) * direct_f64 * domain));
 		LaunchGenerated(*module, "vgpu_gb_direct", grid, g.block, smem, stream_, a, in_bytes, n);
 		if (!fused_final) LaunchGenerated(*module, "vgpu_gb_direct_final", 1, 1024, 0, stream_, a, domain * F * 8, domain);
