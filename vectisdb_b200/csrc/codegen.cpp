@@ -2386,8 +2386,8 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 		  << "\t\t\tif (prev == ~0ull || prev == key) return (i64)s;\n\t\t}\n\t\ts = (s + step) & (D - 1);\n\t}\n\treturn -1;\n}\n\n";
 	}
 	o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_gb_l2_init(KArgs a) {\n" << kKernelHead
-	  << "\tconst u64 D = a.w[" << cb << "];\n\t{\n" << chain_decl
-	  << "\tconst u64 t0 = blockIdx.x * (u64)blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;\n"
+	  << "\tconst u64 D = a.w[" << cb << "];\n\tif (blockIdx.x != 0) {\n" << chain_decl
+	  << "\tconst u64 t0 = (blockIdx.x - 1) * (u64)blockDim.x + threadIdx.x, step = (gridDim.x - 1) * (u64)blockDim.x;\n"
 	  << "\tfor (u64 i = t0; i < 2 + (ntiles + 1) / 2 + ntiles; i += step) chain[i] = 0ull;\n"
 	  << "\tfor (u64 s = t0; s < D / 2; s += step) {\n";
 	for (int f = 0; f < F; f++) {
@@ -2395,8 +2395,9 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 		  << InitValue(fields[f]) << ");\n";
 	}
 	if (hashed) o << "\t\t((ulonglong2*)" << table << ")[s] = make_ulonglong2(~0ull, ~0ull);\n";
-	// the last CTA samples: groups of consecutive rows spread over the input, counted in a small hash table
-	o << "\t}\n\t}\n\tif (blockIdx.x != gridDim.x - 1) return;\n"
+	// the first CTA samples, meanwhile: groups of consecutive rows spread over the input, counted in a small
+	// hash table
+	o << "\t}\n\treturn;\n\t}\n"
 	  << "\t__shared__ u64 claim[" << H << "];\n\t__shared__ " << kt << " skey[" << kL2SampleRows << "];\n\t__shared__ u32 scount[" << kL2SampleRows << "];\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") claim[i] = 0ull;\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << kL2SampleRows << "u; i += " << g.block << ") { skey[i] = ~(" << kt << ")0; scount[i] = 0u; }\n"
