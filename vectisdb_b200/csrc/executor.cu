@@ -1547,11 +1547,14 @@ Executor::HeavyPlan Executor::PlanHeavy(const PipelineCodegen::GroupBySpec &gb, 
 	const uint32_t SC = 1u << 16;
 	uint64_t *skeys = arena_.AllocT<uint64_t>(SC);
 	uint32_t *scount = arena_.AllocT<uint32_t>(SC);
+	kern::HeavyScratch *sscratch = arena_.AllocT<kern::HeavyScratch>(1);
+	uint64_t *slist = arena_.AllocT<uint64_t>(SC);
 	hp.hmap = arena_.AllocT<uint32_t>(P);
 	hp.keys = arena_.AllocT<uint32_t>(K);
 	hp.count = arena_.AllocT<uint32_t>(1);  // selected keys (the caller points `overflow` at its status block)
 	VGPU_CUDA(cudaMemsetAsync(skeys, 0xff, static_cast<size_t>(SC) * 8, stream_));
 	VGPU_CUDA(cudaMemsetAsync(scount, 0, static_cast<size_t>(SC) * 4, stream_));
+	VGPU_CUDA(cudaMemsetAsync(sscratch, 0, sizeof(kern::HeavyScratch), stream_));
 	VGPU_CUDA(cudaMemsetAsync(hp.hmap, 0xff, P * 4, stream_));
 	VGPU_CUDA(cudaMemsetAsync(hp.count, 0, 4, stream_));
 	const uint64_t samples = std::min<uint64_t>(ntiles, 64);
@@ -1570,8 +1573,8 @@ Executor::HeavyPlan Executor::PlanHeavy(const PipelineCodegen::GroupBySpec &gb, 
 	const uint64_t ctas = 2ull * props.sm_count;
 	uint32_t min_count = static_cast<uint32_t>(std::max<uint64_t>(2, (2 * ctas * samples + ntiles - 1) / ntiles));
 	if (mode == 2) min_count = 1;
-	kern::HeavySelect(skeys, scount, SC, hp.hmap, static_cast<uint32_t>(gb.direct_bits), hp.keys, K, min_count,
-	                  mode != 2, hp.count, stream_);
+	kern::HeavySelect(skeys, scount, SC, sscratch, slist, hp.hmap, static_cast<uint32_t>(gb.direct_bits), hp.keys, K,
+	                  min_count, mode != 2, hp.count, stream_);
 	return hp;
 }
 

@@ -1181,7 +1181,7 @@ uint64_t PlanWorkCapacity(uint32_t P, uint64_t rows, uint32_t min_split) {
 namespace {
 constexpr int kHeavyBlock = 1024;
 constexpr uint32_t kHeavyBins = 1024;  // counts at or above the last bin share it
-constexpr int kHeavyUnroll = 8;        // sample slots per thread and batch
+static_assert(kHeavyBins == kHeavyBlock, "a thread per bin");
 
 __device__ uint64_t HeavyBlockSum(uint64_t v, uint64_t *scratch) {
 	for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
@@ -1193,113 +1193,112 @@ __device__ uint64_t HeavyBlockSum(uint64_t v, uint64_t *scratch) {
 	return total;
 }
 
-__global__ void __launch_bounds__(kHeavyBlock) HeavySelectKernel(const uint64_t *keys, uint32_t *counts, uint32_t SC,
-                                                                 uint32_t *hmap, uint32_t dbits, uint32_t *hkeys,
-                                                                 uint32_t K, uint32_t min_count, bool require_cover,
-                                                                 uint32_t *n_heavy) {
-	__shared__ uint32_t hist[kHeavyBins];
+// The sample's counts: a histogram, their sum, and a list of the keys seen min_count times or more, so that the
+// one CTA that selects walks those alone (a thread per slot; walking the whole table four times from one CTA took
+// 82 us, the two kernels together take 21).
+__global__ void __launch_bounds__(kHeavyBlock) HeavyCountKernel(const uint64_t *keys, const uint32_t *counts,
+                                                                uint32_t min_count, HeavyScratch *g, uint2 *list) {
+	__shared__ uint32_t hist[kHeavyBins], warp_base[kHeavyBlock / 32], base;
 	__shared__ uint64_t scratch[32];
-	__shared__ uint32_t threshold, n_keys;
-	const uint32_t dmask = (1u << dbits) - 1;
-	constexpr uint32_t kWon = 0x80000000u;
-	constexpr int kBatch = kHeavyUnroll;
-	for (uint32_t b = threadIdx.x; b < kHeavyBins; b += blockDim.x) hist[b] = 0;
-	if (threadIdx.x == 0) n_keys = 0;
+	const uint32_t s = blockIdx.x * kHeavyBlock + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	hist[threadIdx.x] = 0;
+	const uint64_t key = keys[s];
+	const uint32_t c = key == ~0ull ? 0u : counts[s];
+	const uint32_t chosen = __ballot_sync(0xffffffffu, c >= min_count);
+	if (lane == 0) warp_base[warp] = __popc(chosen);
 	__syncthreads();
-	// Every pass walks the table in batches of kBatch slots per thread, loads first (one CTA: the
-	// loads of a batch must be in flight together). SC is a multiple of kBatch * blockDim.x, so every
-	// lane of a warp runs every iteration.
-	const uint32_t step = kBatch * blockDim.x;
-	uint64_t sampled = 0;
-	for (uint32_t base = threadIdx.x; base < SC; base += step) {
-		uint32_t c[kBatch];
-#pragma unroll
-		for (int j = 0; j < kBatch; ++j) {
-			const uint32_t s = base + j * blockDim.x;
-			c[j] = keys[s] == ~0ull ? 0u : counts[s];
-		}
-#pragma unroll
-		for (int j = 0; j < kBatch; ++j) {
-			// most sampled keys share a few small counts: lanes of one bin add once
-			const uint32_t bin = c[j] < kHeavyBins ? c[j] : kHeavyBins - 1;
-			const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-			if (bin && static_cast<uint32_t>(__ffs(peers) - 1) == (threadIdx.x & 31)) atomicAdd(&hist[bin], __popc(peers));
-			sampled += c[j];
-		}
-	}
-	sampled = HeavyBlockSum(sampled, scratch);
+	// most sampled keys share a few small counts: lanes of one bin add once
+	const uint32_t bin = c < kHeavyBins ? c : kHeavyBins - 1;
+	const uint32_t peers = __match_any_sync(0xffffffffu, bin);
+	if (bin && static_cast<uint32_t>(__ffs(peers) - 1) == lane) atomicAdd(&hist[bin], __popc(peers));
 	if (threadIdx.x == 0) {
-		// the smallest threshold whose keys fit in K (bins summed from the top)
-		uint32_t t = kHeavyBins, keys_at = 0;
-		while (t > min_count && keys_at + hist[t - 1] <= K) {
-			keys_at += hist[t - 1];
-			--t;
+		uint32_t total = 0;
+		for (uint32_t w = 0; w < kHeavyBlock / 32; ++w) {
+			const uint32_t n = warp_base[w];
+			warp_base[w] = total;
+			total += n;
 		}
-		threshold = t;
+		base = total ? atomicAdd(&g->listed, total) : 0;
 	}
+	const uint64_t sampled = HeavyBlockSum(c, scratch);
+	if (threadIdx.x == 0 && sampled) atomicAdd(reinterpret_cast<unsigned long long *>(&g->sampled), sampled);
+	if (c >= min_count) {  // mixed keys of the direct-partitioned group-by: below 2^31
+		list[base + warp_base[warp] + __popc(chosen & ((1u << lane) - 1))] = make_uint2(static_cast<uint32_t>(key), c);
+	}
+	if (hist[threadIdx.x]) atomicAdd(&g->hist[threadIdx.x], hist[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(kHeavyBlock) HeavySelectKernel(const HeavyScratch *g, uint2 *list, uint32_t *hmap,
+                                                                 uint32_t dbits, uint32_t *hkeys, uint32_t K,
+                                                                 uint32_t min_count, bool require_cover,
+                                                                 uint32_t *n_heavy) {
+	__shared__ uint64_t scratch[32];
+	__shared__ uint32_t above[kHeavyBlock / 32];
+	__shared__ uint32_t n_keys;
+	const uint32_t dmask = (1u << dbits) - 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	constexpr uint32_t kWon = 0x80000000u;
+	if (threadIdx.x == 0) n_keys = 0;
+	// the smallest threshold from min_count up whose keys fit in K: keys with counts in this thread's bin or above
+	uint32_t keys_at = g->hist[threadIdx.x];
+	for (int d = 1; d < 32; d <<= 1) {
+		const uint32_t o = __shfl_down_sync(0xffffffffu, keys_at, d);
+		if (lane + d < 32) keys_at += o;
+	}
+	if (lane == 0) above[warp] = keys_at;
 	__syncthreads();
-	const uint32_t t = threshold;
-	// claim each candidate's partition; the winner marks its sample slot
-	for (uint32_t base = threadIdx.x; base < SC; base += step) {
-		uint64_t k[kBatch];
-		uint32_t c[kBatch];
-#pragma unroll
-		for (int j = 0; j < kBatch; ++j) {
-			k[j] = keys[base + j * blockDim.x];
-			c[j] = counts[base + j * blockDim.x];
-		}
-#pragma unroll
-		for (int j = 0; j < kBatch; ++j) {
-			if (k[j] == ~0ull || c[j] < t) continue;
-			const uint32_t p = static_cast<uint32_t>(k[j] >> dbits);
-			if (atomicCAS(&hmap[p], ~0u, 0xfffe0000u | (static_cast<uint32_t>(k[j]) & dmask)) == ~0u) {
-				counts[base + j * blockDim.x] = c[j] | kWon;
-			}
-		}
+	for (uint32_t w = warp + 1; w < kHeavyBlock / 32; ++w) keys_at += above[w];
+	const uint32_t t = min(min_count, kHeavyBins) + __syncthreads_count(threadIdx.x >= min_count && keys_at > K);
+	const uint32_t listed = g->listed;
+	// claim each candidate's partition; the winner marks its entry
+	for (uint32_t i = threadIdx.x; i < listed; i += kHeavyBlock) {
+		const uint2 e = list[i];
+		if (e.y < t) continue;
+		if (atomicCAS(&hmap[e.x >> dbits], ~0u, 0xfffe0000u | (e.x & dmask)) == ~0u) list[i].y = e.y | kWon;
 	}
 	__syncthreads();
 	uint64_t covered = 0;
-	for (uint32_t base = threadIdx.x; base < SC; base += step) {
-		uint32_t c[kBatch];
-#pragma unroll
-		for (int j = 0; j < kBatch; ++j) c[j] = counts[base + j * blockDim.x];
-#pragma unroll
-		for (int j = 0; j < kBatch; ++j) {
-			if (!(c[j] & kWon)) continue;
-			const uint32_t s = base + j * blockDim.x;
-			const uint64_t k = keys[s];
-			const uint32_t p = static_cast<uint32_t>(k >> dbits);
-			const uint32_t idx = atomicAdd(&n_keys, 1u);
-			if (idx < K) {
-				hmap[p] = (idx << 16) | (static_cast<uint32_t>(k) & dmask);
-				hkeys[idx] = static_cast<uint32_t>(k);
-				covered += c[j] & ~kWon;
-			} else {
-				hmap[p] = ~0u;
-				counts[s] = c[j] & ~kWon;
-			}
+	for (uint32_t i = threadIdx.x; i < listed; i += kHeavyBlock) {
+		const uint2 e = list[i];
+		if (!(e.y & kWon)) continue;
+		const uint32_t idx = atomicAdd(&n_keys, 1u);
+		if (idx < K) {
+			hmap[e.x >> dbits] = (idx << 16) | (e.x & dmask);
+			hkeys[idx] = e.x;
+			covered += e.y & ~kWon;
+		} else {
+			hmap[e.x >> dbits] = ~0u;
+			list[i].y = e.y & ~kWon;
 		}
 	}
 	covered = HeavyBlockSum(covered, scratch);
-	const bool drop = require_cover && covered * 10 < sampled;
+	const bool drop = require_cover && covered * 10 < g->sampled;
 	if (drop) {
-		for (uint32_t s = threadIdx.x; s < SC; s += blockDim.x) {
-			if (counts[s] & kWon) hmap[static_cast<uint32_t>(keys[s] >> dbits)] = ~0u;
+		for (uint32_t i = threadIdx.x; i < listed; i += kHeavyBlock) {
+			const uint2 e = list[i];
+			if (e.y & kWon) hmap[e.x >> dbits] = ~0u;
 		}
 	}
 	if (threadIdx.x == 0) *n_heavy = drop ? 0u : (n_keys < K ? n_keys : K);
 }
 } // namespace
 
-void HeavySelect(const uint64_t *sample_keys, uint32_t *sample_counts, uint32_t SC, uint32_t *hmap, uint32_t dbits,
-                 uint32_t *heavy_keys, uint32_t K, uint32_t min_count, bool require_cover, uint32_t *n_heavy,
-                 cudaStream_t stream) {
-	if (SC % (kHeavyBlock * kHeavyUnroll) != 0) {
-		Fail(VGPU_ERR_INTERNAL, "heavy_select: sample table size must be a multiple of 8192");
+void HeavySelect(const uint64_t *sample_keys, const uint32_t *sample_counts, uint32_t SC, HeavyScratch *scratch,
+                 uint64_t *list, uint32_t *hmap, uint32_t dbits, uint32_t *heavy_keys, uint32_t K, uint32_t min_count,
+                 bool require_cover, uint32_t *n_heavy, cudaStream_t stream) {
+	if (SC % kHeavyBlock != 0) {
+		Fail(VGPU_ERR_INTERNAL, "heavy_select: sample table size must be a multiple of 1024");
 	}
-	LaunchScope scope("heavy_select", stream, static_cast<uint64_t>(SC) * 12, SC);
-	HeavySelectKernel<<<1, kHeavyBlock, 0, stream>>>(sample_keys, sample_counts, SC, hmap, dbits, heavy_keys, K,
-	                                                 min_count < 1 ? 1u : min_count, require_cover, n_heavy);
+	if (min_count < 1) min_count = 1;
+	uint2 *entries = reinterpret_cast<uint2 *>(list);
+	{
+		LaunchScope scope("heavy_count", stream, static_cast<uint64_t>(SC) * 12, SC);
+		HeavyCountKernel<<<SC / kHeavyBlock, kHeavyBlock, 0, stream>>>(sample_keys, sample_counts, min_count, scratch,
+		                                                               entries);
+		VGPU_CUDA(cudaGetLastError());
+	}
+	LaunchScope scope("heavy_select", stream, 0, 0);
+	HeavySelectKernel<<<1, kHeavyBlock, 0, stream>>>(scratch, entries, hmap, dbits, heavy_keys, K, min_count, require_cover,
+	                                                 n_heavy);
 	VGPU_CUDA(cudaGetLastError());
 }
 

@@ -152,6 +152,12 @@ void CountAdjacentEqual(const uint64_t *sorted, uint64_t n, uint32_t *out, cudaS
 //! *out = the length of the longest run of equal keys in `sorted` (saturating at 2^32 - 1).
 void MaxRunLength(const uint64_t *sorted, uint64_t n, uint32_t *out, cudaStream_t stream);
 
+//! Counts of a sample by how often its keys were seen; zeroed by the caller of HeavySelect.
+struct HeavyScratch {
+	uint32_t hist[1024];
+	uint64_t sampled;
+	uint32_t listed, pad;
+};
 //! Work list of a partitioned aggregation pass over `P` partitions whose row ranges start at
 //! offsets[p * stride] (the last ends at *total_rows): 16-byte items (partition, first row, end row,
 //! split index or ~0u), longest first, into `items` (capacity PlanWorkCapacity). Partitions larger
@@ -161,14 +167,15 @@ void MaxRunLength(const uint64_t *sorted, uint64_t n, uint32_t *out, cudaStream_
 //! counts[0] = items, counts[1] = split partitions (split_info is written for the first max_split),
 //! counts[3] = *total_rows.
 //! Heavy keys of a direct-partitioned group-by from a sample: sample_keys/sample_counts ([SC], key ~0
-//! = empty) hold the sampled rows' mixed keys and counts (the counts are used as scratch). Keys seen
-//! at least t times, t >= min_count the smallest threshold that selects at most K keys, claim their
+//! = empty) hold the sampled rows' mixed keys and counts. Keys seen at least
+//! t times, t >= min_count the smallest threshold that selects at most K keys, claim their
 //! partition (key >> dbits; the first claim wins, one heavy key per partition): hmap[p] = (index << 16)
 //! | (key & (2^dbits - 1)), heavy_keys[index] = key, *n_heavy = keys selected. hmap must hold ~0 on
-//! entry. With require_cover, a selection covering under a tenth of the sampled rows is dropped.
-void HeavySelect(const uint64_t *sample_keys, uint32_t *sample_counts, uint32_t SC, uint32_t *hmap, uint32_t dbits,
-                 uint32_t *heavy_keys, uint32_t K, uint32_t min_count, bool require_cover, uint32_t *n_heavy,
-                 cudaStream_t stream);
+//! entry. With require_cover, a selection covering under a tenth of the sampled rows is dropped. `list`:
+//! scratch for SC entries.
+void HeavySelect(const uint64_t *sample_keys, const uint32_t *sample_counts, uint32_t SC, HeavyScratch *scratch,
+                 uint64_t *list, uint32_t *hmap, uint32_t dbits, uint32_t *heavy_keys, uint32_t K, uint32_t min_count,
+                 bool require_cover, uint32_t *n_heavy, cudaStream_t stream);
 uint64_t PlanWorkCapacity(uint32_t P, uint64_t rows, uint32_t min_split);
 void PlanWork(const uint32_t *offsets, uint64_t stride, uint32_t P, const uint32_t *total_rows, uint32_t min_split,
               uint32_t ctas, void *items, uint32_t *counts, uint32_t *split_info, uint32_t max_split,
