@@ -1013,6 +1013,7 @@ int PipelineCodegen::DirectSlotBytes(const GroupBySpec &gb) {
 		if (f.kind == "cnt") bytes += 4;
 		if ((f.kind == "f64" && !gb.f64_l2) || f.kind == "min" || f.kind == "max") bytes += 8;
 		if (f.kind == "lo") bytes += 16;
+		if (f.kind == "s64") bytes += 8;
 	}
 	return bytes;
 }
@@ -1036,7 +1037,7 @@ int PipelineCodegen::HeavySlotBytes(const GroupBySpec &gb) {
 	for (auto &a : gb.aggs) {
 		if (a.column < 0 || a.kind == AggKind::COUNT || a.kind == AggKind::COUNT_STAR) continue;
 		const bool int_sum = (a.kind == AggKind::SUM || a.kind == AggKind::AVG) && !IsFloatType(a.input_type);
-		bytes += int_sum ? 16 : 8;
+		bytes += int_sum && !a.sum64 ? 16 : 8;
 	}
 	return bytes;
 }
@@ -1101,9 +1102,14 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		}
 	}
 	std::ostringstream pack;
-	pack << "(0ull";
+	pack << (gb.direct_bits > 0 ? "(0u" : "(0ull");
 	for (auto &k : gb.keys) {
 		const int j = static_cast<int>(&k - gb.keys.data());
+		if (gb.direct_bits > 0) {  // direct-partitioned: at most 29 bits
+			pack << " | (((u32)(i64)(" << visible_[k.column].value << ") - (u32)a.w[" << kKeyWord + 3 * j << "]) << (u32)a.w["
+			     << kKeyWord + 3 * j + 1 << "])";
+			continue;
+		}
 		pack << " | ((u64)((i64)(" << visible_[k.column].value << ") - (i64)a.w[" << kKeyWord + 3 * j << "]) << (u32)a.w["
 		     << kKeyWord + 3 * j + 1 << "])";
 	}
@@ -1316,11 +1322,13 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 	                                       : "partition_of(" + pack.str() + ", pbits)";
 	const std::string key_of_pack = dpart ? "vgpu_dmix(a, " + pack.str() + ")" : pack.str();
 	if (dpart) {
-		// multiplier, inverse and key mask come with the arguments, so the kernel does not depend on the data
-		o << "__device__ __forceinline__ u64 vgpu_dmix(const KArgs &a, u64 k) { return (k * a.w[" << kMixWord
-		  << "]) & a.w[" << kMixWord + 2 << "]; }\n"
-		  << "__device__ __forceinline__ u64 vgpu_dunmix(const KArgs &a, u64 k) { return (k * a.w[" << kMixWord + 1
-		  << "]) & a.w[" << kMixWord + 2 << "]; }\n\n";
+		// multiplier, inverse and key mask come with the arguments, so the kernel does not depend on the data;
+		// 2^14 partitions of at most 2^15 slots: the packed keys and their products are taken in 32 bits (the count
+		// pass of 2^27 rows with two keys and a filter 0.45 -> 0.39 ms; it reads 16 bytes a row, 0.33 ms)
+		o << "__device__ __forceinline__ u64 vgpu_dmix(const KArgs &a, u32 k) { return (k * (u32)a.w[" << kMixWord
+		  << "]) & (u32)a.w[" << kMixWord + 2 << "]; }\n"
+		  << "__device__ __forceinline__ u64 vgpu_dunmix(const KArgs &a, u32 k) { return (k * (u32)a.w[" << kMixWord + 1
+		  << "]) & (u32)a.w[" << kMixWord + 2 << "]; }\n\n";
 	}
 	// Staged tiles (g.staged, direct-partitioned count and scatter): args cb+13 = byte offset of the two
 	// stages in dynamic shared memory, cb+14 = error flag (u32*). A full tile's needed columns land in
@@ -1451,13 +1459,13 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 				hkind[i] = "f64";
 				harr.push_back({"HF" + is, "double", 8});
 			} else {
-				hkind[i] = "int";
+				hkind[i] = ag.sum64 ? "s64" : "int";  // "s64": the sum stays within 64 bits
 			}
 		}
 		harr.push_back({"HC", "u32", 4});
 		for (size_t i = 0; i < gb.aggs.size(); i++) {
-			if (hkind[i] != "int") continue;
-			for (int w = 0; w < 4; w++) harr.push_back({"HW" + std::to_string(i) + "_" + std::to_string(w), "u32", 4});
+			if (hkind[i] != "int" && hkind[i] != "s64") continue;
+			for (int w = 0; w < (hkind[i] == "int" ? 4 : 2); w++) harr.push_back({"HW" + std::to_string(i) + "_" + std::to_string(w), "u32", 4});
 		}
 		// shared layout after the P + 32 counters: hmap [P], heavy keys [K], then the state arrays
 		// (16-byte aligned; the host sizes the launch with the same rule)
@@ -1544,7 +1552,9 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 			if (hkind[i].empty()) continue;
 			const std::string is = std::to_string(i);
 			const std::string v = visible_[gb.aggs[i].column].value;
-			if (hkind[i] == "int") {
+			if (hkind[i] == "s64") {
+				hupd << "\t\t\t\tatomic_add_i64_u32x2(&HW" << is << "_0[h], &HW" << is << "_1[h], (i64)(" << v << "));\n";
+			} else if (hkind[i] == "int") {
 				hupd << "\t\t\t\t{ const i64 x_ = (i64)(" << v << "); atomic_add_i128_u32x4(&HW" << is << "_0[h], &HW" << is
 				     << "_1[h], &HW" << is << "_2[h], &HW" << is << "_3[h], (u64)x_, x_ < 0 ? -1 : 0); }\n";
 			} else if (hkind[i] == "f64") {
@@ -1564,7 +1574,9 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 			if (hkind[i].empty()) continue;
 			const std::string is = std::to_string(i);
 			const std::string v = visible_[gb.aggs[i].column].value;
-			if (hkind[i] == "int") {
+			if (hkind[i] == "s64") {
+				hgrp << "\t\t\ti64 gs" << is << " = (i64)(" << v << ");\n";
+			} else if (hkind[i] == "int") {
 				hgrp << "\t\t\tu64 glo" << is << " = (u64)(i64)(" << v << "); i64 ghi" << is << " = ((i64)(" << v
 				     << ") < 0) ? -1 : 0;\n";
 			} else if (hkind[i] == "f64") {
@@ -1580,7 +1592,9 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		for (size_t i = 0; i < gb.aggs.size(); i++) {
 			if (hkind[i].empty()) continue;
 			const std::string is = std::to_string(i);
-			if (hkind[i] == "int") {
+			if (hkind[i] == "s64") {
+				hgrp << "\t\t\t\t{ const i64 o_ = __shfl_sync(hpeers_, gs" << is << ", src_); if (me_) gs" << is << " += o_; }\n";
+			} else if (hkind[i] == "int") {
 				hgrp << "\t\t\t\t{ const u64 ol_ = __shfl_sync(hpeers_, glo" << is << ", src_); const i64 oh_ = __shfl_sync(hpeers_, ghi"
 				     << is << ", src_);\n\t\t\t\t  if (me_) { const u64 nl_ = glo" << is << " + ol_; ghi" << is
 				     << " += oh_ + (nl_ < glo" << is << " ? 1 : 0); glo" << is << " = nl_; } }\n";
@@ -1596,7 +1610,9 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		for (size_t i = 0; i < gb.aggs.size(); i++) {
 			if (hkind[i].empty()) continue;
 			const std::string is = std::to_string(i);
-			if (hkind[i] == "int") {
+			if (hkind[i] == "s64") {
+				hgrp << "\t\t\t\tatomic_add_i64_u32x2(&HW" << is << "_0[h], &HW" << is << "_1[h], gs" << is << ");\n";
+			} else if (hkind[i] == "int") {
 				hgrp << "\t\t\t\tatomic_add_i128_u32x4(&HW" << is << "_0[h], &HW" << is << "_1[h], &HW" << is << "_2[h], &HW" << is
 				     << "_3[h], glo" << is << ", ghi" << is << ");\n";
 			} else if (hkind[i] == "f64") {
@@ -1619,7 +1635,9 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 			const std::string is = std::to_string(ai);
 			const int wi = sl.offset / 4;
 			std::string bits;
-			if (hkind[ai] == "int") {
+			if (hkind[ai] == "s64") {
+				bits = "((u64)HW" + is + "_0[h] | ((u64)HW" + is + "_1[h] << 32))";
+			} else if (hkind[ai] == "int") {
 				bits = "((u64)HW" + is + "_0[h] | ((u64)HW" + is + "_1[h] << 32))";
 				// the partial travels as a 64-bit value: a sum outside that range flags the launch,
 				// whose caller then runs the query without pre-aggregation
@@ -1792,6 +1810,15 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 			wvars << "\tdouble wf" << f << " = 0.0;\n";
 			wacc << "\t\t\t\t{ const double t_ = __shfl_sync(0xffffffffu, gf" << f << ", src_); if (have_) wf" << f << " += t_; }\n";
 			wflush << "\t\t\tatomicAdd((double*)(T" << f << " + s_), wf" << f << ");\n";
+		} else if (fd.kind == "s64") {  // a sum that stays within 64 bits
+			gdecl << "\t\t\ti64 gs" << f << " = valid ? (i64)" << v << " : 0;\n";
+			gcomb << "\t\t\t\t\t{ const i64 o_ = __shfl_sync(0xffffffffu, gs" << f << ", src_); if (take) gs" << f << " += o_; }\n";
+			gupd << "\t\t\t\t\tatomicAdd((unsigned long long*)(T" << f << " + s_), (u64)gs" << f << ");\n";
+			gxor << "\t\t\t\t\tgs" << f << " += __shfl_xor_sync(0xffffffffu, gs" << f << ", d);\n";
+			wdecl << "\ti64 ws" << f << " = 0;\n";
+			wvars << "\ti64 ws" << f << " = 0;\n";
+			wacc << "\t\t\t\t{ const i64 t_ = __shfl_sync(0xffffffffu, gs" << f << ", src_); if (have_) ws" << f << " += t_; }\n";
+			wflush << "\t\t\tatomicAdd((unsigned long long*)(T" << f << " + s_), (u64)ws" << f << ");\n";
 		} else if (fd.kind == "lo") {
 			gdecl << "\t\t\tu64 glo" << f << " = valid ? (u64)(i64)" << v << " : 0ull; i64 ghi" << f << " = (valid && (i64)"
 			      << v << " < 0) ? -1 : 0;\n";
@@ -1836,7 +1863,8 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		//   cb+5 = work counter (u32*), cb+6 = output count (u64*), cb+7 = split partition count (u32*,
 		//   read by the init kernel), cb+8.. outputs.
 		// Shared table of D slots, one array per state word: 8-byte arrays (FP64 sums, MIN/MAX) first,
-		// then 32-bit arrays (COUNT, and four words per integer SUM accumulated with 32-bit atomics).
+		// then 32-bit arrays (COUNT, and four words -- two when it stays within 64 bits -- per integer SUM,
+		// accumulated with 32-bit atomics).
 		const int dbits = gb.direct_bits;
 		const uint64_t D = 1ull << dbits;
 		struct DArr {
@@ -1852,8 +1880,8 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 		for (int f = 0; f < F; f++) {
 			const auto &fd = fields[f];
 			if (fd.kind == "cnt") arrs.push_back({"DC", "u32", 4});
-			if (fd.kind == "lo") {
-				for (int w = 0; w < 4; w++) arrs.push_back({"DW" + std::to_string(f) + "_" + std::to_string(w), "u32", 4});
+			if (fd.kind == "lo" || fd.kind == "s64") {
+				for (int w = 0; w < (fd.kind == "lo" ? 4 : 2); w++) arrs.push_back({"DW" + std::to_string(f) + "_" + std::to_string(w), "u32", 4});
 			}
 		}
 		std::ostringstream decl;  // array pointers into the shared table `sm`
@@ -1888,8 +1916,8 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 				if (fd.kind == "min" || fd.kind == "max") {
 					r << "\t\t\tDM" << f << "[" << sv << "] = (i64)" << InitValue(fd) << ";\n";
 				}
-				if (fd.kind == "lo") {
-					for (int w = 0; w < 4; w++) r << "\t\t\tDW" << f << "_" << w << "[" << sv << "] = 0u;\n";
+				if (fd.kind == "lo" || fd.kind == "s64") {
+					for (int w = 0; w < (fd.kind == "lo" ? 4 : 2); w++) r << "\t\t\tDW" << f << "_" << w << "[" << sv << "] = 0u;\n";
 				}
 			}
 			return r.str();
@@ -1902,6 +1930,9 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 				if (fd.kind == "cnt") r << "\t\t\tS" << f << "[0] = (u64)DC[" << sv << "];\n";
 				if (fd.kind == "f64") r << "\t\t\tS" << f << "[0] = (u64)__double_as_longlong(" << f64_load(f, sv) << ");\n";
 				if (fd.kind == "min" || fd.kind == "max") r << "\t\t\tS" << f << "[0] = (u64)DM" << f << "[" << sv << "];\n";
+				if (fd.kind == "s64") {
+					r << "\t\t\tS" << f << "[0] = (u64)DW" << f << "_0[" << sv << "] | ((u64)DW" << f << "_1[" << sv << "] << 32);\n";
+				}
 				if (fd.kind == "lo") {
 					r << "\t\t\tS" << f << "[0] = (u64)DW" << f << "_0[" << sv << "] | ((u64)DW" << f << "_1[" << sv
 					  << "] << 32);\n"
@@ -1921,6 +1952,10 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 				if (fd.kind == "f64") r << "\t\t\t\tatomicAdd(&DF" << fs << "[" << sv << "], " << pre << "f" << fs << ");\n";
 				if (fd.kind == "min" || fd.kind == "max") {
 					r << "\t\t\t\tatomic_" << fd.kind << "_i64(&DM" << fs << "[" << sv << "], " << pre << "m" << fs << ");\n";
+				}
+				if (fd.kind == "s64") {
+					r << "\t\t\t\tatomic_add_i64_u32x2(&DW" << fs << "_0[" << sv << "], &DW" << fs << "_1[" << sv << "], " << pre << "s"
+					  << fs << ");\n";
 				}
 				if (fd.kind == "lo") {
 					r << "\t\t\t\tatomic_add_i128_u32x4(&DW" << fs << "_0[" << sv << "], &DW" << fs << "_1[" << sv << "], &DW" << fs
@@ -1980,6 +2015,10 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 				tinit << "\t\t\t\t\tdouble tf" << fs << " = mem ? gf" << fs << " : 0.0;\n";
 				txor << "\t\t\t\t\t\ttf" << fs << " += __shfl_xor_sync(0xffffffffu, tf" << fs << ", d);\n";
 				ttake << "\t\t\t\t\t\tgf" << fs << " = tf" << fs << ";\n";
+			} else if (fd.kind == "s64") {
+				tinit << "\t\t\t\t\ti64 ts" << fs << " = mem ? gs" << fs << " : 0;\n";
+				txor << "\t\t\t\t\t\tts" << fs << " += __shfl_xor_sync(0xffffffffu, ts" << fs << ", d);\n";
+				ttake << "\t\t\t\t\t\tgs" << fs << " = ts" << fs << ";\n";
 			} else if (fd.kind == "lo") {
 				tinit << "\t\t\t\t\tu64 tlo" << fs << " = mem ? glo" << fs << " : 0ull; i64 thi" << fs << " = mem ? ghi" << fs
 				      << " : 0;\n";
@@ -2461,8 +2500,7 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 			tdecl << "\t\t\t\ti64 t" << i << " = mem ? g" << i << " : 0ll;\n";
 			txor << "\t\t\t\t\tt" << i << " += __shfl_xor_sync(0xffffffffu, t" << i << ", d);\n";
 			ttake << "\t\t\t\t\tg" << i << " = t" << i << ";\n";
-			upd << "\t\t\t{ u32 *w_ = (u32*)(T" << i << " + hp); const u32 up_ = (u32)((u64)g" << i
-			    << " >> 32) + add_word_carry(w_, (u64)(u32)g" << i << "); if (up_) atomicAdd(w_ + 1, up_); }\n";
+			upd << "\t\t\t{ u32 *w_ = (u32*)(T" << i << " + hp); atomic_add_i64_u32x2(w_, w_ + 1, g" << i << "); }\n";
 		} else if (fd.kind == "lo") {
 			const std::string h = std::to_string(f + 1);
 			own << "\t\tu64 g" << i << " = (u64)(i64)(" << v << "); i64 g" << h << " = (i64)g" << i << " < 0 ? -1ll : 0ll;\n";

@@ -130,7 +130,8 @@ public:
 		// One-pass group-by, MIN/MAX: >= 0 keeps the shared-memory state as a 32-bit offset from the
 		// value in this argument word (the input's minimum; its range spans less than 2^32).
 		int narrow_word = -1;
-		// L2 table: an integer SUM or AVG whose total over all rows cannot leave 64 bits keeps one word.
+		// L2 table and direct-partitioned: an integer SUM or AVG whose total over all rows cannot leave 64 bits
+		// keeps one 64-bit word.
 		bool sum64 = false;
 	};
 	struct GroupBySpec {

@@ -455,6 +455,9 @@ std::string GenerateSourceText(const PlanNode &plan, const std::vector<vgpu_colu
 	PipelineCodegen::GroupBySpec spec_plain = spec_dp;
 	spec_plain.bucket_plain = true;
 	spec_hv.f64_l2 = PipelineCodegen::F64Fields(spec_hv) > 0;  // FP64 sums of its bucket pass in L2
+	for (auto &ag : spec_hv.aggs) {  // ... and integer sums in 64 bits
+		ag.sum64 = (ag.kind == AggKind::SUM || ag.kind == AggKind::AVG) && !IsFloatType(ag.input_type);
+	}
 	PipelineCodegen::GroupBySpec spec_nc = spec_gb;
 	spec_nc.narrow_count = true;  // one-pass tables whose counts take no carries
 	spec_nc.count_as_flag = true;  // ... or are presence flags

@@ -440,6 +440,11 @@ __device__ __forceinline__ void atomic_add_i128_u32x4(u32 *w0, u32 *w1, u32 *w2,
 	const u32 top = (u32)((u64)hi >> 32) + c;
 	if (top) atomicAdd(w3, top);
 }
+// The same for a sum that stays within 64 bits, in two words.
+__device__ __forceinline__ void atomic_add_i64_u32x2(u32 *w0, u32 *w1, i64 v) {
+	const u32 up = (u32)((u64)v >> 32) + add_word_carry(w0, (u64)(u32)v);
+	if (up) atomicAdd(w1, up);
+}
 
 __device__ __forceinline__ void atomic_min_i64(i64 *p, i64 v) { atomicMin(reinterpret_cast<long long *>(p), (long long)v); }
 __device__ __forceinline__ void atomic_max_i64(i64 *p, i64 v) { atomicMax(reinterpret_cast<long long *>(p), (long long)v); }

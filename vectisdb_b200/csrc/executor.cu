@@ -970,7 +970,16 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	// (at most 4 slots per input row) and splits into at most 2^14 partitions of the largest
 	// shared-memory table: a row then costs no hashing and no probing.
 	const uint64_t smem_cap = std::min<uint64_t>(props.smem_optin > 4096 ? props.smem_optin - 4096 : 48 * 1024, 200 * 1024);
-	const int dbits_max = BitsFor(FloorPow2(smem_cap / static_cast<uint64_t>(PipelineCodegen::DirectSlotBytes(gb)))) - 1;
+	// FP64 sums of the bucket pass in L2 through reductions (VGPU_GB_F64_L2=0: shared CAS loops). Where its slots
+	// then take 24 bytes or less, tables of 2^13 slots: half the partitions keep half as many lines of records open
+	// between the scatter's writes (2^27 rows into 2^24 keys, SUM, AVG, COUNT and MAX: 20 bytes a slot with a
+	// 64-bit sum, scatter 1.46 ms with 2^12 slots, 1.16 with 2^13).
+	const char *env_l2 = std::getenv("VGPU_GB_F64_L2");
+	PipelineCodegen::GroupBySpec gb_part = gb_l2;
+	const int dbits_all = BitsFor(FloorPow2(smem_cap / static_cast<uint64_t>(PipelineCodegen::DirectSlotBytes(gb)))) - 1;
+	gb_part.f64_l2 = PipelineCodegen::F64Fields(gb) > 0 && !(env_l2 && std::strcmp(env_l2, "0") == 0);
+	const int dbits_l2 = BitsFor(FloorPow2(smem_cap / static_cast<uint64_t>(PipelineCodegen::DirectSlotBytes(gb_part)))) - 1;
+	const int dbits_max = std::max(dbits_all, std::min(13, dbits_l2));
 	bool dpart = shift <= dbits_max + 14 && domain <= 4 * n;
 	// Sparser keys: a hashed table in L2 of up to 64 MB with the keys in it, tried first unless one key alone, or
 	// the plan's estimate, says that the groups fill over 58% of it (a table is sure to take three fifths; the
@@ -1182,11 +1191,11 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 				dbits = std::min(dbits_max, std::max(5, std::atoi(env)));
 			}
 			dbits = std::max(dbits, shift - 14);  // at most 2^14 partitions (the partition histograms)
+			gb_part.keys = gb.keys;
+			gb_part.domain = domain;
+			gb = gb_part;
 			gb.direct_bits = dbits;
 			gb.key_bits = shift;
-			// FP64 sums of the bucket pass in L2 through reductions (VGPU_GB_F64_L2=0: shared CAS loops)
-			const char *env_l2 = std::getenv("VGPU_GB_F64_L2");
-			gb.f64_l2 = PipelineCodegen::F64Fields(gb) > 0 && !(env_l2 && std::strcmp(env_l2, "0") == 0);
 			// without heavy-key pre-aggregation the bucket pass groups equal slots per warp step (hot keys);
 			// VGPU_GB_BUCKET_PLAIN=1 makes every record update its slot itself
 			const char *env_plain = std::getenv("VGPU_GB_BUCKET_PLAIN");
