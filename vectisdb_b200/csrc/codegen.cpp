@@ -2585,7 +2585,7 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	return o.str();
 }
 
-std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geometry &g, int tile_rows, int smem_slots,
+std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geometry &g, int smem_slots,
                                               const BatchLayout &L) const {
 	// One kernel for every query of a batch that shares this plan template. Query q's columns, key
 	// packing, table placement and literal constants come from its row of the query table (L.qwords
@@ -2595,7 +2595,8 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	// table, [param_base..] the literal constants as 64-bit patterns.
 	// vgpu_batch_gb args: w[0] queries, w[1] query table, w[2] tiles (uint2 query, tile), w[3] tiles,
 	//   w[4] tile work counter (u32*, zero at launch), w[5] accumulators (u64, F arrays of w[6] words), w[6] accumulator words
-	//   per field, w[7] output pointer table (u64 [out words]), w[8] group counts (u64 [queries]).
+	//   per field, w[7] output pointer table (u64 [out words]), w[8] group counts (u64 [queries]), w[9] rows per tile,
+	//   w[10] segments (uint2 query, segment: 1024 table slots), w[11] live slots of each segment (u32).
 	std::ostringstream o;
 	o << Prologue();
 	o << "#define vgpu_qpd(j) __longlong_as_double((long long)vgpu_qp[(j)])\n"
@@ -2643,12 +2644,14 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	flush << "\t\t\t\t}\n\t\t\t}\n\t\t\t__syncthreads();\n";
 	// tiles are claimed one at a time from a counter (queries differ in size by orders of magnitude;
 	// the queue lists the largest queries first)
-	o << "\twhile (true) {\n"
-	  << "\t\tif (threadIdx.x == 0) cur_t = atomicAdd(work, 1u);\n"
+	o << "\tif (threadIdx.x == 0) cur_t = atomicAdd(work, 1u);\n"
+	  << "\twhile (true) {\n"
 	  << "\t\t__syncthreads();\n"
 	  << "\t\tconst u64 t = cur_t;\n"
 	  << "\t\t__syncthreads();\n"
 	  << "\t\tif (t >= ntiles) break;\n"
+	  // the next claim is in flight behind this tile's rows
+	  << "\t\tu32 next_t = 0;\n\t\tif (threadIdx.x == 0) next_t = atomicAdd(work, 1u);\n"
 	  << "\t\tconst uint2 tl = tiles[t];\n"
 	  << "\t\tconst u64 *qp = qtab + (u64)tl.x * " << L.qwords << "ull;\n"
 	  << "\t\tif (tl.x != cur_q) {\n"
@@ -2661,8 +2664,8 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	o << "\t\t}\n"
 	  << "\t\tconst u64 *vgpu_qp = qp + " << L.param_base << ";\n\t\t(void)vgpu_qp;\n"
 	  << "\t\tconst u64 n = qp[0];\n"
-	  << "\t\tconst u64 t0 = (u64)tl.y * " << tile_rows << "ull;\n"
-	  << "\t\tconst u64 t1 = t0 + " << tile_rows << "ull < n ? t0 + " << tile_rows << "ull : n;\n"
+	  << "\t\tconst u64 t0 = (u64)tl.y * a.w[9];\n"
+	  << "\t\tconst u64 t1 = t0 + a.w[9] < n ? t0 + a.w[9] : n;\n"
 	  << "\t\tfor (u64 sub = t0; sub < t1; sub += " << g.tile() << "ull) {\n"
 	  << "\t\tconst u64 row0 = sub + (u64)threadIdx.x * " << g.items << ";\n";
 	for (size_t i = 0; i < spec_.sources.size(); i++) {
@@ -2676,9 +2679,10 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	  << "\t\tconst u64 row = row0 + r; (void)row;\n\t\tbool keep = row < t1;\n"
 	  << chain_code_ << "\t\tif (keep) {\n"
 	  << "\t\t\tconst u64 slot = " << pack.str() << ";\n"
-	  << "\t\t\tif (cur_sm) {\n" << UpdateCode(fields, "T", "slot", values, true) << "\t\t\t} else {\n"
+	  << "\t\t\tif (cur_sm) {\n" << UpdateCode(fields, "T", "slot", values, true, gb.narrow_count) << "\t\t\t} else {\n"
 	  << UpdateCode(fields, "G", "slot", values, false) << "\t\t\t}\n"
-	  << "\t\t}\n\t\t}\n\t\t}\n\t}\n"
+	  << "\t\t}\n\t\t}\n\t\t}\n"
+	  << "\t\tif (threadIdx.x == 0) cur_t = next_t;\n\t}\n"
 	  << "\tif (cur_sm) {\n" << flush.str() << "\t}\n}\n\n";
 
 	// accumulators to identity (first use of a batch's buffers; the final kernel resets what it reads)
@@ -2689,24 +2693,38 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	for (int f = 0; f < F; f++) o << "\t\tif (f == " << f << "ull) v = " << InitValue(fields[f]) << ";\n";
 	o << "\t\tacc[i] = v;\n\t}\n}\n\n";
 
-	// one CTA per query: its live slots, in key order, into the outputs; the accumulators are reset
+	// live slots of each segment (not launched when every table is one segment)
+	o << "extern \"C\" __global__ void __launch_bounds__(1024) vgpu_batch_count(KArgs a) {\n"
+	  << "\tconst uint2 sg = ((const uint2*)a.w[10])[blockIdx.x];\n"
+	  << "\tconst u64 *qp = (const u64*)a.w[1] + (u64)sg.x * " << L.qwords << "ull;\n"
+	  << "\tconst u64 s = (u64)sg.y * 1024ull + threadIdx.x;\n"
+	  << "\tconst int live = __syncthreads_count(s < qp[" << L.dom_base << "] && ((const u64*)a.w[5])[qp[" << L.dom_base + 1
+	  << "] + s] != 0);\n"
+	  << "\tif (threadIdx.x == 0) ((u32*)a.w[11])[blockIdx.x] = (u32)live;\n}\n\n";
+
+	// One CTA per segment: its live slots, in key order, into the outputs behind those of the query's segments
+	// before it; the accumulators are reset. (One CTA per query walked its table serially: 20 queries with up to
+	// 2^16 slots and 14M rows took 0.147 ms on the device, 0.132 with a CTA per segment.)
 	GroupBySpec aggs_only = gb;
 	aggs_only.keys.clear();
 	const int nk = static_cast<int>(gb.keys.size());
 	o << "extern \"C\" __global__ void __launch_bounds__(1024) vgpu_batch_final(KArgs a) {\n"
 	  << "\t__shared__ u32 scan_scratch[33];\n"
-	  << "\tconst u32 q = blockIdx.x;\n"
+	  << "\tconst uint2 sg = ((const uint2*)a.w[10])[blockIdx.x];\n"
+	  << "\tconst u32 q = sg.x;\n"
 	  << "\tconst u64 *qp = (const u64*)a.w[1] + (u64)q * " << L.qwords << "ull;\n"
 	  << "\tu64 *acc = (u64*)a.w[5];\n\tconst u64 ACC = a.w[6];\n"
 	  << "\tconst u64 *outp = (const u64*)a.w[7];\n"
 	  << "\tconst u64 D = qp[" << L.dom_base << "], outb = qp[" << L.dom_base + 2 << "];\n";
 	for (int f = 0; f < F; f++) o << "\tu64 *G" << f << " = acc + " << f << "ull * ACC + qp[" << L.dom_base + 1 << "];\n";
-	o << "\tu64 base = 0;\n"
-	  << "\tfor (u64 c0 = 0; c0 < D; c0 += blockDim.x) {\n"
-	  << "\t\tconst u64 s = c0 + threadIdx.x;\n"
-	  << "\t\tconst bool live = s < D && G0[s] != 0;\n"
-	  << "\t\tu32 total; const u32 off = block_exclusive_scan(live ? 1u : 0u, scan_scratch, &total);\n"
-	  << "\t\tif (live) {\n\t\t\tconst u64 pos = outb + base + off;\n\t\t\tconst u64 key = s;\n";
+	o << "\tconst u64 s = (u64)sg.y * 1024ull + threadIdx.x;\n"
+	  << "\tconst bool live = s < D && G0[s] != 0;\n"
+	  << "\tu32 before = 0;\n"
+	  << "\tfor (u32 i = threadIdx.x; i < sg.y; i += blockDim.x) before += ((const u32*)a.w[11])[blockIdx.x - sg.y + i];\n"
+	  << "\tu32 base = 0, total;\n"
+	  << "\tif (sg.y) block_exclusive_scan(before, scan_scratch, &base);\n"
+	  << "\tconst u32 off = block_exclusive_scan(live ? 1u : 0u, scan_scratch, &total);\n"
+	  << "\tif (live) {\n\t\tconst u64 pos = outb + base + off;\n\t\tconst u64 key = s;\n";
 	for (int j = 0; j < nk; j++) {
 		const char *t = CudaTypeName(visible_[gb.keys[j].column].type);
 		o << "\t\t\t{ const u32 sb = (u32)qp[" << L.key_base + 2 * j + 1 << "]; const u32 bits = sb >> 8;\n"
@@ -2714,11 +2732,10 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 		  << "\t\t\t  ((" << t << "*)outp[" << j << "])[pos] = (" << t << ")((i64)((key >> (sb & 0xffu)) & mask) + (i64)qp["
 		  << L.key_base + 2 * j << "]); }\n";
 	}
-	o << FinalizeCode(aggs_only, fields, visible_, "G", "s", "key", "pos", nk, "outp") << "\t\t}\n"
-	  << "\t\tif (s < D) {\n";
-	for (int f = 0; f < F; f++) o << "\t\t\tG" << f << "[s] = " << InitValue(fields[f]) << ";\n";
-	o << "\t\t}\n\t\tbase += total;\n\t}\n"
-	  << "\tif (threadIdx.x == 0) ((u64*)a.w[8])[q] = base;\n}\n";
+	o << FinalizeCode(aggs_only, fields, visible_, "G", "s", "key", "pos", nk, "outp") << "\t}\n"
+	  << "\tif (s < D) {\n";
+	for (int f = 0; f < F; f++) o << "\t\tG" << f << "[s] = " << InitValue(fields[f]) << ";\n";
+	o << "\t}\n\tif (threadIdx.x == 0 && (s | 1023ull) >= D - 1) ((u64*)a.w[8])[q] = base + total;\n}\n";
 	return o.str();
 }
 

@@ -203,8 +203,8 @@ public:
 	};
 	//! Batched group-by over many queries sharing this plan template (literals read from the query
 	//! table through vgpu_qp*): vgpu_batch_init, vgpu_batch_gb (persistent over (query, tile) items),
-	//! vgpu_batch_final (one CTA per query).
-	std::string EmitBatchGroupBy(const GroupBySpec &gb, const Geometry &g, int tile_rows, int smem_slots,
+	//! vgpu_batch_count and vgpu_batch_final (one CTA per 1024 slots).
+	std::string EmitBatchGroupBy(const GroupBySpec &gb, const Geometry &g, int smem_slots,
 	                             const BatchLayout &L) const;
 	//! Number of 8-byte per-group aggregate state fields (excluding the key), as laid out by EmitGroupBy.
 	static int StateWords(const GroupBySpec &gb);
