@@ -83,3 +83,13 @@ def test_no_match_and_a_hot_left_key():
     rk = np.concatenate([np.full(150, 7), rng.integers(0, 3000, 3000)]).astype(np.int64)
     names = _join(lk, rk, T.INT64)  # 512 rows of a tile with 150 matches each: past a tile's most
     assert "join_expand" in names, names
+
+
+@pytest.mark.parametrize("spread", [1, 1 << 30])
+@pytest.mark.parametrize("left,ordered", [((1 << 20) - 1, False), (1 << 20, True), ((1 << 20) + 77, True)])
+def test_right_columns_in_run_order_from_four_matches_a_row(left, ordered, spread):
+    """Four matches a right row and a million of them: the right columns are gathered into run order first."""
+    rng = np.random.default_rng(9)
+    rk = rng.permutation(1 << 18).astype(np.int64) * spread
+    names = _join(rng.integers(0, 1 << 18, left).astype(np.int64) * spread, rk, T.INT64)
+    assert ("gather" in names) == ordered and "join_emit" in names, names

@@ -2037,11 +2037,25 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 		if (total > kMaxOutputRows) too_large(total);
 		out = make_out(total);
 		if (total == 0) return true;
+		// Where each right row has four matches or more on average, the right columns are put in run order first, so
+		// that a match reads its neighbours' sectors instead of a row number and then a sector of its own: 1M right
+		// rows, one column, 7.3M matches: emit 0.113 -> 0.088 ms for a gather of 0.014; 2M right rows, 4.2M matches:
+		// 0.090 -> 0.073 for 0.018. Not below a million matches, nor when memory is short.
+		uint64_t right_bytes = 0;
+		for (size_t i = 0; i < sources.size(); i++) right_bytes += from_left[i] ? 0 : rn * TypeSize(sources[i]->type);
+		const bool ordered = total / 4 >= rn && total >= (1u << 20) && Runtime::Get().allocator().HasHeadroom(right_bytes);
 		kern::JoinOuts outs;
 		for (size_t i = 0; i < sources.size(); i++) {
-			outs.c[outs.n++] = {sources[i]->data, out[i].data, static_cast<int>(TypeSize(sources[i]->type)), !from_left[i]};
+			const size_t width = TypeSize(sources[i]->type);
+			const void *src = sources[i]->data;
+			if (ordered && !from_left[i]) {
+				void *by_run = arena_.Alloc(rn * width);
+				kern::Gather(src, width, rows, rn, by_run, stream_);
+				src = by_run;
+			}
+			outs.c[outs.n++] = {src, out[i].data, static_cast<int>(width), !from_left[i]};
 		}
-		kern::JoinEmit(lk.data, kw, ln, view, chain, rows, outs, total, stream_);
+		kern::JoinEmit(lk.data, kw, ln, view, chain, ordered ? nullptr : rows, outs, total, stream_);
 		return true;
 	};
 	if (tiled && dense) {

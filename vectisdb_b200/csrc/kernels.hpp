@@ -124,7 +124,8 @@ struct JoinOuts {
 	JoinOut c[kMaxJoinOuts];
 	int n = 0;
 };
-//! Every output column of the matches, left rows in order and each one's matches in the order of `rows`.
+//! Every output column of the matches, left rows in order and each one's matches in the order of `rows`; without
+//! `rows` the right columns are in that order themselves.
 void JoinEmit(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, const uint64_t *chain,
               const uint32_t *rows, const JoinOuts &outs, uint64_t total, cudaStream_t stream);
 
