@@ -14,7 +14,9 @@ LIMITS = [1 << 20, ((1 << 63) - 1) // N, ((1 << 63) - 1) // N + 1, 1 << 62]
 
 
 @pytest.mark.parametrize("env", [{"VGPU_GB_HEAVY": "0"}, {"VGPU_GB_HEAVY": "0", "VGPU_GB_BUCKET_PLAIN": "1"},
-                                 {"VGPU_GB_HEAVY": "0", "VGPU_GB_SPLIT_ROWS": "256"}, {"VGPU_GB_HEAVY": "2"},
+                                 {"VGPU_GB_HEAVY": "0", "VGPU_GB_SPLIT_ROWS": "256"},
+                                 {"VGPU_GB_HEAVY": "0", "VGPU_GB_DIRECT_BITS": "13"}, {"VGPU_GB_HEAVY": "2"},
+                                 {"VGPU_GB_HEAVY": "2", "VGPU_GB_DIRECT_BITS": "13"},
                                  {"VGPU_GB_HEAVY": "2", "VGPU_GB_HEAVY_WARP": "0"},
                                  {"VGPU_GB_HEAVY": "2", "VGPU_GB_STAGED": "0", "VGPU_GB_SPLIT_ROWS": "256"}])
 @pytest.mark.parametrize("limit", LIMITS)
