@@ -224,3 +224,30 @@ def test_more_sparse_keys_than_the_hashed_table_holds(keys, estimate, tried):
     assert np.array_equal(r.columns[0].data[got], a[want]) and np.array_equal(r.columns[1].data[got], b[want])
     for i in range(6):
         assert np.array_equal(r.columns[2 + i].data[got], cols[2 + i].data[want])
+
+
+@pytest.mark.parametrize("n,taken", [((1 << 23) - 1, False), (1 << 23, True)])
+def test_tables_of_128_megabytes_from_a_row_for_each_slot(n, taken):
+    rng = np.random.default_rng(21)
+    k = (rng.integers(0, 1 << 23, n) - 999).astype(np.int32)
+    k[0], k[-1] = -999, (1 << 23) - 1000
+    v = rng.integers(-1000, 1000, n).astype(np.int32)
+    plan = make_group_by(["k"], [make_aggregate(A.SUM, "v", T.HUGEINT), make_aggregate(A.COUNT_STAR, "", T.INT64)],
+                         make_scan(["k", "v"]))
+    profile_drain()
+    profile_enable(True)
+    try:
+        r = GpuEngine.instance().execute_plan(plan, [make_column("k", T.INT32, k), make_column("v", T.INT32, v)])
+        names = [rec[0] for rec in profile_drain()]
+    finally:
+        profile_enable(False)
+    assert r.success, r.error_message
+    assert (KERNEL in names) == taken and ("vgpu_gb_dbucket" in names) != taken, names
+    at = k.astype(np.int64) + 999
+    counts = np.bincount(at, minlength=1 << 23)
+    sums = np.bincount(at, weights=v, minlength=1 << 23).astype(np.int64)  # exact: below 2^53
+    got = r.columns[0].data.astype(np.int64) + 999
+    order = np.argsort(got)
+    assert np.array_equal(got[order], np.flatnonzero(counts))
+    assert np.array_equal(r.columns[2].data[order], counts[counts > 0])
+    assert np.array_equal(r.columns[1].data["lower"][order].view(np.int64), sums[counts > 0])

@@ -2352,7 +2352,8 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 }
 
 // One-pass group-by into one table in global memory that stays in L2, for key spaces past the shared-memory
-// tables whose table (domain * state words * 8 bytes) is at most kL2TableBytes. Bound by the L2 reductions:
+// tables whose table (domain * state words * 8 bytes) is at most kL2TableBytes (twice that for one row to
+// eight in each slot). Bound by the L2 reductions:
 // about 190 G/s whatever their type, up to a 64 MB table (60 G/s from 128 MB on), against the partitioned
 // strategies' record written, read back and aggregated in shared memory: 10M rows into 2^20 keys, SUM and
 // COUNT, kernels 0.48 ms in ten launches -> 0.16 ms in three; 1.34e8 skewed rows (half filtered away) into
