@@ -125,12 +125,9 @@ struct Walker {
 			if (SatMul(groups, fields * 8) <= 96 * 1024) {
 				// one pass: per-CTA shared tables, one global table over the key domain, outputs
 				bytes = SatAdd(SatMul(groups, fields * 8 + out_width), 64);
-			} else if (n.estimated_rows && SatMul(groups, fields * 8) <= PipelineCodegen::kL2TableBytes / 4) {
-				// one pass into a table over the key domain (dense keys: up to twice the groups), outputs
-				bytes = SatMul(groups, 2 * fields * 8 + out_width);
 			} else {
-				// partitioned: one record per passing row (packed key + carried values, 32-byte aligned),
-				// outputs per group, per-(partition, CTA) offsets, tables of split partitions
+				// partitioned (whether the keys fit a table in L2 shows at run time; it mostly takes less): one
+				// record per passing row (packed key + carried values, 32-byte aligned), outputs per group, per-(partition, CTA) offsets, tables of split partitions
 				const uint64_t record = (carried + 31) / 32 * 32;
 				bytes = SatMul(c.rows, record);
 				bytes = SatAdd(bytes, SatMul(groups, out_width));
