@@ -682,13 +682,15 @@ __global__ void __launch_bounds__(kJoinBlock) JoinMatchCountKernel(const K *keys
 	u64 *starts = reinterpret_cast<u64 *>(chain + 2 + (ntiles + 1) / 2);
 	if (threadIdx.x == 0) next = atomicAdd(words, 1u);
 	__syncthreads();
-	if (next == 0) {
+	const uint32_t ticket = next;
+	__syncthreads();  // read by every thread: the following ticket comes in the same word
+	if (ticket == 0) {
 		const u64 t = tile_scanner(counts, starts, ntiles, scratch, &bound);
 		if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long *>(chain), t == ~0ull ? 1ull << 63 : t);
 		return;
 	}
 	uint32_t longest = 0;
-	for (uint64_t tile = next - 1ull; tile < ntiles;) {
+	for (uint64_t tile = ticket - 1ull; tile < ntiles;) {
 		const uint64_t row0 = tile * kJoinTile + threadIdx.x * static_cast<uint64_t>(kJoinItems);
 		K k[kJoinItems];
 #pragma unroll
