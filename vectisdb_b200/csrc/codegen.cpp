@@ -679,8 +679,8 @@ std::string PipelineCodegen::EmitMaterializeOnePass(const std::vector<int> &outs
 	  << "\t__syncthreads();\n"
 	  << "\tif (vgpu_next == 0u) {\n"
 	  << "\t\t__shared__ u32 vgpu_bound;\n"
-	  << "\t\tconst u64 t_ = tile_scanner(counts, starts, ntiles, scan_scratch, &vgpu_bound);\n"
-	  << "\t\tif (threadIdx.x == 0) atomicAdd(chain, t_ == ~0ull ? 1ull << 63 : t_);\n\t\treturn;\n\t}\n"
+	  << "\t\tconst u64 t_ = tile_scanner(counts, starts, ntiles, scan_scratch, &vgpu_bound, a.w[" << kWaitWord << "]);\n"
+	  << "\t\tif (threadIdx.x == 0) tiles_total(chain, t_);\n\t\treturn;\n\t}\n"
 	  << "\tu64 tile = (u64)vgpu_next - 1, held = ~0ull;  // held: the tile whose rows wait in the other half\n"
 	  << "\tu32 ticket = threadIdx.x == 0 ? atomicAdd((u32*)(chain + 1), 1u) : 0u;  // thread 0: of the tile after\n"
 	  << "\tu32 held_rows = 0;\n\tchar *st = vgpu_st, *st_held = vgpu_st + " << bytes << ";\n"
@@ -718,7 +718,8 @@ std::string PipelineCodegen::EmitMaterializeOnePass(const std::vector<int> &outs
 	  << "\t\tif (tile < ntiles) {\n" << LoadBlock(g, needed, false) << "\t\t}\n"
 	  << "\t\tif (threadIdx.x == 0) {\n"
 	  << "\t\t\tu64 b_ = 0;\n\t\t\tif (held != ~0ull && held != 0) {\n"
-	  << "\t\t\t\tb_ = tile_wait(starts + held);\n\t\t\t\tif (b_ == ~0ull) atomicOr(chain, 1ull << 63);\n\t\t\t}\n"
+	  << "\t\t\t\tb_ = tile_wait(starts + held, a.w[" << kWaitWord << "]);\n"
+	  << "\t\t\t\tif (b_ == ~0ull) tiles_total(chain, b_);\n\t\t\t}\n"
 	  << "\t\t\tvgpu_base = b_;\n\t\t}\n"
 	  << "\t\t__syncthreads();\n"
 	  << "\t\tconst u64 base = vgpu_base;\n\t\tif (base == ~0ull) return;\n"
@@ -2555,8 +2556,8 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	  << "\tif (threadIdx.x == 0) vgpu_next = atomicAdd((u32*)(chain + 1), 1u);\n"
 	  << "\t__syncthreads();\n"
 	  << "\tif (vgpu_next == 0u) {\n\t\t__shared__ u32 vgpu_bound;\n"
-	  << "\t\tconst u64 t_ = tile_scanner(counts, starts, ntiles, scan_scratch, &vgpu_bound);\n"
-	  << "\t\tif (threadIdx.x == 0) atomicAdd(chain, t_ == ~0ull ? 1ull << 63 : t_);\n\t\treturn;\n\t}\n"
+	  << "\t\tconst u64 t_ = tile_scanner(counts, starts, ntiles, scan_scratch, &vgpu_bound, a.w[" << kWaitWord << "]);\n"
+	  << "\t\tif (threadIdx.x == 0) tiles_total(chain, t_);\n\t\treturn;\n\t}\n"
 	  << "\tfor (u64 tile = (u64)vgpu_next - 1; tile < ntiles;) {\n"
 	  << "\t\tconst u64 s0 = tile * " << fin_tile << "ull + threadIdx.x;\n"
 	  << (hashed ? "\t\tconst u64 p0 = s0;\n"
@@ -2573,8 +2574,8 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	  << "\t\t\tvgpu_warps[lane] = incl_ - own_;\n"
 	  << "\t\t\tif (lane == 31) {\n\t\t\t\tst_relaxed(counts + tile, incl_ + 1u);\n"
 	  << "\t\t\t\tconst u32 next_ = atomicAdd((u32*)(chain + 1), 1u);\n"
-	  << "\t\t\t\tconst u64 b_ = tile == 0 ? 0ull : tile_wait(starts + tile);\n"
-	  << "\t\t\t\tif (b_ == ~0ull) atomicOr(chain, 1ull << 63);\n\t\t\t\tvgpu_base = b_;\n\t\t\t\tvgpu_next = next_;\n\t\t\t}\n\t\t}\n"
+	  << "\t\t\t\tconst u64 b_ = tile == 0 ? 0ull : tile_wait(starts + tile, a.w[" << kWaitWord << "]);\n"
+	  << "\t\t\t\tif (b_ == ~0ull) tiles_total(chain, b_);\n\t\t\t\tvgpu_base = b_;\n\t\t\t\tvgpu_next = next_;\n\t\t\t}\n\t\t}\n"
 	  << "\t\t__syncthreads();\n\t\tif (vgpu_base == ~0ull) return;\n"
 	  << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < 4; ++r) {\n\t\t\tif (!((live[r] >> lane) & 1u)) continue;\n"
 	  << "\t\t\tconst u64 at = p0 + " << apart << "ull * r;\n\t\t\tconst u64 key = "

@@ -80,6 +80,8 @@ constexpr int kMaxPackedKeys = 8;
 constexpr int kMixWord = 120;
 // One-pass group-by (which does not mix): copies of every shared-memory slot, a power of two.
 constexpr int kCopiesWord = kMixWord;
+// Kernels that wait for the starts of tiles in their own launch (no mixed keys there either): the longest wait in ns.
+constexpr int kWaitWord = kMixWord + 1;
 // Join-source words: [kJoinWord] sorted right keys (u64, biased), [+1] radix directory (u32),
 // [+2] bias (the right minimum), [+3] shift | bucket count << 8.
 constexpr int kJoinWord = 123;

@@ -337,21 +337,32 @@ __device__ __forceinline__ void st_relaxed(u32 *p, u32 v) {
 	asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// A bounded wait's clock: true once about two seconds (or 2^26 polls) have passed since the first call.
+// A bounded wait's clock: true once limit_ns (or 2^26 polls) have passed since the first call; with a limit of 0,
+// which lets a test see waits run out, at the first call.
 struct PollLimit {
+	u64 limit_ns;
 	u32 polls = 0;
 	u64 t0 = 0;
+	__device__ __forceinline__ explicit PollLimit(u64 ns) : limit_ns(ns) {}
 	__device__ __forceinline__ bool Expired() {
-		if ((++polls & 255u) != 0) return false;
+		if ((++polls & 255u) != 0) return limit_ns == 0;
 		const u64 now = global_ns();
 		if (t0 == 0) t0 = now;
-		return now - t0 > 2000000000ull || polls >= (1u << 26);
+		return now - t0 > limit_ns || polls >= (1u << 26);
 	}
 };
 
+// The mark of a wait that ran out, in the word that takes the total: set, not added, so that a second one leaves it.
+constexpr u64 kTilesFailed = 1ull << 63;
+__device__ __forceinline__ void tiles_total(u64 *word, u64 total) {
+	unsigned long long *w = reinterpret_cast<unsigned long long *>(word);
+	if (total == ~0ull) atomicOr(w, kTilesFailed);
+	else atomicAdd(w, total);
+}
+
 // One thread: the start of a tile, or ~0 when the wait ran out.
-__device__ __forceinline__ u64 tile_wait(const u64 *start) {
-	PollLimit limit;
+__device__ __forceinline__ u64 tile_wait(const u64 *start, u64 limit_ns) {
+	PollLimit limit(limit_ns);
 	for (;;) {
 		const u64 v = ld_relaxed(start);
 		if (v != 0) return v - 1;
@@ -362,10 +373,11 @@ __device__ __forceinline__ u64 tile_wait(const u64 *start) {
 // The scanning CTA (blockDim.x a multiple of 32; `scratch` 33 words and `bound` one word of shared memory):
 // up to four tiles per thread and step, as far as their counts are published without a gap. Returns the
 // total, or ~0 when the tiles stopped making progress.
-__device__ __forceinline__ u64 tile_scanner(const u32 *counts, u64 *starts, u64 ntiles, u32 *scratch, u32 *bound) {
+__device__ __forceinline__ u64 tile_scanner(const u32 *counts, u64 *starts, u64 ntiles, u32 *scratch, u32 *bound,
+                                            u64 limit_ns) {
 	constexpr u32 kEach = 4;
 	u64 carry = 0, first = 0;
-	PollLimit limit;
+	PollLimit limit(limit_ns);
 	while (first < ntiles) {
 		u32 c[kEach];
 		u32 ready = 0;  // leading published counts of this thread's tiles
@@ -394,7 +406,7 @@ __device__ __forceinline__ u64 tile_scanner(const u32 *counts, u64 *starts, u64 
 		}
 		carry += total;
 		first += n;
-		if (n != 0) limit = PollLimit();
+		if (n != 0) limit = PollLimit(limit_ns);
 		if (__syncthreads_or(n == 0 && limit.Expired())) return ~0ull;
 	}
 	return carry;

@@ -602,6 +602,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 		KArgsHost a;
 		FillArgs(pin, a);
 		a.SetPtr(cb, chain);
+		a.SetWord(kWaitWord, kern::WaitLimitNs());
 		add_columns(a, n);
 		CUfunction f = module->Get("vgpu_mat_onepass");
 		const int occ = std::max(1, Runtime::Get().MaxActiveBlocks(f, g.block, smem));
@@ -611,7 +612,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 		// at the root, outputs without NULL masks may leave the count on the device
 		if (at_root && !null_outs && DeferRows(chain, 8, 0)) return out;
 		out_rows = ReadU64(chain);
-		if (out_rows > n) Fail(VGPU_ERR_CUDA, "gpu_executor: a row filter's tiles were not completed within two seconds");
+		if (out_rows > n) Fail(VGPU_ERR_CUDA, "gpu_executor: a row filter's tiles were not completed in time");
 		for (auto &col : out) {
 			col.rows = out_rows;
 			// a result that keeps few of many rows does not hold on to the room for all of them
@@ -1493,6 +1494,7 @@ bool Executor::GroupByL2(const PlanNode &node, PipelineInput &pin, const Pipelin
 	for (int f = 0; f < F; f++) a.SetPtr(cb + 1 + f, fields + slots * f);
 	for (size_t w = 0; w < out.size(); w++) a.SetPtr(cb + 1 + F + static_cast<int>(w), out[w].data);
 	a.SetPtr(cg.L2ChainWord(gb), chain);
+	a.SetWord(kWaitWord, kern::WaitLimitNs());
 	a.SetPtr(cg.L2ChainWord(gb) + 1, arena_.AllocT<uint64_t>(PipelineCodegen::kL2HotSlots));
 	if (hashed) a.SetPtr(cg.L2ChainWord(gb) + 2, fields + slots * F);
 	const uint64_t sms = static_cast<uint64_t>(props.sm_count);
@@ -1515,7 +1517,7 @@ bool Executor::GroupByL2(const PlanNode &node, PipelineInput &pin, const Pipelin
 		arena_.FreeNow(fields);
 		return false;
 	}
-	if (head[0] > cap_rows) Fail(VGPU_ERR_CUDA, "gpu_groupby: the groups were not compacted within two seconds");
+	if (head[0] > cap_rows) Fail(VGPU_ERR_CUDA, "gpu_groupby: the groups were not compacted in time");
 	*groups = head[0];
 	return true;
 }

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <limits>
 #include <type_traits>
@@ -674,7 +675,7 @@ constexpr int kJoinBlock = 256, kJoinItems = 4, kJoinTile = kJoinBlock * kJoinIt
 // than 2^31 matches counts as failed too: the caller takes the other way.
 template <typename K>
 __global__ void __launch_bounds__(kJoinBlock) JoinMatchCountKernel(const K *keys, uint64_t n, JoinRunsView view, uint64_t ntiles,
-                                                              uint64_t *chain) {
+                                                              uint64_t *chain, uint64_t wait_ns) {
 	__shared__ uint32_t scratch[33], bound, next;
 	__shared__ unsigned long long wide;
 	uint32_t *words = reinterpret_cast<uint32_t *>(chain + 1);
@@ -685,8 +686,8 @@ __global__ void __launch_bounds__(kJoinBlock) JoinMatchCountKernel(const K *keys
 	const uint32_t ticket = next;
 	__syncthreads();  // read by every thread: the following ticket comes in the same word
 	if (ticket == 0) {
-		const u64 t = tile_scanner(counts, starts, ntiles, scratch, &bound);
-		if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long *>(chain), t == ~0ull ? 1ull << 63 : t);
+		const u64 t = tile_scanner(counts, starts, ntiles, scratch, &bound, wait_ns);
+		if (threadIdx.x == 0) tiles_total(reinterpret_cast<u64 *>(chain), t);
 		return;
 	}
 	uint32_t longest = 0;
@@ -1452,6 +1453,11 @@ void JoinDenseRuns(const void *keys, size_t kwidth, uint64_t n, uint64_t bias, u
 	VGPU_CUDA(cudaGetLastError());
 }
 
+uint64_t WaitLimitNs() {
+	const char *env = std::getenv("VGPU_WAIT_LIMIT_NS");
+	return env ? std::min<uint64_t>(std::strtoull(env, nullptr, 10), 10000000000ull) : 2000000000ull;
+}
+
 uint64_t JoinChainWords(uint64_t n_left) {
 	const uint64_t tiles = (n_left + kJoinTile - 1) / kJoinTile;
 	return 2 + (tiles + 1) / 2 + tiles;
@@ -1465,7 +1471,7 @@ void JoinCountMatches(const void *keys, size_t kwidth, uint64_t n, const JoinRun
 	const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles + 1, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8));
 	WithKeys(keys, kwidth, [&](auto *k) {
 		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
-		JoinMatchCountKernel<K><<<grid, kJoinBlock, 0, stream>>>(k, n, view, tiles, chain);
+		JoinMatchCountKernel<K><<<grid, kJoinBlock, 0, stream>>>(k, n, view, tiles, chain, WaitLimitNs());
 	});
 	VGPU_CUDA(cudaGetLastError());
 }

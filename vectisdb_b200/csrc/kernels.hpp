@@ -108,6 +108,9 @@ constexpr uint32_t kJoinRunLimit = 4096;
 //! becomes the longest run's length: past kJoinRunLimit that run is not in order, and the caller sorts instead.
 void JoinDenseRuns(const void *keys, size_t kwidth, uint64_t n, uint64_t bias, uint64_t range, uint64_t *entries,
                    uint32_t *rows, uint32_t *list, uint32_t *info, cudaStream_t stream);
+//! Longest wait in ns of a kernel for tiles counted in the same launch (VGPU_WAIT_LIMIT_NS, for testing: up to 10 s;
+//! with 0 every wait that is not over at its first look runs out).
+uint64_t WaitLimitNs();
 //! Matches of the left rows (raw keys): chain [JoinChainWords] = the total (bits 62 and 63 set when a tile has 2^31
 //! or a wait ran out), [1] >> 32 = the most matches of one tile of left rows, then the tiles' starts for JoinEmit.
 uint64_t JoinChainWords(uint64_t n_left);
