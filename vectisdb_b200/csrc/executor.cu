@@ -1821,11 +1821,15 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 			JoinTableCache::Get().Insert(cache_key, t);
 		};
 		// Key range and, with an inline column, its raw bits' range: from the cached columns' own when those
-		// are not negative (raw bits then order like values) and dense, else measured in one launch.
+		// are not negative (raw bits then order like values) and dense, else measured in one launch. Booleans are
+		// always measured: any byte but 0 is true in the cache's range, and the tables are indexed by the byte.
 		uint64_t lo = 0, hi = 0;
 		auto dense = [&](uint64_t r) { return r < (1ull << 28) && r < 4 * rn; };
-		if (rk->has_stats && rk->min >= 0 && dense(static_cast<uint64_t>(rk->max) - static_cast<uint64_t>(rk->min)) &&
-		    (!inline_col || (inline_col->has_stats && inline_col->min >= 0 && IsIntegerKeyType(inline_col->type)))) {
+		auto raw_range = [](const DevColumn &c) {
+			return c.has_stats && c.min >= 0 && IsIntegerKeyType(c.type) && c.type != ValueType::BOOLEAN;
+		};
+		if (raw_range(*rk) && dense(static_cast<uint64_t>(rk->max) - static_cast<uint64_t>(rk->min)) &&
+		    (!inline_col || raw_range(*inline_col))) {
 			lo = static_cast<uint64_t>(rk->min);
 			hi = static_cast<uint64_t>(rk->max);
 			if (inline_col) {
