@@ -400,7 +400,7 @@ std::string PipelineCodegen::LoadBlock(const Geometry &g, const std::vector<bool
 		} else {
 			const char *idx = src.side == 0 ? "li[r]" : "rj[r]";
 			o << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < " << g.items << "; ++r) {\n";
-			o << "\t\t\ts" << i << "[r] = (row0 + r < n) ? ((const " << t << "*)a.w[" << w << "])[" << idx << "] : ("
+			o << "\t\t\ts" << i << "[r] = (row0 + r < n) ? ld_scalar((const " << t << "*)a.w[" << w << "] + " << idx << ") : ("
 			  << t << ")0;\n";
 			if (src.nullable) {
 				o << "\t\t\tsv" << i << "[r] = (row0 + r < n) ? (((const u8*)a.w[" << w + 1 << "])[" << idx
@@ -452,8 +452,8 @@ std::string PipelineCodegen::LoadBlock(const Geometry &g, const std::vector<bool
 				  << t << ">((u64)(u32)jm[r]) : (" << t << ")0;\n";
 				continue;
 			}
-			o << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < " << g.items << "; ++r) s" << i << "[r] = jm[r] >= 0 ? ((const "
-			  << t << "*)a.w[" << w << "])[jm[r]] : (" << t << ")0;\n";
+			o << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < " << g.items << "; ++r) s" << i << "[r] = jm[r] >= 0 ? ld_scalar((const "
+			  << t << "*)a.w[" << w << "] + jm[r]) : (" << t << ")0;\n";
 			if (src.nullable) {
 				o << "\t\t#pragma unroll\n\t\tfor (int r = 0; r < " << g.items << "; ++r) sv" << i
 				  << "[r] = jm[r] >= 0 ? (((const u8*)a.w[" << w + 1 << "])[jm[r]] != 0) : false;\n";
@@ -484,7 +484,7 @@ std::string PipelineCodegen::ItemOpen(const Geometry &g, const std::vector<bool>
 			continue;
 		}
 		const int w = 2 + 2 * static_cast<int>(i);
-		o << "\t\ts" << i << "[r] = ((const " << t << "*)a.w[" << w << "])[jp_];\n";
+		o << "\t\ts" << i << "[r] = ld_scalar((const " << t << "*)a.w[" << w << "] + jp_);\n";
 		if (src.nullable) o << "\t\tsv" << i << "[r] = ((const u8*)a.w[" << w + 1 << "])[jp_] != 0;\n";
 	}
 	o << "\t\tbool keep = true;\n";

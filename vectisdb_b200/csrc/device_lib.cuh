@@ -80,6 +80,10 @@ __device__ __forceinline__ u32 ld_stream_u32(const void *p) {
 template <typename T> __device__ __forceinline__ T ld_scalar(const T *p) {
 	return *p;
 }
+// Any byte but 0 is true, as in word_element: BOOLEAN keys are packed into the one bit of their truth values.
+template <> __device__ __forceinline__ bool ld_scalar<bool>(const bool *p) {
+	return *reinterpret_cast<const u8 *>(p) != 0;
+}
 
 // Extracts element `i` (of size sizeof(T)) from a little-endian array of 32-bit words.
 template <typename T> __device__ __forceinline__ T word_element(const u32 *words, int i) {
@@ -207,7 +211,7 @@ template <typename T, int R> __device__ __forceinline__ void load_stage(const T 
 		for (int r = 0; r < R; ++r) out[r] = word_element<T>(words, r);
 	} else {
 #pragma unroll
-		for (int r = 0; r < R; ++r) out[r] = p[r];
+		for (int r = 0; r < R; ++r) out[r] = ld_scalar(p + r);
 	}
 }
 
