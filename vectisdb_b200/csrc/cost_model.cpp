@@ -144,8 +144,9 @@ struct Walker {
 				// one pass: per-CTA shared tables, one global table over the key domain, outputs
 				bytes = SatAdd(SatMul(groups, fields * 8 + out_width), 64);
 			} else {
-				// partitioned (whether the keys fit a table in L2 shows at run time; it mostly takes less): one
-				// record per passing row (packed key + carried values, 32-byte aligned), outputs per group, per-(partition, CTA) offsets, tables of split partitions
+				// partitioned: one record per passing row (packed key + carried values, 32-byte aligned), outputs per
+				// group, per-(partition, CTA) offsets, tables of split partitions. Whether the keys fit a table in L2
+				// shows at run time; a request admitted by this figure takes one only within it.
 				const uint64_t record = (carried + 31) / 32 * 32;
 				bytes = SatMul(c.rows, record);
 				bytes = SatAdd(bytes, SatMul(groups, out_width));

@@ -312,6 +312,12 @@ private:
 	const PlanNode *root_ = nullptr;
 	void *deferred_rows_ = nullptr;
 	int deferred_rows_bytes_ = 8;
+	//! Room for a form that takes `bytes` where the general one takes less: within the budget, and for a request that
+	//! was admitted by an estimate within that.
+	bool Room(uint64_t bytes) const {
+		return Runtime::Get().allocator().HasHeadroom(bytes) &&
+		       (options_.admitted_bytes == 0 || arena_.Bytes() + bytes <= options_.admitted_bytes);
+	}
 	//! The root's outputs stay on the device and the caller does not wait (device output, no sync): a
 	//! row count nothing after the root needs stays on the device too, read when the result's columns
 	//! are first asked for, the columns sized for `capacity_bytes` meanwhile. False when the count must
@@ -948,6 +954,8 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	// partitioned strategies. Below that size it wins at every row count, key distribution and number of
 	// aggregates measured, SUM and COUNT or SUM, SUM and MAX: 300K rows into 2^20 keys 0.11 against 0.14 ms, 20M
 	// 0.36 against 0.94 ms uniform and 0.62 against 0.94 ms Zipf(1.1), 1.34e8 skewed rows 2.1 against 2.4 ms.
+	// Few rows leave most of such a table unused: it is taken only where the budget has room for it (4096 rows into 2^22
+	// keys 0.124 against 0.143 ms, but 67 MB against 0.2).
 	// VGPU_GB_STRATEGY: "l2" or one of the partitioned ones (testing); the partition overrides keep those too.
 	PipelineCodegen::GroupBySpec gb_l2 = gb;
 	for (auto &ag : gb_l2.aggs) {
@@ -972,6 +980,15 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	          cg.L2ChainWord(gb_l2) + 1 < kKeyWord;
 	if (const char *env = std::getenv("VGPU_GB_STRATEGY")) l2 = l2 && std::strcmp(env, "l2") == 0;
 	if (std::getenv("VGPU_GB_TABLE_SLOTS") || std::getenv("VGPU_GB_PARTITIONS")) l2 = false;
+	uint64_t out_row = 0;
+	for (int c : key_cols) out_row += TypeSize(cg.visible()[c].type);
+	for (auto &ag : node.aggregates) out_row += TypeSize(ag.output_type);
+	// room for a table of `slots` of `slot` bytes in L2 with the chain of its compaction, beside the outputs
+	auto table_room = [&](uint64_t slots, uint64_t slot) {
+		const uint64_t rows = pin.spec.join_multi ? domain : std::min<uint64_t>(domain, n);
+		return Room(slots * slot + slots / 64 + (64 << 10) + rows * out_row);
+	};
+	l2 = l2 && table_room(domain, 8 * static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2)));
 	// Direct-partitioned when the packed key space is dense enough to be walked slot by slot
 	// (at most 4 slots per input row) and splits into at most 2^14 partitions of the largest
 	// shared-memory table: a row then costs no hashing and no probing.
@@ -1003,6 +1020,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	                     58 * l2_slots;
 	if (const char *env = std::getenv("VGPU_GB_STRATEGY")) l2_hashed = l2_hashed && std::strcmp(env, "l2") == 0;
 	if (std::getenv("VGPU_GB_TABLE_SLOTS") || std::getenv("VGPU_GB_PARTITIONS")) l2_hashed = false;
+	l2_hashed = l2_hashed && table_room(l2_slots, l2_slot);
 	if (!direct && !l2 && pin.spec.join_multi) {
 		// the partitioned strategies take one item per input row: expand the join's matches into a
 		// relation first, then group that

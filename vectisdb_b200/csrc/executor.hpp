@@ -44,6 +44,9 @@ struct ExecOptions {
 	int64_t cache_chunk_index = -1;
 	bool output_on_device = false;
 	bool no_sync = false;
+	//! What the execution was admitted for (0: no such figure): forms that would hold more memory than the general
+	//! ones are then only taken within it.
+	uint64_t admitted_bytes = 0;
 };
 
 struct ExecResult {

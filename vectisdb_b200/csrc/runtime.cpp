@@ -208,6 +208,12 @@ bool DeviceAllocator::HasHeadroom(uint64_t bytes) {
 	return in_use_ + bytes <= budget_;
 }
 
+uint64_t DeviceAllocator::SizeOf(void *ptr) {
+	std::lock_guard<std::mutex> lock(mu_);
+	auto it = sizes_.find(ptr);
+	return it == sizes_.end() ? 0 : it->second;
+}
+
 vgpu_memory_stats DeviceAllocator::Stats() {
 	std::lock_guard<std::mutex> lock(mu_);
 	EnsureBudgetLocked();
@@ -253,6 +259,13 @@ bool Arena::Take(void *ptr) {
 	if (it == owned_.end()) return false;
 	owned_.erase(it);
 	return true;
+}
+
+uint64_t Arena::Bytes() const {
+	auto &alloc = Runtime::Get().allocator();
+	uint64_t bytes = 0;
+	for (void *p : owned_) bytes += alloc.SizeOf(p);
+	return bytes;
 }
 
 void Arena::FreeNow(void *ptr) {

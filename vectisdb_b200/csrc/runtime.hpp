@@ -72,6 +72,8 @@ public:
 	//! requests at once reserves what they will hold together).
 	void Reserve(uint64_t bytes, cudaStream_t stream);
 	bool HasHeadroom(uint64_t bytes);
+	//! Bytes of an allocation (0: not this allocator's).
+	uint64_t SizeOf(void *ptr);
 	vgpu_memory_stats Stats();
 	//! Restarts the peak at the bytes in use now (the pool's reserve is unaffected).
 	void ResetPeak();
@@ -150,6 +152,8 @@ public:
 	//! has already handed over.
 	bool Take(void *ptr);
 	void FreeNow(void *ptr);
+	//! Bytes the arena owns.
+	uint64_t Bytes() const;
 	cudaStream_t stream() const {
 		return stream_;
 	}

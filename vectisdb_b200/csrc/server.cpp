@@ -85,6 +85,7 @@ uint64_t Server::Submit(std::shared_ptr<PlanNode> plan, std::vector<vgpu_column>
 	req->submitted = Clock::now();
 	req->est = Estimate(*req->plan, req->inputs, req->options);
 	req->info.estimated_bytes = req->est;
+	req->options.admitted_bytes = req->est;
 	// Only small requests batch: the batch launch pays off by sharing one launch among queries that are
 	// each too small to fill the GPU; a large request's own kernels fill it at least as well and run
 	// beside the other slots' work (VGPU_SERVE_BATCH_ROWS: the largest input that still batches).
@@ -197,7 +198,9 @@ void Server::WorkerLoop(int slot) {
 				BatchOptions bo;
 				bo.use_graph = false;  // compositions change from launch to launch
 				BatchStats st;
-				results = ExecutePrepared(*PrepareBatch(plans), ins, head->options, bo, stream, &st);
+				ExecOptions eo = head->options;
+				for (auto &r : job) eo.admitted_bytes = std::min(eo.admitted_bytes, r->est);
+				results = ExecutePrepared(*PrepareBatch(plans), ins, eo, bo, stream, &st);
 				batched = st.batched > 0 ? 1 : -1;
 			} catch (const Error &e) {
 				for (size_t i = 0; i < job.size(); i++) {
