@@ -549,13 +549,13 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 	bool null_outs = false;
 	for (int c : out_cols) null_outs = null_outs || cg.visible()[c].nullable;
 	// One pass or two. One pass needs room for a row per input row before it knows how many are kept: taken
-	// while that is at most 8 GiB and within the budget, and unless the plan's own estimate says that under
+	// while that is at most 8 GiB and within the budget (with as much again three times over for the operators above,
+	// where there are any), and unless the plan's own estimate says that under
 	// two rows in five survive (what the admission estimate charges for the outputs then stays near what
 	// they take). Its two staged tiles of 512 rows allow 96 bytes a row (96 KB a CTA, two CTAs per SM).
 	// VGPU_MAT_PASSES=2: always two (testing).
 	bool one_pass = cg.has_filter() && n > 0 && !pin.spec.join_multi && row_bytes > 0 && row_bytes <= 96 &&
-	                n <= (8ull << 30) / row_bytes &&
-	                Runtime::Get().allocator().HasHeadroom(n * row_bytes);
+	                n <= (8ull << 30) / row_bytes && Room((at_root ? 1 : 4) * n * row_bytes);
 	for (const PlanNode *node : pin.spec.chain) {
 		if (node->op == OpType::FILTER && node->estimated_rows && 5 * node->estimated_rows < 2 * n) one_pass = false;
 	}
@@ -580,14 +580,22 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 	uint64_t in_bytes = 0;
 	for (auto &s : pin.sources) in_bytes += s.rows * TypeSize(s.type);
 	Relation out;
-	auto add_columns = [&](KArgsHost &a, uint64_t rows) {
+	auto block_size = [&](uint64_t rows) {
+		uint64_t bytes = 0;
+		for (int c : out_cols) bytes += (rows * TypeSize(cg.visible()[c].type) + 255) / 256 * 256;
+		return bytes;
+	};
+	auto add_columns = [&](KArgsHost &a, uint64_t rows, char *block) {
+		uint64_t at = 0;
 		for (size_t c = 0; c < out_cols.size(); c++) {
 			const auto &vc = cg.visible()[out_cols[c]];
 			DevColumn col;
 			col.name = names[c];
 			col.type = vc.type;
 			col.rows = rows;
-			col.data = arena_.Alloc(rows * TypeSize(vc.type));
+			col.data = block ? block + at : arena_.Alloc(rows * TypeSize(vc.type));
+			col.block = block;
+			at += (rows * TypeSize(vc.type) + 255) / 256 * 256;
 			if (vc.nullable) {
 				col.valid = arena_.AllocT<uint8_t>(rows);
 			}
@@ -609,7 +617,8 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 		FillArgs(pin, a);
 		a.SetPtr(cb, chain);
 		a.SetWord(kWaitWord, kern::WaitLimitNs());
-		add_columns(a, n);
+		char *block = static_cast<char *>(arena_.Alloc(block_size(n)));
+		add_columns(a, n, block);
 		CUfunction f = module->Get("vgpu_mat_onepass");
 		const int occ = std::max(1, Runtime::Get().MaxActiveBlocks(f, g.block, smem));
 		LaunchGenerated(*module, "vgpu_mat_onepass",
@@ -619,19 +628,27 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 		if (at_root && !null_outs && DeferRows(chain, 8, 0)) return out;
 		out_rows = ReadU64(chain);
 		if (out_rows > n) Fail(VGPU_ERR_CUDA, "gpu_executor: a row filter's tiles were not completed in time");
-		for (auto &col : out) {
-			col.rows = out_rows;
-			// a result that keeps few of many rows does not hold on to the room for all of them
-			if (n * row_bytes > (64ull << 20) && out_rows < n / 4) {
-				auto shrink = [&](void *p, size_t width) {
-					void *q = arena_.Alloc(out_rows * width);
-					if (out_rows) VGPU_CUDA(cudaMemcpyAsync(q, p, out_rows * width, cudaMemcpyDeviceToDevice, stream_));
-					arena_.FreeNow(p);
-					return q;
-				};
-				col.data = shrink(col.data, TypeSize(col.type));
-				if (col.valid) col.valid = static_cast<uint8_t *>(shrink(col.valid, 1));
+		for (auto &col : out) col.rows = out_rows;
+		// rows that stay on the device do not hold on to the room of many more
+		const uint64_t spare = (n - out_rows) * row_bytes;
+		if ((!at_root || options_.output_on_device) && spare > (4ull << 20) && out_rows < n / 4) {
+			std::vector<kern::BufferCopy> copies;
+			char *to = static_cast<char *>(arena_.Alloc(block_size(out_rows)));
+			uint64_t at = 0;
+			for (auto &col : out) {
+				const uint64_t bytes = out_rows * TypeSize(col.type);
+				copies.push_back({col.data, to + at, bytes});
+				col.data = to + at;
+				col.block = to;
+				at += (bytes + 255) / 256 * 256;
+				if (col.valid && !at_root) {  // (the root's masks are packed next, and these freed)
+					copies.push_back({col.valid, arena_.Alloc(out_rows), out_rows});
+					col.valid = static_cast<uint8_t *>(copies.back().dst);
+				}
 			}
+			kern::CopyBuffers(copies.data(), static_cast<int>(copies.size()), stream_);
+			arena_.FreeNow(block);
+			for (auto &c : copies) arena_.FreeNow(const_cast<void *>(c.src));  // masks
 		}
 		return out;
 	}
@@ -669,7 +686,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 	KArgsHost a;
 	FillArgs(pin, a);
 	a.SetPtr(cb, tile_offsets);
-	add_columns(a, out_rows);
+	add_columns(a, out_rows, nullptr);
 	if (n > 0 && (out_rows > 0 || !cg.has_filter())) {
 		LaunchGenerated(*module, "vgpu_mat_write", grid, g.block, 0, stream_, a, 0, n);
 	}
@@ -2186,6 +2203,7 @@ ExecResult ExecutePlan(const PlanNode &plan, const std::vector<vgpu_column> &inp
 	ExecResult result;
 	result.stream = stream;
 	bool copies = false;
+	void *block = nullptr;  // the last one handed over
 	if (void *rows = ex.deferred_rows()) {
 		result.pending_rows = rows;
 		result.pending_rows_bytes = ex.deferred_rows_bytes();
@@ -2202,13 +2220,17 @@ ExecResult ExecutePlan(const PlanNode &plan, const std::vector<vgpu_column> &inp
 			// inputs, cache entries, a buffer already handed to another column) is copied, so the result
 			// never aliases memory it does not own.
 			void *d = nullptr;
-			if (bytes && ex.arena().Take(c.data)) {
+			if (bytes && c.block && (c.block == block || ex.arena().Take(c.block))) {
+				if (c.block != block) result.device_buffers.push_back(c.block);
+				block = c.block;
+				o.device_data = d = c.data;
+			} else if (bytes && ex.arena().Take(c.data)) {
 				d = c.data;
 			} else {
 				d = Runtime::Get().allocator().Alloc(bytes, stream);
 				if (bytes) VGPU_CUDA(cudaMemcpyAsync(d, c.data, bytes, cudaMemcpyDeviceToDevice, stream));
 			}
-			result.device_buffers.push_back(d);
+			if (!o.device_data) result.device_buffers.push_back(d);
 			o.device_data = d;
 			if (c.valid) {
 				const size_t vb = (c.rows + 7) / 8;

@@ -23,6 +23,7 @@ struct DevColumn {
 	bool has_stats = false;
 	int64_t min = 0, max = 0;
 	uint64_t distinct = 0;  // about how many distinct values there are, 0 = not known
+	void *block = nullptr;  // the allocation `data` lies in, when columns share one
 	std::shared_ptr<uint8_t> host;  // `data` is this page-locked memory, complete: a root result on the host
 };
 using Relation = std::vector<DevColumn>;

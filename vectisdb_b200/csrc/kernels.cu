@@ -192,6 +192,19 @@ template <typename T> __global__ void GatherKernel(const T *src, const uint32_t 
 	}
 }
 
+struct CopyArgs {
+	BufferCopy c[kMaxCopies];
+};
+
+// blockIdx.y picks the buffer. Bound by the bytes; one launch, since a few kilobytes are copied as often as not.
+__global__ void __launch_bounds__(256) CopyBuffersKernel(CopyArgs a) {
+	const BufferCopy &c = a.c[blockIdx.y];
+	const uint64_t vecs = (c.bytes + 15) / 16, stride = (uint64_t)gridDim.x * blockDim.x;
+	const uint4 *src = static_cast<const uint4 *>(c.src);
+	uint4 *dst = static_cast<uint4 *>(c.dst);
+	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < vecs; i += stride) dst[i] = src[i];
+}
+
 // Key bits zero-extended to 64 bits, minus `bias`.
 template <typename T> __global__ void WidenKernel(const T *src, uint64_t n, uint64_t bias, uint64_t *dst) {
 	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -1361,6 +1374,25 @@ void Gather(const void *src, size_t width, const uint32_t *idx, uint64_t n, void
 		Fail(VGPU_ERR_INTERNAL, "gather: unsupported width");
 	}
 	VGPU_CUDA(cudaGetLastError());
+}
+
+void CopyBuffers(const BufferCopy *copies, int n, cudaStream_t stream) {
+	for (int first = 0; first < n; first += kMaxCopies) {
+		CopyArgs a;
+		const int count = std::min(n - first, kMaxCopies);
+		uint64_t most = 0, bytes = 0;
+		for (int j = 0; j < count; j++) {
+			a.c[j] = copies[first + j];
+			most = std::max(most, a.c[j].bytes);
+			bytes += a.c[j].bytes;
+		}
+		if (most == 0) continue;
+		LaunchScope scope("copy_buffers", stream, 2 * bytes, 0);
+		const uint64_t cap = std::max<uint64_t>(1, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8 / count);
+		const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(cap, (most + 4095) / 4096));
+		CopyBuffersKernel<<<dim3(grid, static_cast<unsigned>(count)), 256, 0, stream>>>(a);
+		VGPU_CUDA(cudaGetLastError());
+	}
 }
 
 void WidenKeys(const void *src, size_t width, uint64_t n, uint64_t bias, uint64_t *dst, cudaStream_t stream) {

@@ -29,6 +29,16 @@ void PackValidity(const uint8_t *bytes, uint8_t *bitmap, uint64_t n, cudaStream_
 //! dst[o] = src[idx[o]] for `width`-byte values (1, 2, 4, 8 or 16).
 void Gather(const void *src, size_t width, const uint32_t *idx, uint64_t n, void *dst, cudaStream_t stream);
 
+//! Several buffers copied in one launch per kMaxCopies of them: sources and destinations 16-byte aligned, with room up
+//! to the next multiple of 16 bytes.
+constexpr int kMaxCopies = 24;
+struct BufferCopy {
+	const void *src;
+	void *dst;
+	uint64_t bytes;
+};
+void CopyBuffers(const BufferCopy *copies, int n, cudaStream_t stream);
+
 //! Raw key bits zero-extended to 64 bits (the reference's WidenKeyKernel semantics,
 //! cuda_engine/src/operators/gpu_groupby.cu:76-94), minus `bias`.
 void WidenKeys(const void *src, size_t width, uint64_t n, uint64_t bias, uint64_t *dst, cudaStream_t stream);
