@@ -2074,6 +2074,8 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	// 2^16 matches (one CTA writes a tile: at 64 matches a row the longest one still takes microseconds; past
 	// that the expansion below spreads a row's matches over many CTAs). Dense right keys need no sort.
 	const bool tiled = sources.size() <= static_cast<size_t>(kern::kMaxJoinOuts);
+	uint64_t out_width = 0;
+	for (auto *c : sources) out_width += TypeSize(c->type);
 	// two words for JoinDenseRuns' info, then the chain of the count: read back together
 	uint64_t *info = tiled ? arena_.AllocT<uint64_t>(2 + kern::JoinChainWords(ln)) : nullptr;
 	uint64_t *chain = info + 2;
@@ -2084,6 +2086,7 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 		if ((head[2] >> 62) != 0 || (head[3] >> 32) > (1u << 16)) return false;
 		const uint64_t total = head[2];
 		if (total > kMaxOutputRows) too_large(total);
+		if (view.entries && !Room(total * out_width)) return false;  // the sort gives its buffers back before the outputs
 		out = make_out(total);
 		if (total == 0) return true;
 		// Where each right row has four matches or more on average, the right columns are put in run order first, so
@@ -2107,7 +2110,8 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 		kern::JoinEmit(lk.data, kw, ln, view, chain, ordered ? nullptr : rows, outs, total, stream_);
 		return true;
 	};
-	if (tiled && dense) {
+	// (at 8 bytes a key value that is up to 36 bytes a right row, the sort 24: only where there is room)
+	if (tiled && dense && Room((range + 1) * 8 + rn * 4 + rn / 4 + 4096)) {
 		uint64_t *entries = arena_.AllocT<uint64_t>(range + 1);
 		uint32_t *rows = arena_.AllocT<uint32_t>(rn);
 		uint32_t *list = arena_.AllocT<uint32_t>(rn / 17 + 1);
@@ -2120,6 +2124,7 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 		if (emit_tiles(view, rows, out)) return out;
 		arena_.FreeNow(entries);
 		arena_.FreeNow(rows);
+		arena_.FreeNow(list);
 	}
 	uint64_t *rw = arena_.AllocT<uint64_t>(rn);
 	kern::WidenKeys(rk.data, kw, rn, bias, rw, stream_);
