@@ -50,7 +50,8 @@ static void atomicMax(uint32_t *p, uint32_t v) {
 template <typename T> static void st_relaxed(T *p, T v) { *p = v; }
 template <typename... A> static u64 tile_scanner(A...) { return 0; }  // the CTA below is not the scanning one
 template <typename... A> static void tiles_total(A...) {}
-struct JoinRunsView {};
+constexpr uint32_t kJoinRunLimit = 4096;
+struct JoinRunsView { const uint32_t *info = nullptr; };
 struct uint2 { uint32_t x, y; };
 static uint2 JoinRunOf(const JoinRunsView &, uint64_t key) { return {0, static_cast<uint32_t>(key)}; }  // key = matches
 """

@@ -12,6 +12,7 @@
 #include "executor.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -2058,12 +2059,15 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	}
 	if (ln >= (1ull << 32) || rn >= (1ull << 32)) Fail(VGPU_ERR_UNSUPPORTED, "gpu_hash_join: side too large");
 	const size_t kw = TypeSize(lk.type);
-	uint64_t *words = arena_.AllocT<uint64_t>(2);
+	uint64_t *words = arena_.AllocT<uint64_t>(4);
 	const kern::BoundsColumn want {rk.data, rn, kern::RawBoundsKind(kw)};
-	kern::ColumnBounds(&want, 1, words, stream_);
-	const std::vector<uint64_t> bounds = ReadWords(words, 2);
+	kern::ColumnBounds(&want, 1, words, stream_, false, words + 2);
+	const std::vector<uint64_t> bounds = ReadWords(words, 4);
 	const uint64_t bias = kern::BoundsLow(bounds.data(), want.kind);
 	const uint64_t range = kern::BoundsHigh(bounds.data(), want.kind) - bias;
+	// About how many right rows share a right row's key, on the mean over the rows: one key in a tenth of them counts for
+	// a hundredth of all rows.
+	const double shared = bounds[3] ? static_cast<double>(rn) * bounds[2] / bounds[3] : 0;
 	const int bits = BitsFor(range);
 	const bool dense = range < (1ull << 28) && range < 4 * rn;
 	auto too_large = [](uint64_t rows) {
@@ -2072,20 +2076,32 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 	};
 	// Matches written by tiles of left rows: for up to 16 output columns, while no tile of 1024 left rows has over
 	// 2^16 matches (one CTA writes a tile: at 64 matches a row the longest one still takes microseconds; past
-	// that the expansion below spreads a row's matches over many CTAs). Dense right keys need no sort.
-	const bool tiled = sources.size() <= static_cast<size_t>(kern::kMaxJoinOuts);
+	// that the expansion below spreads a row's matches over many CTAs), and not where a row's matches are sure to be
+	// more (the count and its read-back would be lost).
+	// Dense right keys need no sort, but rows of one key queue at its entry and are put in order by themselves: grouping
+	// pays up to some 16 rows a key (1M right rows, 2, 16, 24 and 64 to a key: 0.17, 0.24, 0.33 and 0.51 ms, sorted 0.31, 0.26,
+	// 0.26 and 0.25), and not where few keys have many of them (half of 4M rows on one key: 3.2 ms, sorted 0.44). Under
+	// 2^15 rows a run may be as long as the grouping takes.
+	const bool small = rn < (1u << 15) && std::sqrt(shared * static_cast<double>(rn)) <= 5000;
+	const bool tiled = sources.size() <= static_cast<size_t>(kern::kMaxJoinOuts) && rn <= 64 * (range + 1) && (shared <= 128 || small);
+	const bool grouped = tiled && dense && rn <= 16 * (range + 1) && (shared <= 16 || small);
 	uint64_t out_width = 0;
 	for (auto *c : sources) out_width += TypeSize(c->type);
 	// two words for JoinDenseRuns' info, then the chain of the count: read back together
 	uint64_t *info = tiled ? arena_.AllocT<uint64_t>(2 + kern::JoinChainWords(ln)) : nullptr;
 	uint64_t *chain = info + 2;
-	auto emit_tiles = [&](const kern::JoinRunsView &view, const uint32_t *rows, Relation &out) {
+	// false: not written; *expand then tells whether the view will do for the expansion
+	auto emit_tiles = [&](const kern::JoinRunsView &view, const uint32_t *rows, Relation &out, bool *expand) {
 		kern::JoinCountMatches(lk.data, kw, ln, view, chain, stream_);
 		const std::vector<uint64_t> head = ReadWords(info, 4);
 		if (view.entries && (head[0] >> 32) > kern::kJoinRunLimit) return false;  // a run not in row order
-		if ((head[2] >> 62) != 0 || (head[3] >> 32) > (1u << 16)) return false;
+		if ((head[2] >> 62) != 0) return false;
 		const uint64_t total = head[2];
 		if (total > kMaxOutputRows) too_large(total);
+		if ((head[3] >> 32) > (1u << 16)) {
+			*expand = Room(16 * ln + total * (8 + out_width));
+			return false;
+		}
 		if (view.entries && !Room(total * out_width)) return false;  // the sort gives its buffers back before the outputs
 		out = make_out(total);
 		if (total == 0) return true;
@@ -2095,7 +2111,7 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 		// 0.090 -> 0.073 for 0.018. Not below a million matches, nor when memory is short.
 		uint64_t right_bytes = 0;
 		for (size_t i = 0; i < sources.size(); i++) right_bytes += from_left[i] ? 0 : rn * TypeSize(sources[i]->type);
-		const bool ordered = total / 4 >= rn && total >= (1u << 20) && Runtime::Get().allocator().HasHeadroom(right_bytes);
+		const bool ordered = total / 4 >= rn && total >= (1u << 20) && Room(right_bytes);
 		kern::JoinOuts outs;
 		for (size_t i = 0; i < sources.size(); i++) {
 			const size_t width = TypeSize(sources[i]->type);
@@ -2107,54 +2123,61 @@ Relation Executor::JoinMaterialize(const PlanNode &node, Relation &left, Relatio
 			}
 			outs.c[outs.n++] = {src, out[i].data, static_cast<int>(width), !from_left[i]};
 		}
-		kern::JoinEmit(lk.data, kw, ln, view, chain, ordered ? nullptr : rows, outs, total, stream_);
+		kern::JoinEmit(lk.data, kw, ln, view, chain, ordered ? nullptr : rows, outs, total,
+		               static_cast<uint32_t>(head[3] >> 32), stream_);
 		return true;
 	};
+	kern::JoinRunsView view;
+	uint32_t *perm = nullptr;  // the right rows in the view's order
 	// (at 8 bytes a key value that is up to 36 bytes a right row, the sort 24: only where there is room)
-	if (tiled && dense && Room((range + 1) * 8 + rn * 4 + rn / 4 + 4096)) {
+	if (grouped && Room((range + 1) * 8 + rn * 4 + rn / 4 + 4096)) {
 		uint64_t *entries = arena_.AllocT<uint64_t>(range + 1);
 		uint32_t *rows = arena_.AllocT<uint32_t>(rn);
 		uint32_t *list = arena_.AllocT<uint32_t>(rn / 17 + 1);
 		kern::JoinDenseRuns(rk.data, kw, rn, bias, range, entries, rows, list, reinterpret_cast<uint32_t *>(info), stream_);
-		kern::JoinRunsView view;
 		view.entries = entries;
 		view.nb = range + 1;
 		view.bias = bias;
+		view.info = reinterpret_cast<const uint32_t *>(info);
 		Relation out;
-		if (emit_tiles(view, rows, out)) return out;
-		arena_.FreeNow(entries);
-		arena_.FreeNow(rows);
+		bool expand = false;
+		if (emit_tiles(view, rows, out, &expand)) return out;
+		if (expand) {
+			perm = rows;
+		} else {
+			arena_.FreeNow(entries);
+			arena_.FreeNow(rows);
+		}
 		arena_.FreeNow(list);
 	}
-	uint64_t *rw = arena_.AllocT<uint64_t>(rn);
-	kern::WidenKeys(rk.data, kw, rn, bias, rw, stream_);
-	uint32_t *perm = arena_.AllocT<uint32_t>(rn);
-	uint64_t *rw_alt = arena_.AllocT<uint64_t>(rn);
-	uint32_t *perm_alt = arena_.AllocT<uint32_t>(rn);
-	kern::RadixSortPairs(rw, perm, rw_alt, perm_alt, rn, bits, arena_);
-	arena_.FreeNow(rw_alt);
-	arena_.FreeNow(perm_alt);
-	// each left key's run of equal right keys through a radix directory: one bucket per key value when
-	// the key range is dense (the run is read, not searched), else 2^22 buckets and a short search
-	const uint32_t shift = dense ? 0u : bits > 22 ? static_cast<uint32_t>(bits - 22) : 0u;
-	const uint64_t nb = (range >> shift) + 1;
-	uint32_t *dir = arena_.AllocT<uint32_t>(nb + 1);
-	kern::JoinDirectory(rw, rn, shift, nb, dir, stream_);
-	if (tiled && !dense) {
-		kern::JoinRunsView view;
+	if (!perm) {
+		uint64_t *rw = arena_.AllocT<uint64_t>(rn);
+		kern::WidenKeys(rk.data, kw, rn, bias, rw, stream_);
+		perm = arena_.AllocT<uint32_t>(rn);
+		uint64_t *rw_alt = arena_.AllocT<uint64_t>(rn);
+		uint32_t *perm_alt = arena_.AllocT<uint32_t>(rn);
+		kern::RadixSortPairs(rw, perm, rw_alt, perm_alt, rn, bits, arena_);
+		arena_.FreeNow(rw_alt);
+		arena_.FreeNow(perm_alt);
+		// each left key's run of equal right keys through a radix directory: one bucket per key value when
+		// the key range is dense (the run is read, not searched), else 2^22 buckets and a short search
+		const uint32_t shift = dense ? 0u : bits > 22 ? static_cast<uint32_t>(bits - 22) : 0u;
+		const uint64_t nb = (range >> shift) + 1;
+		uint32_t *dir = arena_.AllocT<uint32_t>(nb + 1);
+		kern::JoinDirectory(rw, rn, shift, nb, dir, stream_);
+		view = kern::JoinRunsView();
 		view.sorted = rw;
 		view.dir = dir;
 		view.nb = nb;
 		view.bias = bias;
 		view.shift = shift;
 		Relation out;
-		if (emit_tiles(view, perm, out)) return out;
+		bool expand = false;
+		if (tiled && emit_tiles(view, perm, out, &expand)) return out;
 	}
-	uint64_t *lw = arena_.AllocT<uint64_t>(ln);
-	kern::WidenKeys(lk.data, kw, ln, 0, lw, stream_);
 	uint64_t *lower = arena_.AllocT<uint64_t>(ln);
 	uint64_t *counts = arena_.AllocT<uint64_t>(ln);
-	kern::JoinRuns(lw, ln, rw, dir, nb, shift, bias, lower, counts, stream_);
+	kern::JoinRuns(lk.data, kw, ln, view, lower, counts, stream_);
 	uint64_t *total = arena_.AllocT<uint64_t>(1);
 	kern::ExclusiveScanU64(counts, counts, ln, total, arena_);
 	const uint64_t total_rows = ReadU64(total);

@@ -233,6 +233,7 @@ struct BoundsArgs {
 	BoundsColumn c[kMaxBoundsColumns];
 	unsigned long long *out;
 	unsigned int *ranks;  // kDistinctRanks per column, or null
+	unsigned long long *pairs;  // two words per column, or null
 };
 
 // Out of line: few values come here, and the kernel's eight unrolled readers stay small.
@@ -243,13 +244,13 @@ __device__ __noinline__ void NoteValue(u64 v, uint32_t *ranks) {
 	if (*reinterpret_cast<volatile uint32_t *>(r) < rank) atomicMax(r, rank);
 }
 
-template <typename T, bool kBool>
-__device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx, uint32_t *ranks) {
+template <typename T, bool kBool, bool kPairs>
+__device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx, uint32_t *ranks, uint2 &seen) {
 	auto take = [&](T v) {
 		if constexpr (kBool) v = v != 0 ? 1 : 0;
 		mn = v < mn ? v : mn;
 		mx = v > mx ? v : mx;
-		if constexpr (sizeof(T) >= 4) {
+		if constexpr (sizeof(T) >= 4 && !kPairs) {
 			u32 w = static_cast<u32>(v);
 			if constexpr (sizeof(T) == 8) w ^= static_cast<u32>(static_cast<u64>(v) >> 32);
 			if (w * 0x9e3779b1u < (1u << (32 - kDistinctShift)) && ranks) NoteValue(static_cast<u64>(v), ranks);
@@ -278,15 +279,25 @@ __device__ __forceinline__ void RangeOf(const T *p, uint64_t n, T &mn, T &mx, ui
 		take4(b);
 		take4(c);
 		take4(d);
+		if constexpr (kPairs) {
+			T x[kPer], y[kPer], z[kPer], w[kPer];
+			memcpy(x, &a, 16);
+			memcpy(y, &b, 16);
+			memcpy(z, &c, 16);
+			memcpy(w, &d, 16);
+#pragma unroll
+			for (uint64_t j = 0; j < kPer; j++) seen.x += (x[j] == y[j] ? 1u : 0u) + (z[j] == w[j] ? 1u : 0u);
+			seen.y += 2 * kPer;
+		}
 	}
 	for (; i < vecs; i += stride) take4(v[i]);
 }
 
-template <typename T, bool kBool = false>
+template <typename T, bool kPairs, bool kBool = false>
 __device__ __forceinline__ void RangeImage(const void *p, uint64_t n, unsigned long long &lo, unsigned long long &hi,
-                                           uint32_t *ranks) {
+                                           uint32_t *ranks, uint2 &seen) {
 	T mn = std::numeric_limits<T>::max(), mx = std::numeric_limits<T>::lowest();
-	RangeOf<T, kBool>(static_cast<const T *>(p), n, mn, mx, ranks);
+	RangeOf<T, kBool, kPairs>(static_cast<const T *>(p), n, mn, mx, ranks, seen);
 	constexpr unsigned long long kFlip = std::is_signed<T>::value ? 1ull << 63 : 0ull;
 	const bool any = mn <= mx;  // a thread without values leaves the identity
 	lo = any ? static_cast<unsigned long long>(mn) ^ kFlip : ~0ull;
@@ -295,23 +306,24 @@ __device__ __forceinline__ void RangeImage(const void *p, uint64_t n, unsigned l
 
 constexpr int kBoundsBlock = 256;
 
-__global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a) {
+template <bool kPairs> __global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a) {
 	const BoundsColumn &c = a.c[blockIdx.y];
 	unsigned long long lo = ~0ull, hi = 0ull;
 	__shared__ uint32_t shared_ranks[kDistinctRanks];
 	static_assert(kDistinctRanks == kBoundsBlock, "one rank per thread");
 	shared_ranks[threadIdx.x] = 0;
 	uint32_t *ranks = a.ranks ? shared_ranks : nullptr;
+	uint2 seen = make_uint2(0, 0);  // equal pairs, pairs
 	__syncthreads();
 	switch (c.kind) {
-	case BoundsKind::U8: RangeImage<uint8_t>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::U16: RangeImage<uint16_t>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::U32: RangeImage<uint32_t>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::U64: RangeImage<unsigned long long>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::I16: RangeImage<int16_t>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::I32: RangeImage<int32_t>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::I64: RangeImage<long long>(c.data, c.rows, lo, hi, ranks); break;
-	case BoundsKind::BOOL: RangeImage<uint8_t, true>(c.data, c.rows, lo, hi, ranks); break;
+	case BoundsKind::U8: RangeImage<uint8_t, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::U16: RangeImage<uint16_t, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::U32: RangeImage<uint32_t, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::U64: RangeImage<unsigned long long, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::I16: RangeImage<int16_t, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::I32: RangeImage<int32_t, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::I64: RangeImage<long long, kPairs>(c.data, c.rows, lo, hi, ranks, seen); break;
+	case BoundsKind::BOOL: RangeImage<uint8_t, kPairs, true>(c.data, c.rows, lo, hi, ranks, seen); break;
 	}
 	__shared__ unsigned long long slo[kBoundsBlock / 32], shi[kBoundsBlock / 32];
 	for (int o = 16; o > 0; o >>= 1) {
@@ -319,11 +331,26 @@ __global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a)
 		lo = x < lo ? x : lo;
 		hi = y > hi ? y : hi;
 	}
+	__shared__ uint2 sseen[kBoundsBlock / 32];
+	if constexpr (kPairs) {
+		seen.x = __reduce_add_sync(0xffffffffu, seen.x);
+		seen.y = __reduce_add_sync(0xffffffffu, seen.y);
+	}
 	if ((threadIdx.x & 31) == 0) {
 		slo[threadIdx.x >> 5] = lo;
 		shi[threadIdx.x >> 5] = hi;
+		sseen[threadIdx.x >> 5] = seen;
 	}
 	__syncthreads();
+	if (kPairs && threadIdx.x == 32) {
+		unsigned long long equal = 0, all = 0;
+		for (int w = 0; w < kBoundsBlock / 32; w++) {
+			equal += sseen[w].x;
+			all += sseen[w].y;
+		}
+		if (equal) atomicAdd(a.pairs + 2 * blockIdx.y, equal);
+		if (all) atomicAdd(a.pairs + 2 * blockIdx.y + 1, all);
+	}
 	if (threadIdx.x == 0) {
 		for (int w = 1; w < kBoundsBlock / 32; w++) {
 			lo = slo[w] < lo ? slo[w] : lo;
@@ -332,7 +359,7 @@ __global__ void __launch_bounds__(kBoundsBlock) ColumnBoundsKernel(BoundsArgs a)
 		atomicMax(a.out + 2 * blockIdx.y, ~lo);
 		atomicMax(a.out + 2 * blockIdx.y + 1, hi);
 	}
-	if (a.ranks) {  // (the values were all taken before the barrier above)
+	if (!kPairs && a.ranks) {  // (the values were all taken before the barrier above)
 		// few CTAs raise a rank the others have raised before: looked at first (a thousand CTAs' atomics on the
 		// same eight lines took 20 us)
 		unsigned int *to = a.ranks + blockIdx.y * kDistinctRanks + threadIdx.x;
@@ -563,17 +590,42 @@ __global__ void __launch_bounds__(kExpandBlock) JoinExpandKernel(const uint64_t 
 // columns out, 0.574 ms of kernels by sorting, offsets, expansion and a gather per column, 0.221 ms here (the emit pass, bound
 // by random reads of 8-byte right values, 0.113 ms; 0.088 with the values in run order, see the caller).
 
-// Dense keys: an entry per key value, x = end of its run in `rows`, y = its length.
-template <typename K> __global__ void JoinEntryCountKernel(const K *keys, uint64_t n, uint64_t bias, uint2 *entries) {
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		atomicAdd(&entries[static_cast<uint64_t>(keys[i]) - bias].y, 1u);
+// info of the kernels below: [0] runs listed for the last of them, [1] the longest run, [2] the cursor of the runs'
+// places; zero at the first launch. A run past kJoinRunLimit makes the result useless: from then on they return.
+__device__ __forceinline__ bool JoinRunTooLong(const uint32_t *info) {
+	return *reinterpret_cast<const volatile uint32_t *>(info + 1) > kJoinRunLimit;
+}
+
+// Dense keys: an entry per key value, x = end of its run in `rows`, y = its length. Adds to one entry queue at its
+// address (0.7 ns each: a key in every second of 4M rows held this kernel for 1.4 ms), so a warp with equal
+// neighbours adds each of its keys once and looks at the counts it meets: the pass ends soon after one is too long.
+template <typename K>
+__global__ void JoinEntryCountKernel(const K *keys, uint64_t n, uint64_t bias, uint2 *entries, uint32_t *info) {
+	const uint32_t lane = threadIdx.x & 31;
+	for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); w < n; w += (uint64_t)gridDim.x * blockDim.x) {
+		if (__any_sync(0xffffffffu, JoinRunTooLong(info))) return;
+		const uint64_t i = w + lane;
+		const uint64_t k = static_cast<uint64_t>(keys[i < n ? i : n - 1]) - bias;
+		const uint64_t next = __shfl_down_sync(0xffffffffu, k, 1);
+		const uint32_t live = __ballot_sync(0xffffffffu, i < n);
+		if (__any_sync(0xffffffffu, lane < 31 && i + 1 < n && next == k)) {
+			const uint32_t peers = __match_any_sync(0xffffffffu, k) & live;
+			if (i < n && static_cast<uint32_t>(__ffs(peers) - 1) == lane) {
+				const uint32_t count = atomicAdd(&entries[k].y, __popc(peers)) + __popc(peers);
+				if (count > kJoinRunLimit) atomicMax(info + 1, count);
+			}
+		} else if (i < n) {
+			atomicAdd(&entries[k].y, 1u);
+		}
 	}
 }
 
 // Runs laid out tile by tile in whatever order the tiles arrive (a run's place does not matter); entry x becomes
-// its start. *cursor zero at launch.
-__global__ void __launch_bounds__(256) JoinEntryPlaceKernel(uint2 *entries, uint64_t count, uint32_t *cursor) {
+// its start.
+__global__ void __launch_bounds__(256) JoinEntryPlaceKernel(uint2 *entries, uint64_t count, uint32_t *info) {
 	__shared__ uint32_t scratch[33], base;
+	if (__syncthreads_or(JoinRunTooLong(info))) return;
+	uint32_t longest = 0;
 	for (uint64_t first = blockIdx.x * 1024ull; first < count; first += gridDim.x * 1024ull) {
 		const uint64_t i = first + threadIdx.x * 4ull;
 		uint32_t c[4], sum = 0;
@@ -581,10 +633,11 @@ __global__ void __launch_bounds__(256) JoinEntryPlaceKernel(uint2 *entries, uint
 		for (int j = 0; j < 4; j++) {
 			c[j] = i + j < count ? entries[i + j].y : 0u;
 			sum += c[j];
+			longest = max(longest, c[j]);
 		}
 		uint32_t total;
 		uint32_t at = BlockScanExclusive<uint32_t>(sum, scratch, &total);
-		if (threadIdx.x == 0) base = total ? atomicAdd(cursor, total) : 0u;
+		if (threadIdx.x == 0) base = total ? atomicAdd(info + 2, total) : 0u;
 		__syncthreads();
 		at += base;
 #pragma unroll
@@ -594,25 +647,37 @@ __global__ void __launch_bounds__(256) JoinEntryPlaceKernel(uint2 *entries, uint
 		}
 		__syncthreads();
 	}
+	longest = __reduce_max_sync(0xffffffffu, longest);
+	if ((threadIdx.x & 31) == 0 && longest > *reinterpret_cast<volatile uint32_t *>(info + 1)) atomicMax(info + 1, longest);
 }
 
 // Each right row's number into its key's run, in any order; entry x moves to the run's end.
 template <typename K>
-__global__ void JoinEntryFillKernel(const K *keys, uint64_t n, uint64_t bias, uint2 *entries, uint32_t *rows) {
+__global__ void JoinEntryFillKernel(const K *keys, uint64_t n, uint64_t bias, uint2 *entries, uint32_t *rows,
+                                    const uint32_t *info) {
+	if (JoinRunTooLong(info)) return;
 	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
 		rows[atomicAdd(&entries[static_cast<uint64_t>(keys[i]) - bias].x, 1u)] = static_cast<uint32_t>(i);
 	}
 }
 
 // Row order within the runs. A thread sorts a run of up to 16 rows in registers and local memory; longer ones
-// go to a list for the kernel after, one CTA each. info: [0] listed runs, [1] the longest run.
-constexpr uint32_t kRunShort = 16;
+// go to a list for the kernel after.
+constexpr uint32_t kRunShort = 16, kRunWarp = 256;
 
 __global__ void JoinEntrySortKernel(const uint2 *entries, uint64_t count, uint32_t *rows, uint32_t *list, uint32_t *info) {
-	uint32_t longest = 0;
-	for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < count; k += (uint64_t)gridDim.x * blockDim.x) {
-		const uint2 e = entries[k];
-		longest = max(longest, e.y);
+	if (JoinRunTooLong(info)) return;
+	const uint32_t lane = threadIdx.x & 31;
+	for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); w < count; w += (uint64_t)gridDim.x * blockDim.x) {
+		const uint64_t k = w + lane;
+		const uint2 e = k < count ? entries[k] : make_uint2(0, 0);
+		const uint32_t listed = __ballot_sync(0xffffffffu, e.y > kRunShort);
+		if (listed) {
+			uint32_t at = 0;
+			if (lane == 0) at = atomicAdd(info, __popc(listed));
+			at = __shfl_sync(0xffffffffu, at, 0);
+			if (e.y > kRunShort) list[at + __popc(listed & ((1u << lane) - 1))] = static_cast<uint32_t>(k);
+		}
 		if (e.y < 2) continue;
 		uint32_t *r = rows + (e.x - e.y);
 		if (e.y == 2) {
@@ -630,20 +695,55 @@ __global__ void JoinEntrySortKernel(const uint2 *entries, uint64_t count, uint32
 				v[j] = x;
 			}
 			for (uint32_t i = 0; i < e.y; i++) r[i] = v[i];
-		} else if (e.y <= kJoinRunLimit) {
-			list[atomicAdd(info, 1u)] = static_cast<uint32_t>(k);
 		}
 	}
-	longest = __reduce_max_sync(0xffffffffu, longest);
-	if ((threadIdx.x & 31) == 0 && longest > info[1]) atomicMax(info + 1, longest);
 }
 
-// A CTA per listed run, sorted in shared memory by a bitonic network over the next power of two.
+// Listed runs. Up to 256 rows a warp ranks them: a row's place is the number of smaller ones (row numbers differ),
+// counted while the others pass by. Longer ones a CTA sorts in shared memory by a bitonic network over the next power
+// of two.
 __global__ void __launch_bounds__(256) JoinEntrySortLongKernel(const uint2 *entries, uint32_t *rows, const uint32_t *list,
                                                               const uint32_t *info) {
 	__shared__ uint32_t v[kJoinRunLimit];
+	if (__syncthreads_or(JoinRunTooLong(info))) return;
+	const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+	for (uint32_t item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < info[0]; item += warps) {
+		const uint2 e = entries[list[item]];
+		if (e.y > kRunWarp) continue;
+		uint32_t *r = rows + (e.x - e.y);
+		if (e.y <= 32) {
+			const uint32_t own = lane < e.y ? r[lane] : 0xffffffffu;
+			uint32_t rank = 0;
+#pragma unroll
+			for (int l = 0; l < 32; l++) rank += __shfl_sync(0xffffffffu, own, l) < own ? 1u : 0u;
+			if (lane < e.y) r[rank] = own;
+			continue;
+		}
+		constexpr int kEach = kRunWarp / 32;
+		uint32_t own[kEach], rank[kEach];
+#pragma unroll
+		for (int j = 0; j < kEach; j++) {
+			own[j] = j * 32 + lane < e.y ? r[j * 32 + lane] : 0xffffffffu;
+			rank[j] = 0;
+		}
+#pragma unroll
+		for (int s = 0; s < kEach; s++) {
+			if (s * 32 >= e.y) break;
+			for (int l = 0; l < 32; l++) {  // (rows past the run's end are above every row)
+				const uint32_t other = __shfl_sync(0xffffffffu, own[s], l);
+#pragma unroll
+				for (int j = 0; j < kEach; j++) rank[j] += other < own[j] ? 1u : 0u;
+			}
+		}
+		__syncwarp();
+#pragma unroll
+		for (int j = 0; j < kEach; j++) {
+			if (j * 32 + lane < e.y) r[rank[j]] = own[j];
+		}
+	}
 	for (uint32_t item = blockIdx.x; item < info[0]; item += gridDim.x) {
 		const uint2 e = entries[list[item]];
+		if (e.y <= kRunWarp) continue;
 		uint32_t *r = rows + (e.x - e.y);
 		const uint32_t size = 1u << (32 - __clz(e.y - 1));
 		for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) v[i] = i < e.y ? r[i] : 0xffffffffu;
@@ -694,6 +794,7 @@ __global__ void __launch_bounds__(kJoinBlock) JoinMatchCountKernel(const K *keys
 	uint32_t *words = reinterpret_cast<uint32_t *>(chain + 1);
 	u32 *counts = reinterpret_cast<u32 *>(chain + 2);
 	u64 *starts = reinterpret_cast<u64 *>(chain + 2 + (ntiles + 1) / 2);
+	if (view.info && *(view.info + 1) > kJoinRunLimit) return;  // (written by earlier launches)
 	if (threadIdx.x == 0) next = atomicAdd(words, 1u);
 	__syncthreads();
 	const uint32_t ticket = next;
@@ -738,9 +839,12 @@ template <typename T> __device__ __forceinline__ void JoinCopy(const JoinOut &c,
 
 template <typename K>
 __global__ void __launch_bounds__(kJoinBlock) JoinEmitKernel(const K *keys, uint64_t n, JoinRunsView view, uint64_t ntiles,
-                                                            const uint64_t *starts, const uint32_t *rows, JoinOuts outs) {
+                                                            const uint64_t *starts, const uint32_t *rows, JoinOuts outs,
+                                                            uint32_t parts) {
 	__shared__ uint32_t scratch[33], offset[kJoinTile], first[kJoinTile];
-	for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+	for (uint64_t item = blockIdx.x; item < ntiles * parts; item += gridDim.x) {
+		const uint64_t tile = item / parts;
+		const uint32_t part = static_cast<uint32_t>(item % parts);
 		const uint64_t row0 = tile * kJoinTile + threadIdx.x * static_cast<uint64_t>(kJoinItems);
 		K k[kJoinItems];
 #pragma unroll
@@ -762,7 +866,7 @@ __global__ void __launch_bounds__(kJoinBlock) JoinEmitKernel(const K *keys, uint
 		}
 		__syncthreads();
 		const uint64_t base = starts[tile] - 1;
-		for (uint32_t o = threadIdx.x; o < total; o += kJoinBlock) {
+		for (uint32_t o = part * kJoinBlock + threadIdx.x; o < total; o += kJoinBlock * parts) {
 			uint32_t r = 0;  // the last row whose matches start at or before o (rows without any share their start)
 #pragma unroll
 			for (uint32_t step = kJoinTile / 2; step > 0; step >>= 1) r += offset[r + step] <= o ? step : 0u;
@@ -784,37 +888,13 @@ __global__ void __launch_bounds__(kJoinBlock) JoinEmitKernel(const K *keys, uint
 	}
 }
 
-// Each probe key's run in the sorted right keys through a radix directory (see vgpu_join_run): shift 0
-// indexes the directory by the key itself, so the run is read, not searched.
-__global__ void JoinRunKernel(const uint64_t *probe, uint64_t n_probe, const uint64_t *sorted, const uint32_t *dir,
-                              uint64_t nb, uint32_t shift, uint64_t bias, uint64_t *lower, uint64_t *count) {
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_probe; i += (uint64_t)gridDim.x * blockDim.x) {
-		const uint64_t k = probe[i] - bias;  // below the bias wraps past every bucket: no match
-		const uint64_t b = k >> shift;
-		uint64_t lo = 0, c = 0;
-		if (b < nb) {
-			uint64_t a = dir[b], e = dir[b + 1];
-			if (shift != 0) {
-				uint64_t hi = e;
-				while (a < hi) {
-					const uint64_t mid = (a + hi) >> 1;
-					if (sorted[mid] < k) a = mid + 1;
-					else hi = mid;
-				}
-				uint64_t up = a;
-				hi = e;
-				while (up < hi) {
-					const uint64_t mid = (up + hi) >> 1;
-					if (sorted[mid] <= k) up = mid + 1;
-					else hi = mid;
-				}
-				e = up;
-			}
-			lo = a;
-			c = e - a;
-		}
-		lower[i] = lo;
-		count[i] = c;
+// Each left key's run: its first place in the right rows' order, and its length.
+template <typename K>
+__global__ void JoinRunKernel(const K *keys, uint64_t n, JoinRunsView view, uint64_t *lower, uint64_t *count) {
+	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+		const uint2 run = JoinRunOf(view, static_cast<uint64_t>(keys[i]));
+		lower[i] = run.x;
+		count[i] = run.y;
 	}
 }
 
@@ -1072,8 +1152,10 @@ void JoinDenseFill(const void *keys, size_t kwidth, const void *values, size_t v
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream, bool distinct) {
+void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream, bool distinct, uint64_t *pairs) {
 	if (n <= 0) return;
+	if (pairs && distinct) Fail(VGPU_ERR_INTERNAL, "column bounds: distinct counts or pairs, not both");
+	if (pairs) VGPU_CUDA(cudaMemsetAsync(pairs, 0, static_cast<size_t>(n) * 16, stream));
 	VGPU_CUDA(cudaMemsetAsync(out, 0, BoundsWords(n, distinct) * 8, stream));
 	unsigned int *ranks = distinct ? reinterpret_cast<unsigned int *>(out + 2 * n) : nullptr;
 	for (int first = 0; first < n; first += kMaxBoundsColumns) {
@@ -1090,11 +1172,14 @@ void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t s
 		if (widest == 0) continue;
 		a.out = reinterpret_cast<unsigned long long *>(out + 2 * first);
 		a.ranks = ranks ? ranks + static_cast<size_t>(first) * kDistinctRanks : nullptr;
+		a.pairs = pairs ? reinterpret_cast<unsigned long long *>(pairs + 2 * first) : nullptr;
 		LaunchScope scope("column_bounds", stream, bytes, rows);
 		// four 16-byte loads per thread, at most eight CTAs per SM over all columns
 		const uint64_t cap = std::max<uint64_t>(1, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8 / count);
 		const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(cap, (widest + kBoundsBlock * 64 - 1) / (kBoundsBlock * 64)));
-		ColumnBoundsKernel<<<dim3(grid, static_cast<unsigned>(count)), kBoundsBlock, 0, stream>>>(a);
+		const dim3 ctas(grid, static_cast<unsigned>(count));
+		if (pairs) ColumnBoundsKernel<true><<<ctas, kBoundsBlock, 0, stream>>>(a);
+		else ColumnBoundsKernel<false><<<ctas, kBoundsBlock, 0, stream>>>(a);
 		VGPU_CUDA(cudaGetLastError());
 	}
 }
@@ -1460,11 +1545,14 @@ void JoinExpand(const uint64_t *offsets, const uint64_t *lower, uint64_t n_left,
 	VGPU_CUDA(cudaGetLastError());
 }
 
-void JoinRuns(const uint64_t *probe, uint64_t n_probe, const uint64_t *sorted, const uint32_t *dir, uint64_t nb,
-              uint32_t shift, uint64_t bias, uint64_t *lower, uint64_t *count, cudaStream_t stream) {
-	if (n_probe == 0) return;
-	LaunchScope scope("join_runs", stream, n_probe * 24, n_probe);
-	JoinRunKernel<<<GridFor(n_probe, 256), 256, 0, stream>>>(probe, n_probe, sorted, dir, nb, shift, bias, lower, count);
+void JoinRuns(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, uint64_t *lower, uint64_t *count,
+              cudaStream_t stream) {
+	if (n == 0) return;
+	LaunchScope scope("join_runs", stream, n * (kwidth + 16), n);
+	WithKeys(keys, kwidth, [&](auto *k) {
+		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
+		JoinRunKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, view, lower, count);
+	});
 	VGPU_CUDA(cudaGetLastError());
 }
 
@@ -1476,9 +1564,9 @@ void JoinDenseRuns(const void *keys, size_t kwidth, uint64_t n, uint64_t bias, u
 	VGPU_CUDA(cudaMemsetAsync(info, 0, 12, stream));
 	WithKeys(keys, kwidth, [&](auto *k) {
 		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
-		JoinEntryCountKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, bias, e);
-		JoinEntryPlaceKernel<<<GridFor((range + 1024) / 4, 256), 256, 0, stream>>>(e, range + 1, info + 2);
-		JoinEntryFillKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, bias, e, rows);
+		JoinEntryCountKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, bias, e, info);
+		JoinEntryPlaceKernel<<<GridFor((range + 1024) / 4, 256), 256, 0, stream>>>(e, range + 1, info);
+		JoinEntryFillKernel<K><<<GridFor(n, 256), 256, 0, stream>>>(k, n, bias, e, rows, info);
 	});
 	JoinEntrySortKernel<<<GridFor(range + 1, 256), 256, 0, stream>>>(e, range + 1, rows, list, info);
 	JoinEntrySortLongKernel<<<Runtime::Get().props().sm_count * 2, 256, 0, stream>>>(e, rows, list, info);
@@ -1509,15 +1597,18 @@ void JoinCountMatches(const void *keys, size_t kwidth, uint64_t n, const JoinRun
 }
 
 void JoinEmit(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, const uint64_t *chain,
-              const uint32_t *rows, const JoinOuts &outs, uint64_t total, cudaStream_t stream) {
+              const uint32_t *rows, const JoinOuts &outs, uint64_t total, uint32_t longest, cudaStream_t stream) {
+	// CTAs that share a tile's matches (and each find all of its runs): a few left rows with many matches each are
+	// otherwise left to as few CTAs (15600 left rows with 64 each: 0.28 -> 0.03 ms)
+	const uint32_t parts = std::max<uint32_t>(1, longest / 4096);
 	uint64_t row_bytes = 0;
 	for (int c = 0; c < outs.n; c++) row_bytes += outs.c[c].width;
 	LaunchScope scope("join_emit", stream, n * kwidth + 2 * total * row_bytes, total);
 	const uint64_t tiles = (n + kJoinTile - 1) / kJoinTile;
-	const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8));
+	const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles * parts, static_cast<uint64_t>(Runtime::Get().props().sm_count) * 8));
 	WithKeys(keys, kwidth, [&](auto *k) {
 		using K = std::remove_const_t<std::remove_pointer_t<decltype(k)>>;
-		JoinEmitKernel<K><<<grid, kJoinBlock, 0, stream>>>(k, n, view, tiles, chain + 2 + (tiles + 1) / 2, rows, outs);
+		JoinEmitKernel<K><<<grid, kJoinBlock, 0, stream>>>(k, n, view, tiles, chain + 2 + (tiles + 1) / 2, rows, outs, parts);
 	});
 	VGPU_CUDA(cudaGetLastError());
 }

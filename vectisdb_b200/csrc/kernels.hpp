@@ -67,7 +67,10 @@ BoundsKind SignedBoundsKind(ValueType t);
 //! With `distinct`, kDistinctRanks 32-bit ranks per column follow in `out` (BoundsWords in all), from which
 //! DistinctEstimate (on the words read back) gives about how many distinct values a 4- or 8-byte column has
 //! (within some 7%; 0 for narrower ones).
-void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream, bool distinct = false);
+//! With `pairs` (2n words) instead, also how many pairs of values far apart it looked at, [2c + 1], and how many of those were
+//! equal, [2c]: their share is the chance that two rows have the same value.
+void ColumnBounds(const BoundsColumn *cols, int n, uint64_t *out, cudaStream_t stream, bool distinct = false,
+                  uint64_t *pairs = nullptr);
 constexpr int kDistinctRanks = 256;
 inline size_t BoundsWords(int n, bool distinct) {
 	return static_cast<size_t>(n) * (2 + (distinct ? kDistinctRanks / 2 : 0));
@@ -96,10 +99,6 @@ void Iota(uint32_t *out, uint64_t n, cudaStream_t stream);
 //! the left rows a tile spans staged in shared memory.
 void JoinExpand(const uint64_t *offsets, const uint64_t *lower, uint64_t n_left, const uint32_t *sorted_perm,
                 uint64_t total, uint32_t *out_left, uint32_t *out_right, cudaStream_t stream);
-//! For each probe key (widened): the first position of its run of equal keys in `sorted` (normalized by
-//! `bias`) and the run's length, through the radix directory `dir` (nb buckets of key >> shift).
-void JoinRuns(const uint64_t *probe, uint64_t n_probe, const uint64_t *sorted, const uint32_t *dir, uint64_t nb,
-              uint32_t shift, uint64_t bias, uint64_t *lower, uint64_t *count, cudaStream_t stream);
 
 //! Where a left key's right rows are: dense keys by an entry per key value (JoinDenseRuns), else a sorted key
 //! array with its radix directory (`entries` null).
@@ -110,12 +109,17 @@ struct JoinRunsView {
 	uint64_t nb = 0;  // entries, or directory buckets
 	uint64_t bias = 0;
 	uint32_t shift = 0;
+	const uint32_t *info = nullptr;  // of JoinDenseRuns, with entries: the count does nothing when a run is too long
 };
+//! For each left row (raw keys): the first place of its run in the right rows' order, and the run's length.
+void JoinRuns(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, uint64_t *lower, uint64_t *count,
+              cudaStream_t stream);
 //! Longest run JoinDenseRuns puts in row order.
 constexpr uint32_t kJoinRunLimit = 4096;
 //! The rows of each key value contiguous in `rows` [n], in row order, and an entry per value of the range (range
 //! + 1 words of `entries`), without sorting the keys. `list` [n / 17 + 1] and `info` [3] are scratch; info[1]
-//! becomes the longest run's length: past kJoinRunLimit that run is not in order, and the caller sorts instead.
+//! becomes the longest run's length, or one past kJoinRunLimit as soon as a run is: the rest is then left out, and the
+//! caller sorts instead.
 void JoinDenseRuns(const void *keys, size_t kwidth, uint64_t n, uint64_t bias, uint64_t range, uint64_t *entries,
                    uint32_t *rows, uint32_t *list, uint32_t *info, cudaStream_t stream);
 //! Longest wait in ns of a kernel for tiles counted in the same launch (VGPU_WAIT_LIMIT_NS, for testing: up to 10 s;
@@ -138,9 +142,9 @@ struct JoinOuts {
 	int n = 0;
 };
 //! Every output column of the matches, left rows in order and each one's matches in the order of `rows`; without
-//! `rows` the right columns are in that order themselves.
+//! `rows` the right columns are in that order themselves. `longest`: the most matches of one tile.
 void JoinEmit(const void *keys, size_t kwidth, uint64_t n, const JoinRunsView &view, const uint64_t *chain,
-              const uint32_t *rows, const JoinOuts &outs, uint64_t total, cudaStream_t stream);
+              const uint32_t *rows, const JoinOuts &outs, uint64_t total, uint32_t longest, cudaStream_t stream);
 
 //! Radix directory of a sorted (biased) key array: dir[b] = first position whose key >> shift >= b,
 //! for b in [0, nb]; dir needs nb + 1 entries and nb must exceed every key >> shift.
