@@ -2370,7 +2370,12 @@ std::string PipelineCodegen::EmitGroupBy(const GroupBySpec &gb, bool partitioned
 // instead took 0.61 ms for Zipf(1.1), and with a fence to read them back in the same launch 0.74 ms.
 //
 // `hashed`, for keys too sparse to be places: the same over a table of D key words with double hashing (one more
-// read of a random word per row, 280 G/s). More keys than fit raise a flag beside the ticket that ends the pass.
+// read of a random word per row, 280 G/s). More keys than fit raise a flag beside the ticket that ends the pass. Where
+// they may be more, a sample of 2^16 rows says first whether they are: of its keys f1 are met once and f2 twice, so
+// there are about f0 = f1 * f1 / 2 f2 more of them than it met (Chao's estimate, which frequent keys do not disturb), and
+// the rows t times as many as it would meet f0 (1 - exp(-(t - 1) f1 / f0)) of those; counters shared by different keys are
+// taken off. 1.5M rows of as many pairs, more than fit: 0.45 -> 0.32 ms whole query
+// (partitioned at once 0.30); 8M of 8M 1.02 -> 0.84 (0.82); 8M rows of 3600 pairs 0.30 (0.71).
 // Arguments: cb = D, field arrays, outputs, the compaction's chain (see EmitMaterializeOnePass; the flag in the
 // ticket's word), the hot keys' tags ([kL2HotSlots] u32, u64 when hashed: key + 1, or 0), hashed: the keys.
 std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry &g, bool hashed) const {
@@ -2426,8 +2431,38 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 		  << "\t\tif (cur == ~0ull) {\n\t\t\tconst u64 prev = atomicCAS((unsigned long long*)(K + s), ~0ull, key);\n"
 		  << "\t\t\tif (prev == ~0ull || prev == key) return (i64)s;\n\t\t}\n\t\ts = (s + step) & (D - 1);\n\t}\n\treturn -1;\n}\n\n";
 	}
+	if (hashed) {
+		const std::string counters = "(u32*)a.w[" + std::to_string(chain_word + 3) + "]", B = std::to_string(kL2GuessCounters);
+		Geometry one = g;
+		one.items = 1;
+		o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_gb_l2_guess(KArgs a) {\n" << kKernelHead
+		  << "\tu32 *counters = " << counters << ";\n\t__shared__ int once, twice;\n"
+		  << "\tif (threadIdx.x == 0) once = twice = 0;\n\t__syncthreads();\n"
+		  << "\tconst u64 sample = blockIdx.x * (u64)blockDim.x + threadIdx.x, apart = n / " << kL2GuessRows << "ull;\n"
+		  << LoadBlock(one, needed, true, "sample * apart + mix64(sample) % apart") << "\t\tint f1 = 0, f2 = 0;\n" << ItemOpen(one, needed)
+		  << chain_code_ << "\t\tif (keep) {\n\t\t\tconst u64 slot = " << pack.str() << ";\n"
+		  << "\t\t\tconst u32 before = atomicAdd(counters + (mix64(slot) >> " << 64 - BitLength(static_cast<uint32_t>(kL2GuessCounters - 1))
+		  << "), 1u);\n"
+		  << "\t\t\tf1 = before == 0u ? 1 : before == 1u ? -1 : 0;\n\t\t\tf2 = before == 1u ? 1 : before == 2u ? -1 : 0;\n\t\t}\n"
+		  << ItemClose() << "\tif (f1) atomicAdd(&once, f1);\n\tif (f2) atomicAdd(&twice, f2);\n\t__syncthreads();\n"
+		  << "\tif (threadIdx.x == 0) {\n\t\tatomicAdd((int*)counters + " << B << ", once);\n\t\tatomicAdd((int*)counters + " << B
+		  << " + 1, twice);\n\t}\n}\n\n"
+		  // too few sampled rows pass a filter: no guess
+		  << "__device__ __forceinline__ bool vgpu_l2_refused(const KArgs &a, u64 n, u64 D) {\n\tconst int *c = (const int*)" << counters
+		  << ";\n\tif (c == nullptr || c[" << B << "] < 16384) return false;\n"
+		  << "\tconst double f1 = (double)c[" << B << "], f2 = (double)c[" << B << " + 1], pairs = f1 * f1 * 0.5;\n"
+		  << "\tconst double unseen = pairs / fmax(f2 - pairs / " << B << ".0, 1.0), rest = f1 * ((double)n / " << kL2GuessRows
+		  << ".0 - 1.0);\n"
+		  << "\treturn f1 + f2 + unseen * -expm1(-rest / unseen) > 0.62 * (double)D;\n}\n\n";
+	}
 	o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_gb_l2_init(KArgs a) {\n" << kKernelHead
-	  << "\tconst u64 D = a.w[" << cb << "];\n\tif (blockIdx.x != 0) {\n" << chain_decl
+	  << "\tconst u64 D = a.w[" << cb << "];\n";
+	if (hashed) {
+		o << "\tif (vgpu_l2_refused(a, n, D)) {  // a flag for the kernels behind, instead of a table\n"
+		  << "\t\tif (blockIdx.x == 0 && threadIdx.x == 0) { ((u64*)a.w[" << chain_word << "])[0] = 0ull; ((u64*)a.w[" << chain_word
+		  << "])[1] = 1ull << 32; }\n\t\treturn;\n\t}\n";
+	}
+	o << "\tif (blockIdx.x != 0) {\n" << chain_decl
 	  << "\tconst u64 t0 = (blockIdx.x - 1) * (u64)blockDim.x + threadIdx.x, step = (gridDim.x - 1) * (u64)blockDim.x;\n"
 	  << "\tfor (u64 i = t0; i < 2 + (ntiles + 1) / 2 + ntiles; i += step) chain[i] = 0ull;\n"
 	  << "\tfor (u64 s = t0; s < D / 2; s += step) {\n";
@@ -2469,7 +2504,7 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	}
 	if (hashed) {
 		o << "\tu64 *K = " << table << ";\n\tconst u64 D = a.w[" << cb << "];\n\tvolatile u32 *vgpu_full = (volatile u32*)(" << "(u64*)a.w["
-		  << chain_word << "] + 1) + 1;\n";
+		  << chain_word << "] + 1) + 1;\n\tif (__syncthreads_or(*vgpu_full != 0u)) return;\n";
 	}
 	o << "\t__shared__ " << kt << " tag[" << H << "];\n\tconst u32 lane = threadIdx.x & 31; (void)lane;\n"
 	  << "\tfor (u32 i = threadIdx.x; i < " << H << "u; i += " << g.block << ") {\n"
@@ -2551,6 +2586,7 @@ std::string PipelineCodegen::EmitGroupByL2(const GroupBySpec &gb, const Geometry
 	  << "\tconst u64 D = a.w[" << cb << "];\n" << chain_decl
 	  << "\tu32 *counts = (u32*)(chain + 2);\n\tu64 *starts = chain + 2 + (ntiles + 1) / 2;\n";
 	for (int f = 0; f < F; f++) o << "\tconst u64 *G" << f << " = (const u64*)a.w[" << cb + 1 + f << "];\n";
+	if (hashed) o << "\tif ((chain[1] >> 32) != 0ull) return;  // keys without a place: the caller takes another way\n";
 	o << "\t__shared__ u32 scan_scratch[33], vgpu_warps[32];\n\t__shared__ u32 vgpu_next;\n\t__shared__ u64 vgpu_base;\n"
 	  << "\tconst u32 lane = threadIdx.x & 31;\n"
 	  << "\tif (threadIdx.x == 0) vgpu_next = atomicAdd((u32*)(chain + 1), 1u);\n"

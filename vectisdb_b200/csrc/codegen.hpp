@@ -189,9 +189,12 @@ public:
 	//! vgpu_gb_l2_init, vgpu_gb_l2 (kL2HotSlots * StateWords words of dynamic shared memory), vgpu_gb_l2_final.
 	static constexpr uint64_t kL2TableBytes = 64ull << 20;
 	static constexpr int kL2HotSlots = 512, kL2SampleRows = 2048, kL2FinalTile = 1024;
+	//! A hashed table whose keys are not known to fit: rows that vgpu_gb_l2_guess samples, and the counters it needs
+	//! (u32, zero at launch, two sums behind them).
+	static constexpr uint64_t kL2GuessRows = 1 << 16, kL2GuessCounters = 1 << 20;
 	std::string EmitGroupByL2(const GroupBySpec &gb, const Geometry &g, bool hashed = false) const;
 	//! Argument word of its compaction chain (total, ticket, tile counts and starts); the next two take
-	//! the hot keys' tags (kL2HotSlots words at most) and a hashed table's keys.
+	//! the hot keys' tags (kL2HotSlots words at most), a hashed table's keys and its counters for the guess (or null).
 	int L2ChainWord(const GroupBySpec &gb) const {
 		return ConsumerBase() + 1 + StateWords(gb) + static_cast<int>(gb.keys.size() + gb.aggs.size());
 	}

@@ -244,8 +244,8 @@ private:
 	Relation JoinForPipeline(const PlanNode &node, PipelineInput &pin, bool *fused, bool multi_ok, bool any_order);
 	Relation GroupByPipeline(const PlanNode &node, PipelineInput &pin);
 	bool GroupByL2(const PlanNode &node, PipelineInput &pin, const PipelineCodegen &cg,
-	               const PipelineCodegen::GroupBySpec &gb, uint64_t slots, bool hashed, uint64_t cap_rows, Relation &out,
-	               uint64_t *groups);
+	               const PipelineCodegen::GroupBySpec &gb, uint64_t slots, bool hashed, bool guess, uint64_t cap_rows,
+	               Relation &out, uint64_t *groups);
 	Relation CrossProduct(const PlanNode &node);
 	//! Ranges of visible columns, and about how many distinct values the source behind each has (0 = not known).
 	void ComputeStats(PipelineInput &pin, const PipelineCodegen &cg, const std::vector<int> &cols,
@@ -1026,14 +1026,17 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	// the plan's estimate, says that the groups fill over 58% of it (a table is sure to take three fifths; the
 	// distinct counts are good to some 7%, and do not see filters). Groups that do not fit after all end the pass
 	// early, and the rows are partitioned. 8M rows of 600K ids, SUM and COUNT: 0.62 -> 0.28 ms, of 100 ids 2.17 ->
-	// 0.26; 70K rows of 1000 ids 0.139 -> 0.104; 3M or 30M different ids as before.
+	// 0.26; 70K rows of 1000 ids 0.139 -> 0.104; 3M or 30M different ids as before. What several keys come to together is
+	// not known: see vgpu_gb_l2_guess.
 	const uint64_t l2_slot = 8 * (1 + static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2)));
 	uint64_t l2_slots = std::min<uint64_t>(FloorPow2(PipelineCodegen::kL2TableBytes / l2_slot),
 	                                       std::max<uint64_t>(2048, NextPow2(2 * std::min<uint64_t>(n, 1ull << 32))));
 	// one key whose distinct values are known to be few: no larger a table to fill and to walk than they need
 	// with a margin for the estimate (8M rows of 100 ids 0.257 -> 0.241 ms)
 	if (distinct.size() == 1 && distinct[0]) l2_slots = std::min(l2_slots, NextPow2(5 * distinct[0] / 2 + (1u << 16)));
-	bool l2_hashed = !direct && !l2 && !dpart && !pin.spec.join_multi && cg.L2ChainWord(gb_l2) + 2 < kKeyWord &&
+	// known to fit by one key's count, or since the rows are no more
+	const bool l2_fits = (distinct.size() == 1 && distinct[0]) || 100 * n <= 58 * l2_slots;
+	bool l2_hashed = !direct && !l2 && !dpart && !pin.spec.join_multi && cg.L2ChainWord(gb_l2) + 3 < kKeyWord &&
 	                 100 * std::max<uint64_t>(node.estimated_rows, *std::max_element(distinct.begin(), distinct.end())) <=
 	                     58 * l2_slots;
 	if (const char *env = std::getenv("VGPU_GB_STRATEGY")) l2_hashed = l2_hashed && std::strcmp(env, "l2") == 0;
@@ -1198,8 +1201,8 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 			groups = ReadU64(count);
 		}
 	} else if (l2) {
-		GroupByL2(node, pin, cg, gb_l2, domain, false, cap_rows, out, &groups);
-	} else if (l2_hashed && GroupByL2(node, pin, cg, gb_l2, l2_slots, true, cap_rows, out, &groups)) {
+		GroupByL2(node, pin, cg, gb_l2, domain, false, false, cap_rows, out, &groups);
+	} else if (l2_hashed && GroupByL2(node, pin, cg, gb_l2, l2_slots, true, !l2_fits, cap_rows, out, &groups)) {
 		// grouped
 	} else {
 		// Partitioned. Tier-1 bucket tables are small (about 48 KB, 128 threads per CTA, several CTAs per
@@ -1507,8 +1510,8 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 // One pass into a table held in L2 (see EmitGroupByL2): `slots` places, the packed keys themselves or hashed.
 // False when a hashed table had no place for a key (nothing of the result is written then).
 bool Executor::GroupByL2(const PlanNode &node, PipelineInput &pin, const PipelineCodegen &cg,
-                         const PipelineCodegen::GroupBySpec &gb, uint64_t slots, bool hashed, uint64_t cap_rows, Relation &out,
-                         uint64_t *groups) {
+                         const PipelineCodegen::GroupBySpec &gb, uint64_t slots, bool hashed, bool guess, uint64_t cap_rows,
+                         Relation &out, uint64_t *groups) {
 	const auto &props = Runtime::Get().props();
 	const int F = PipelineCodegen::StateWords(gb);
 	const int cb = cg.ConsumerBase();
@@ -1533,6 +1536,14 @@ bool Executor::GroupByL2(const PlanNode &node, PipelineInput &pin, const Pipelin
 	a.SetWord(kWaitWord, kern::WaitLimitNs());
 	a.SetPtr(cg.L2ChainWord(gb) + 1, arena_.AllocT<uint64_t>(PipelineCodegen::kL2HotSlots));
 	if (hashed) a.SetPtr(cg.L2ChainWord(gb) + 2, fields + slots * F);
+	if (guess) {
+		const uint64_t bytes = (PipelineCodegen::kL2GuessCounters + 2) * 4;
+		void *counters = arena_.Alloc(bytes);
+		VGPU_CUDA(cudaMemsetAsync(counters, 0, bytes, stream_));
+		a.SetPtr(cg.L2ChainWord(gb) + 3, counters);
+		LaunchGenerated(*module, "vgpu_gb_l2_guess", PipelineCodegen::kL2GuessRows / g.block, g.block, 0, stream_, a, 0,
+		                PipelineCodegen::kL2GuessRows);
+	}
 	const uint64_t sms = static_cast<uint64_t>(props.sm_count);
 	const size_t smem = static_cast<size_t>(F) * PipelineCodegen::kL2HotSlots * 8;
 	const int occ = std::max(1, Runtime::Get().MaxActiveBlocks(module->Get("vgpu_gb_l2"), g.block, smem));
