@@ -248,8 +248,10 @@ private:
 	               Relation &out, uint64_t *groups);
 	Relation CrossProduct(const PlanNode &node);
 	//! Ranges of visible columns, and about how many distinct values the source behind each has (0 = not known).
+	//! With `joined`, ranges of right columns of a join that are those of all its right rows are left out instead, and
+	//! measured over the rows that the join keeps.
 	void ComputeStats(PipelineInput &pin, const PipelineCodegen &cg, const std::vector<int> &cols,
-	                  std::vector<std::pair<int64_t, int64_t>> &out, std::vector<uint64_t> &distinct);
+	                  std::vector<std::pair<int64_t, int64_t>> &out, std::vector<uint64_t> &distinct, bool joined = false);
 	void FillArgs(const PipelineInput &pin, KArgsHost &args);
 	uint64_t DirectBuckets(Module &module, const PipelineCodegen::GroupBySpec &gb, const PipelineInput &pin, uint64_t P,
 	                       uint64_t G, const uint32_t *offsets, const uint32_t *total, const char *records, uint64_t n,
@@ -600,7 +602,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 			if (vc.nullable) {
 				col.valid = arena_.AllocT<uint8_t>(rows);
 			}
-			if (vc.source >= 0 && pin.sources[vc.source].has_stats) {
+			if (vc.source >= 0 && pin.sources[vc.source].has_stats && !pin.sources[vc.source].unjoined_stats) {
 				col.has_stats = true;
 				col.min = pin.sources[vc.source].min;
 				col.max = pin.sources[vc.source].max;
@@ -730,7 +732,7 @@ Relation Executor::CrossProduct(const PlanNode &node) {
 }
 
 void Executor::ComputeStats(PipelineInput &pin, const PipelineCodegen &cg, const std::vector<int> &cols,
-                            std::vector<std::pair<int64_t, int64_t>> &out, std::vector<uint64_t> &distinct) {
+                            std::vector<std::pair<int64_t, int64_t>> &out, std::vector<uint64_t> &distinct, bool joined) {
 	out.assign(cols.size(), {0, 0});
 	distinct.assign(cols.size(), 0);
 	std::vector<int> missing;
@@ -743,10 +745,11 @@ void Executor::ComputeStats(PipelineInput &pin, const PipelineCodegen &cg, const
 	std::vector<size_t> own_pos;
 	for (size_t i = 0; i < cols.size(); i++) {
 		const auto &vc = cg.visible()[cols[i]];
-		if (vc.source >= 0 && pin.sources[vc.source].has_stats) {
+		const bool right = joined && vc.source >= 0 && pin.spec.sources[vc.source].side == 1;
+		if (vc.source >= 0 && pin.sources[vc.source].has_stats && !(right && pin.sources[vc.source].unjoined_stats)) {
 			out[i] = {pin.sources[vc.source].min, pin.sources[vc.source].max};
 			distinct[i] = pin.sources[vc.source].distinct;
-		} else if (vc.source >= 0 && IsIntegerKeyType(vc.type)) {
+		} else if (vc.source >= 0 && IsIntegerKeyType(vc.type) && !right) {
 			const DevColumn &src = pin.sources[vc.source];
 			own.push_back({src.data, src.rows, kern::SignedBoundsKind(src.type)});
 			own_pos.push_back(i);
@@ -943,15 +946,24 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	std::vector<uint64_t> distinct;
 	ComputeStats(pin, cg, key_cols, ranges, distinct);
 	int shift = 0;
-	for (size_t i = 0; i < key_cols.size(); i++) {
-		PipelineCodegen::GroupKey k;
-		k.column = key_cols[i];
-		k.min = ranges[i].first;
-		const uint64_t span = static_cast<uint64_t>(ranges[i].second) - static_cast<uint64_t>(ranges[i].first);
-		k.bits = BitsFor(span);
-		k.shift = shift;
-		shift += k.bits;
-		gb.keys.push_back(k);
+	auto pack = [&] {
+		gb.keys.clear();
+		shift = 0;
+		for (size_t i = 0; i < key_cols.size(); i++) {
+			PipelineCodegen::GroupKey k;
+			k.column = key_cols[i];
+			k.min = ranges[i].first;
+			const uint64_t span = static_cast<uint64_t>(ranges[i].second) - static_cast<uint64_t>(ranges[i].first);
+			k.bits = BitsFor(span);
+			k.shift = shift;
+			shift += k.bits;
+			gb.keys.push_back(k);
+		}
+	};
+	pack();
+	if (shift > 63 && pin.spec.join) {  // right rows without a match may hold any value
+		ComputeStats(pin, cg, key_cols, ranges, distinct, true);
+		pack();
 	}
 	if (shift > 63) {
 		Fail(VGPU_ERR_UNSUPPORTED, "gpu_groupby: the group key ranges need " + std::to_string(shift) +
@@ -1811,7 +1823,7 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 				const uint32_t sign = c.type == ValueType::BOOLEAN ? 0u : 1u << (8 * w - 1);
 				if ((vmin & sign) == (vmax & sign)) {
 					const uint64_t high = (vmin & sign) ? ~0ull << (8 * w) : 0ull;
-					c.has_stats = true;
+					c.has_stats = c.unjoined_stats = true;
 					c.min = c.type == ValueType::BOOLEAN ? 0 : static_cast<int64_t>(vmin | high);
 					c.max = c.type == ValueType::BOOLEAN ? 1 : static_cast<int64_t>(vmax | high);
 				}

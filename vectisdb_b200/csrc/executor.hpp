@@ -22,6 +22,7 @@ struct DevColumn {
 	uint8_t *valid = nullptr;
 	bool has_stats = false;
 	int64_t min = 0, max = 0;
+	bool unjoined_stats = false;  // min and max are those of a join's right rows, matched or not
 	uint64_t distinct = 0;  // about how many distinct values there are, 0 = not known
 	void *block = nullptr;  // the allocation `data` lies in, when columns share one
 	std::shared_ptr<uint8_t> host;  // `data` is this page-locked memory, complete: a root result on the host
