@@ -234,15 +234,16 @@ private:
 	                            bool any_order = false);
 	//! A pipeline with no chain over the columns of a relation.
 	PipelineInput PipelineOver(const Relation &rel);
-	//! `at_root`: the outputs are the plan's result (their row count may stay on the device).
+	//! `at_root`: the outputs are the plan's result (their row count may stay on the device). `waits`: kernels may wait
+	//! for tiles of their own launch (not again when such a wait ran out).
 	Relation Materialize(PipelineInput &pin, const std::vector<int> &out_cols, const std::vector<std::string> &names,
-	                     bool at_root = false);
+	                     bool at_root = false, bool waits = true);
 	Relation RunChain(const PlanNode &node);
 	Relation GroupBy(const PlanNode &node);
 	Relation Join(const PlanNode &node);
 	Relation JoinMaterialize(const PlanNode &node, Relation &left, Relation &right);
 	Relation JoinForPipeline(const PlanNode &node, PipelineInput &pin, bool *fused, bool multi_ok, bool any_order);
-	Relation GroupByPipeline(const PlanNode &node, PipelineInput &pin);
+	Relation GroupByPipeline(const PlanNode &node, PipelineInput &pin, bool waits = true);
 	bool GroupByL2(const PlanNode &node, PipelineInput &pin, const PipelineCodegen &cg,
 	               const PipelineCodegen::GroupBySpec &gb, uint64_t slots, bool hashed, bool guess, uint64_t cap_rows,
 	               Relation &out, uint64_t *groups);
@@ -544,7 +545,7 @@ Executor::PipelineInput Executor::PipelineOver(const Relation &rel) {
 }
 
 Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_cols,
-                               const std::vector<std::string> &names, bool at_root) {
+                               const std::vector<std::string> &names, bool at_root, bool waits) {
 	auto cgp = CodegenFor(pin.spec, pin.Key());
 	const PipelineCodegen &cg = *cgp;
 	const uint64_t n = pin.rows;
@@ -557,7 +558,7 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 	// two rows in five survive (what the admission estimate charges for the outputs then stays near what
 	// they take). Its two staged tiles of 512 rows allow 96 bytes a row (96 KB a CTA, two CTAs per SM).
 	// VGPU_MAT_PASSES=2: always two (testing).
-	bool one_pass = cg.has_filter() && n > 0 && !pin.spec.join_multi && row_bytes > 0 && row_bytes <= 96 &&
+	bool one_pass = waits && cg.has_filter() && n > 0 && !pin.spec.join_multi && row_bytes > 0 && row_bytes <= 96 &&
 	                n <= (8ull << 30) / row_bytes && Room((at_root ? 1 : 4) * n * row_bytes);
 	for (const PlanNode *node : pin.spec.chain) {
 		if (node->op == OpType::FILTER && node->estimated_rows && 5 * node->estimated_rows < 2 * n) one_pass = false;
@@ -630,7 +631,11 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 		// at the root, outputs without NULL masks may leave the count on the device
 		if (at_root && !null_outs && DeferRows(chain, 8, 0)) return out;
 		out_rows = ReadU64(chain);
-		if (out_rows > n) Fail(VGPU_ERR_CUDA, "gpu_executor: a row filter's tiles were not completed in time");
+		if (out_rows > n) {  // a wait ran out (a device shared with others can keep a CTA back for seconds): two passes
+			for (auto &col : out) arena_.FreeNow(col.valid);
+			arena_.FreeNow(block);
+			return Materialize(pin, out_cols, names, at_root, false);
+		}
 		for (auto &col : out) col.rows = out_rows;
 		// rows that stay on the device do not hold on to the room of many more
 		const uint64_t spare = (n - out_rows) * row_bytes;
@@ -906,7 +911,7 @@ Relation Executor::GroupBy(const PlanNode &node) {
 	return GroupByPipeline(node, pin);
 }
 
-Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
+Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin, bool waits) {
 	auto cgp = CodegenFor(pin.spec, pin.Key());
 	const PipelineCodegen &cg = *cgp;
 	if (cg.visible().empty()) {
@@ -1005,7 +1010,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	// 0.83; 34M skewed rows by 3.2M keys, four aggregates, 0.83 and 0.75 ms, but 2.6M of them by 2.1M keys 0.158 and
 	// 0.184, and 1.34e8 by 3.2M 2.40 and 2.53.
 	const uint64_t l2_most = PipelineCodegen::kL2TableBytes * (domain <= n && n / 8 <= domain ? 2 : 1);
-	bool l2 = !direct && shift >= 10 && shift <= 26 &&
+	bool l2 = waits && !direct && shift >= 10 && shift <= 26 &&
 	          domain * static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2)) * 8 <= l2_most &&
 	          cg.L2ChainWord(gb_l2) + 1 < kKeyWord;
 	if (const char *env = std::getenv("VGPU_GB_STRATEGY")) l2 = l2 && std::strcmp(env, "l2") == 0;
@@ -1048,7 +1053,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	if (distinct.size() == 1 && distinct[0]) l2_slots = std::min(l2_slots, NextPow2(5 * distinct[0] / 2 + (1u << 16)));
 	// known to fit by one key's count, or since the rows are no more
 	const bool l2_fits = (distinct.size() == 1 && distinct[0]) || 100 * n <= 58 * l2_slots;
-	bool l2_hashed = !direct && !l2 && !dpart && !pin.spec.join_multi && cg.L2ChainWord(gb_l2) + 3 < kKeyWord &&
+	bool l2_hashed = waits && !direct && !l2 && !dpart && !pin.spec.join_multi && cg.L2ChainWord(gb_l2) + 3 < kKeyWord &&
 	                 100 * std::max<uint64_t>(node.estimated_rows, *std::max_element(distinct.begin(), distinct.end())) <=
 	                     58 * l2_slots;
 	if (const char *env = std::getenv("VGPU_GB_STRATEGY")) l2_hashed = l2_hashed && std::strcmp(env, "l2") == 0;
@@ -1213,7 +1218,10 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 			groups = ReadU64(count);
 		}
 	} else if (l2) {
-		GroupByL2(node, pin, cg, gb_l2, domain, false, false, cap_rows, out, &groups);
+		if (!GroupByL2(node, pin, cg, gb_l2, domain, false, false, cap_rows, out, &groups)) {
+			for (auto &c : out) arena_.FreeNow(c.data);
+			return GroupByPipeline(node, pin, false);
+		}
 	} else if (l2_hashed && GroupByL2(node, pin, cg, gb_l2, l2_slots, true, !l2_fits, cap_rows, out, &groups)) {
 		// grouped
 	} else {
@@ -1519,8 +1527,9 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin) {
 	return out;
 }
 
-// One pass into a table held in L2 (see EmitGroupByL2): `slots` places, the packed keys themselves or hashed.
-// False when a hashed table had no place for a key (nothing of the result is written then).
+// One pass into a table held in L2 (see EmitGroupByL2): `slots` places, the packed keys themselves or hashed, then (with
+// `guess`) only if a sample says that the keys fit. False when a hashed table had no place for a key, or a wait of the
+// compaction ran out: the output columns may then hold leftovers, which another form overwrites.
 bool Executor::GroupByL2(const PlanNode &node, PipelineInput &pin, const PipelineCodegen &cg,
                          const PipelineCodegen::GroupBySpec &gb, uint64_t slots, bool hashed, bool guess, uint64_t cap_rows,
                          Relation &out, uint64_t *groups) {
@@ -1572,11 +1581,10 @@ bool Executor::GroupByL2(const PlanNode &node, PipelineInput &pin, const Pipelin
 		return true;
 	}
 	const std::vector<uint64_t> head = ReadWords(chain, 2);
-	if (hashed && (head[1] >> 32) != 0) {
+	if ((hashed && (head[1] >> 32) != 0) || head[0] > cap_rows) {
 		arena_.FreeNow(fields);
 		return false;
 	}
-	if (head[0] > cap_rows) Fail(VGPU_ERR_CUDA, "gpu_groupby: the groups were not compacted in time");
 	*groups = head[0];
 	return true;
 }
