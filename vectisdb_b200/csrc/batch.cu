@@ -303,7 +303,7 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 	PipelineCodegen::BatchLayout L;
 	L.key_base = 1 + 2 * nsrc;
 	L.dom_base = L.key_base + 2 * nkeys;
-	L.param_base = L.dom_base + 4;
+	L.param_base = L.dom_base + 3;
 	L.qwords = L.param_base + nparams;
 	const int F = PipelineCodegen::StateWords(gb);
 	const auto &props = Runtime::Get().props();
@@ -425,8 +425,7 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 			}
 			row[L.dom_base] = dom[qi];
 			row[L.dom_base + 1] = acc_words;
-			row[L.dom_base + 2] = out_rows;
-			row[L.dom_base + 3] = dom[qi] <= static_cast<uint64_t>(g.smem_slots) ? 1 : 0;
+			row[L.dom_base + 2] = dom[qi] <= static_cast<uint64_t>(g.smem_slots) ? 1 : 0;
 			for (int p = 0; p < nparams; p++) row[L.param_base + p] = qs[qi]->params[p];
 			out_base[qi] = out_rows;
 			out_cap[qi] = std::max<uint64_t>(1, std::min<uint64_t>(dom[qi], qs[qi]->rows));
@@ -486,19 +485,19 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 		e->qtab = static_cast<uint64_t *>(al.Alloc(qt.size() * 8, stream));
 		e->tiles = al.Alloc(std::max<size_t>(8, tl.size() * 4), stream);
 		e->acc = static_cast<uint64_t *>(al.Alloc(e->acc_words * F * 8, stream));
-		e->outp = static_cast<uint64_t *>(al.Alloc(out_words * 8, stream));
+		e->outp = static_cast<uint64_t *>(al.Alloc(qs.size() * out_words * 8, stream));
 		e->work = static_cast<uint32_t *>(al.Alloc(16 + nseg * 4, stream));
 		e->segs = static_cast<uint32_t *>(e->tiles) + tile_words;
 		if (transient) {
 			e->pinned = false;
-			e->host_stage.assign(qs.size() + out_words, 0);
+			e->host_stage.assign(qs.size() * (1 + out_words), 0);
 			e->counts = static_cast<uint64_t *>(al.Alloc(qs.size() * 8, stream));
 			e->counts_host = e->host_stage.data();
 			e->outp_host = e->host_stage.data() + qs.size();
 		} else {
 			VGPU_CUDA(cudaMallocHost(&e->counts_host, qs.size() * 8));
 			e->counts = e->counts_host;  // written there by the finalize kernel
-			VGPU_CUDA(cudaMallocHost(&e->outp_host, out_words * 8));
+			VGPU_CUDA(cudaMallocHost(&e->outp_host, qs.size() * out_words * 8));
 		}
 		VGPU_CUDA(cudaMemcpyAsync(e->qtab, qt.data(), qt.size() * 8, cudaMemcpyHostToDevice, stream));
 		if (!tl.empty()) VGPU_CUDA(cudaMemcpyAsync(e->tiles, tl.data(), tl.size() * 4, cudaMemcpyHostToDevice, stream));
@@ -558,6 +557,24 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 	std::shared_ptr<BatchEntry> best;
 	double best_ms = 1e30;
 	const size_t out_words = gb.keys.size() + gb.aggs.size();
+	std::vector<ValueType> out_types;
+	std::vector<std::string> out_names;
+	for (int j = 0; j < nkeys; j++) {
+		out_types.push_back(cg->visible()[key_cols[j]].type);
+		out_names.push_back(root.group_keys[j]);
+	}
+	for (size_t i = 0; i < root.aggregates.size(); i++) {
+		out_types.push_back(root.aggregates[i].output_type);
+		out_names.push_back("agg_" + std::to_string(i));
+	}
+	// each query's rows of the outputs, one buffer per column
+	auto device_outputs = [&](BatchEntry &e, const std::vector<void *> &columns) {
+		for (size_t qi = 0; qi < qs.size(); qi++) {
+			for (size_t w = 0; w < out_words; w++) {
+				e.outp_host[qi * out_words + w] = reinterpret_cast<uint64_t>(columns[w]) + e.out_base[qi] * TypeSize(out_types[w]);
+			}
+		}
+	};
 	if (candidates.size() > 1) {
 		DeviceBuffers scratch_out;
 		scratch_out.stream = stream;
@@ -573,8 +590,8 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 				max_out = e->out_rows;
 				for (size_t w = 0; w < out_words; w++) scratch_out.ptrs.push_back(Runtime::Get().allocator().Alloc(max_out * 16, stream));
 			}
-			for (size_t w = 0; w < out_words; w++) e->outp_host[w] = reinterpret_cast<uint64_t>(scratch_out.ptrs[w]);
-			VGPU_CUDA(cudaMemcpyAsync(e->outp, e->outp_host, out_words * 8, cudaMemcpyHostToDevice, stream));
+			device_outputs(*e, scratch_out.ptrs);
+			VGPU_CUDA(cudaMemcpyAsync(e->outp, e->outp_host, qs.size() * out_words * 8, cudaMemcpyHostToDevice, stream));
 			init_if_needed(*e);
 			enqueue(*e, false);
 			float ms_best = 1e30f;
@@ -604,39 +621,41 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 	// Outputs of this call, shared by its queries' results.
 	auto holder = std::make_shared<DeviceBuffers>();
 	holder->stream = stream;
-	std::vector<ValueType> out_types;
-	std::vector<std::string> out_names;
-	for (int j = 0; j < nkeys; j++) {
-		out_types.push_back(cg->visible()[key_cols[j]].type);
-		out_names.push_back(root.group_keys[j]);
-	}
-	for (size_t i = 0; i < root.aggregates.size(); i++) {
-		out_types.push_back(root.aggregates[i].output_type);
-		out_names.push_back("agg_" + std::to_string(i));
-	}
-	// Host results of moderate size go straight to page-locked memory, which each query's columns then share:
-	// only the groups there are cross the link, as the finalize kernel finds them. (Copies of the whole
-	// capacity into pageable memory and out of it again took four fifths of a call: 20 queries with 1.6e5 groups
-	// 0.85 -> 0.27 ms in the engine.) Past 32 MB of capacity the memory held would outweigh that.
+	// Host results of moderate size go straight to page-locked memory: only the groups there are cross the link, as
+	// the finalize kernel finds them. (Copies of the whole capacity into pageable memory and out of it again took
+	// four fifths of a call: 20 queries with 1.6e5 groups 0.85 -> 0.27 ms in the engine.) Past 32 MB of capacity the
+	// memory held would outweigh that. A query has a buffer of its own, so that a result that is kept holds its own
+	// capacity alone; the smallest share buffers of 64 KB, the least that the pool gives out.
+	auto padded = [&](size_t qi, size_t w) { return (e.out_cap[qi] * TypeSize(out_types[w]) + 255) / 256 * 256; };
 	uint64_t capacity = 0;
-	for (size_t w = 0; w < out_words; w++) capacity += (std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]) + 255) / 256 * 256;
-	std::shared_ptr<uint8_t> host;
-	std::vector<uint64_t> host_off(out_words, 0);
+	for (size_t qi = 0; qi < qs.size(); qi++) {
+		for (size_t w = 0; w < out_words; w++) capacity += padded(qi, w);
+	}
+	std::vector<std::shared_ptr<uint8_t>> host;  // per query
 	if (!options.output_on_device && capacity <= (32ull << 20)) {
-		host = PinnedPool::Get().Acquire(capacity);
-		uint64_t off = 0;
-		for (size_t w = 0; w < out_words; w++) {
-			host_off[w] = off;
-			e.outp_host[w] = reinterpret_cast<uint64_t>(host.get() + off);
-			off += (std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]) + 255) / 256 * 256;
+		constexpr uint64_t kShared = 64 * 1024;
+		std::shared_ptr<uint8_t> buffer;
+		uint64_t used = kShared;
+		for (size_t qi = 0; qi < qs.size(); qi++) {
+			uint64_t bytes = 0;
+			for (size_t w = 0; w < out_words; w++) bytes += padded(qi, w);
+			if (used + bytes > kShared) {
+				buffer = PinnedPool::Get().Acquire(std::max(bytes, kShared));
+				used = 0;
+			}
+			host.push_back(std::shared_ptr<uint8_t>(buffer, buffer.get() + used));
+			for (size_t w = 0; w < out_words; w++) {
+				e.outp_host[qi * out_words + w] = reinterpret_cast<uint64_t>(buffer.get() + used);
+				used += padded(qi, w);
+			}
 		}
 	} else {
 		for (size_t w = 0; w < out_words; w++) {
 			holder->ptrs.push_back(Runtime::Get().allocator().Alloc(std::max<uint64_t>(1, e.out_rows) * TypeSize(out_types[w]), stream));
-			e.outp_host[w] = reinterpret_cast<uint64_t>(holder->ptrs[w]);
 		}
+		device_outputs(e, holder->ptrs);
 	}
-	VGPU_CUDA(cudaMemcpyAsync(e.outp, e.outp_host, out_words * 8, cudaMemcpyHostToDevice, stream));
+	VGPU_CUDA(cudaMemcpyAsync(e.outp, e.outp_host, qs.size() * out_words * 8, cudaMemcpyHostToDevice, stream));
 	init_if_needed(e);
 	const bool can_graph = bopts.use_graph && stream != nullptr && stream != cudaStreamLegacy && stream != cudaStreamPerThread;
 	if (can_graph) {
@@ -668,7 +687,7 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 	}
 	if (!e.pinned) VGPU_CUDA(cudaMemcpyAsync(e.counts_host, e.counts, e.nq * 8, cudaMemcpyDeviceToHost, stream));
 	std::vector<std::vector<uint8_t>> host_out;
-	if (!options.output_on_device && !host) {
+	if (!options.output_on_device && host.empty()) {
 		host_out.resize(out_words);
 		for (size_t w = 0; w < out_words; w++) {
 			host_out[w].resize(e.out_rows * TypeSize(out_types[w]));
@@ -690,8 +709,8 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 			const size_t width = TypeSize(out_types[w]);
 			if (options.output_on_device) {
 				c.device_data = static_cast<char *>(holder->ptrs[w]) + e.out_base[qi] * width;
-			} else if (host) {
-				if (cnt) c.host = std::shared_ptr<uint8_t>(host, host.get() + host_off[w] + e.out_base[qi] * width);
+			} else if (!host.empty()) {
+				if (cnt) c.host = std::shared_ptr<uint8_t>(host[qi], reinterpret_cast<uint8_t *>(e.outp_host[qi * out_words + w]));
 			} else {
 				const uint8_t *src = host_out[w].data() + e.out_base[qi] * width;
 				c.data.assign(src, src + cnt * width);

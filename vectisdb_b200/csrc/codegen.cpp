@@ -2629,11 +2629,11 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	// packing, table placement and literal constants come from its row of the query table (L.qwords
 	// u64 words): [0] rows, [1+2i] source i data, [2+2i] source i validity (unused), [key_base+2j]
 	// key j minimum, [key_base+2j+1] key j shift | bits << 8, [dom_base] table slots D,
-	// [dom_base+1] accumulator offset, [dom_base+2] output row offset, [dom_base+3] 1 = shared-memory
+	// [dom_base+1] accumulator offset, [dom_base+2] 1 = shared-memory
 	// table, [param_base..] the literal constants as 64-bit patterns.
 	// vgpu_batch_gb args: w[0] queries, w[1] query table, w[2] tiles (uint2 query, tile), w[3] tiles,
 	//   w[4] tile work counter (u32*, zero at launch), w[5] accumulators (u64, F arrays of w[6] words), w[6] accumulator words
-	//   per field, w[7] output pointer table (u64 [out words]), w[8] group counts (u64 [queries]), w[9] rows per tile,
+	//   per field, w[7] output pointer table (u64 [queries][out words]), w[8] group counts (u64 [queries]), w[9] rows per tile,
 	//   w[10] segments (uint2 query, segment: 1024 table slots), w[11] live slots of each segment (u32).
 	std::ostringstream o;
 	o << Prologue();
@@ -2695,7 +2695,7 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	  << "\t\tif (tl.x != cur_q) {\n"
 	  << "\t\t\t// the CTA moves to another query: its shared table goes to the previous query's accumulators\n"
 	  << "\t\t\tif (cur_sm) {\n" << flush.str() << "\t\t\t}\n"
-	  << "\t\t\tcur_q = tl.x; cur_d = qp[" << L.dom_base << "]; cur_sm = qp[" << L.dom_base + 3 << "] != 0;\n";
+	  << "\t\t\tcur_q = tl.x; cur_d = qp[" << L.dom_base << "]; cur_sm = qp[" << L.dom_base + 2 << "] != 0;\n";
 	for (int f = 0; f < F; f++) {
 		o << "\t\t\tG" << f << " = acc + " << f << "ull * ACC + qp[" << L.dom_base + 1 << "];\n";
 	}
@@ -2752,8 +2752,8 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	  << "\tconst u32 q = sg.x;\n"
 	  << "\tconst u64 *qp = (const u64*)a.w[1] + (u64)q * " << L.qwords << "ull;\n"
 	  << "\tu64 *acc = (u64*)a.w[5];\n\tconst u64 ACC = a.w[6];\n"
-	  << "\tconst u64 *outp = (const u64*)a.w[7];\n"
-	  << "\tconst u64 D = qp[" << L.dom_base << "], outb = qp[" << L.dom_base + 2 << "];\n";
+	  << "\tconst u64 *outp = (const u64*)a.w[7] + (u64)q * " << nk + gb.aggs.size() << "ull;\n"
+	  << "\tconst u64 D = qp[" << L.dom_base << "];\n";
 	for (int f = 0; f < F; f++) o << "\tu64 *G" << f << " = acc + " << f << "ull * ACC + qp[" << L.dom_base + 1 << "];\n";
 	o << "\tconst u64 s = (u64)sg.y * 1024ull + threadIdx.x;\n"
 	  << "\tconst bool live = s < D && G0[s] != 0;\n"
@@ -2762,7 +2762,7 @@ std::string PipelineCodegen::EmitBatchGroupBy(const GroupBySpec &gb, const Geome
 	  << "\tu32 base = 0, total;\n"
 	  << "\tif (sg.y) block_exclusive_scan(before, scan_scratch, &base);\n"
 	  << "\tconst u32 off = block_exclusive_scan(live ? 1u : 0u, scan_scratch, &total);\n"
-	  << "\tif (live) {\n\t\tconst u64 pos = outb + base + off;\n\t\tconst u64 key = s;\n";
+	  << "\tif (live) {\n\t\tconst u64 pos = base + off;\n\t\tconst u64 key = s;\n";
 	for (int j = 0; j < nk; j++) {
 		const char *t = CudaTypeName(visible_[gb.keys[j].column].type);
 		o << "\t\t\t{ const u32 sb = (u32)qp[" << L.key_base + 2 * j + 1 << "]; const u32 bits = sb >> 8;\n"
