@@ -680,7 +680,8 @@ bool RunTemplate(const std::vector<Prepared *> &qs, const ExecOptions &options, 
 			stats->graph_replays++;
 		}
 		LaunchScope scope("vgpu_batch_graph", stream, e.in_bytes, e.rows);
-		Runtime::Get().CountLaunch(2);  // the aggregate and finalize kernels inside the graph
+		// the graph's kernels -- aggregate, the count of the segments if there is one, finalize -- of which the scope counts one
+		Runtime::Get().CountLaunch(e.nseg > e.nq ? 2 : 1);
 		VGPU_CUDA(cudaGraphLaunch(e.graph, stream));
 	} else {
 		enqueue(e, true);
