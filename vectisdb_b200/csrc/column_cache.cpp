@@ -209,17 +209,16 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 	auto &alloc = Runtime::Get().allocator();
 	std::vector<std::pair<std::string, Entry>> done;
 	std::vector<kern::BoundsColumn> ranged;
-	for (auto &kv : it->second) {
-		Staged &st = kv.second;
+	auto build = [&](const std::string &name, Staged &st) {
 		if (st.failed || st.rows != scanned_rows) {
 			for (auto &c : st.chunks) {
 				staged_ -= c.bytes;
 				FreeChunk(c);
 			}
-			continue;
+			return;
 		}
 		Entry e;
-		e.column.name = kv.first;
+		e.column.name = name;
 		e.column.type = st.type;
 		e.column.rows = st.rows;
 		bool any_valid = false;
@@ -256,25 +255,43 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		if (IsIntegerKeyType(st.type) || st.type == ValueType::DICTIONARY_STRING) {
 			ranged.push_back({e.column.data, st.rows, kern::SignedBoundsKind(st.type)});
 		}
-		done.emplace_back(kv.first, std::move(e));
+		done.emplace_back(name, std::move(e));
+	};
+	// the integer columns' ranges and distinct counts: one launch and one read-back for the table. What is finished
+	// when a column fails (no memory, say) is committed, without ranges if those are what failed, and no longer staged.
+	std::exception_ptr failure;
+	int columns = 0;
+	std::vector<uint64_t> bounds;
+	uint64_t *mm = nullptr;
+	for (auto col = it->second.begin(); !failure && col != it->second.end();) {
+		try {
+			build(col->first, col->second);
+			col = it->second.erase(col);
+		} catch (...) {
+			failure = std::current_exception();
+		}
 	}
-	// the integer columns' ranges and distinct counts: one launch and one read-back for the table
-	const int columns = static_cast<int>(ranged.size());
-	std::vector<uint64_t> bounds(kern::BoundsWords(columns, true));
-	if (!ranged.empty()) {
-		uint64_t *mm = static_cast<uint64_t *>(alloc.Alloc(bounds.size() * 8, s));
-		kern::ColumnBounds(ranged.data(), columns, mm, s, true);
-		VGPU_CUDA(cudaMemcpyAsync(bounds.data(), mm, bounds.size() * 8, cudaMemcpyDeviceToHost, s));
-		VGPU_CUDA(cudaStreamSynchronize(s));
-		alloc.Free(mm, s);
+	try {
+		if (!ranged.empty()) {
+			std::vector<uint64_t> words(kern::BoundsWords(static_cast<int>(ranged.size()), true));
+			mm = static_cast<uint64_t *>(alloc.Alloc(words.size() * 8, s));
+			kern::ColumnBounds(ranged.data(), static_cast<int>(ranged.size()), mm, s, true);
+			VGPU_CUDA(cudaMemcpyAsync(words.data(), mm, words.size() * 8, cudaMemcpyDeviceToHost, s));
+			VGPU_CUDA(cudaStreamSynchronize(s));
+			bounds = std::move(words);
+			columns = static_cast<int>(ranged.size());
+		}
+	} catch (...) {
+		if (!failure) failure = std::current_exception();
 	}
+	alloc.Free(mm, s);
 	size_t next = 0;
 	for (auto &named : done) {
 		Entry &e = named.second;
 		if (IsIntegerKeyType(e.column.type) || e.column.type == ValueType::DICTIONARY_STRING) {
-			const uint64_t *words = &bounds[2 * next];
-			const kern::BoundsKind kind = ranged[next].kind;
-			if (e.column.rows > 0) {
+			if (columns && e.column.rows > 0) {
+				const uint64_t *words = &bounds[2 * next];
+				const kern::BoundsKind kind = ranged[next].kind;
 				e.column.distinct = kern::DistinctEstimate(bounds.data(), columns, static_cast<int>(next), kind);
 				e.column.has_stats = true;
 				e.column.min = static_cast<int64_t>(kern::BoundsLow(words, kind));
@@ -293,9 +310,11 @@ void ColumnCache::CommitStaging(const TableRef &table, uint64_t scanned_rows) {
 		auto &cols = table_columns_[tk];
 		if (std::find(cols.begin(), cols.end(), named.first) == cols.end()) cols.push_back(named.first);
 	}
+	if (!done.empty()) generation_[tk]++;  // new contents: identities taken before no longer match
+	if (failure) std::rethrow_exception(failure);
 	VGPU_CUDA(cudaStreamSynchronize(s));
 	staging_.erase(it);
-	generation_[tk]++;  // new contents: identities taken before no longer match
+	if (done.empty()) generation_[tk]++;
 }
 
 void ColumnCache::AbortStaging(const TableRef &table) {
