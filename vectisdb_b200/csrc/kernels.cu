@@ -592,9 +592,8 @@ __global__ void __launch_bounds__(kExpandBlock) JoinExpandKernel(const uint64_t 
 
 // info of the kernels below: [0] runs listed for the last of them, [1] the longest run, [2] the cursor of the runs'
 // places; zero at the first launch. A run past kJoinRunLimit makes the result useless: from then on they return.
-__device__ __forceinline__ bool JoinRunTooLong(const uint32_t *info) {
-	return *reinterpret_cast<const volatile uint32_t *>(info + 1) > kJoinRunLimit;
-}
+// (Read through L1: a load of that one word past it from every warp took as long as the rest of such a pass.)
+__device__ __forceinline__ bool JoinRunTooLong(const uint32_t *info) { return __ldg(info + 1) > kJoinRunLimit; }
 
 // Dense keys: an entry per key value, x = end of its run in `rows`, y = its length. Adds to one entry queue at its
 // address (0.7 ns each: a key in every second of 4M rows held this kernel for 1.4 ms), so a warp with equal
@@ -602,9 +601,10 @@ __device__ __forceinline__ bool JoinRunTooLong(const uint32_t *info) {
 template <typename K>
 __global__ void JoinEntryCountKernel(const K *keys, uint64_t n, uint64_t bias, uint2 *entries, uint32_t *info) {
 	const uint32_t lane = threadIdx.x & 31;
-	for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); w < n; w += (uint64_t)gridDim.x * blockDim.x) {
-		if (__any_sync(0xffffffffu, JoinRunTooLong(info))) return;
-		const uint64_t i = w + lane;
+	for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
+		// (this launch writes the word: past L1, once for the CTA)
+		if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t *>(info + 1) > kJoinRunLimit)) return;
+		const uint64_t i = base + threadIdx.x;
 		const uint64_t k = static_cast<uint64_t>(keys[i < n ? i : n - 1]) - bias;
 		const uint64_t next = __shfl_down_sync(0xffffffffu, k, 1);
 		const uint32_t live = __ballot_sync(0xffffffffu, i < n);
@@ -624,7 +624,8 @@ __global__ void JoinEntryCountKernel(const K *keys, uint64_t n, uint64_t bias, u
 // its start.
 __global__ void __launch_bounds__(256) JoinEntryPlaceKernel(uint2 *entries, uint64_t count, uint32_t *info) {
 	__shared__ uint32_t scratch[33], base;
-	if (__syncthreads_or(JoinRunTooLong(info))) return;
+	const bool stop = threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t *>(info + 1) > kJoinRunLimit;  // (written here)
+	if (__syncthreads_or(stop)) return;
 	uint32_t longest = 0;
 	for (uint64_t first = blockIdx.x * 1024ull; first < count; first += gridDim.x * 1024ull) {
 		const uint64_t i = first + threadIdx.x * 4ull;
@@ -647,8 +648,13 @@ __global__ void __launch_bounds__(256) JoinEntryPlaceKernel(uint2 *entries, uint
 		}
 		__syncthreads();
 	}
+	__shared__ uint32_t most;
+	if (threadIdx.x == 0) most = 0;
+	__syncthreads();
 	longest = __reduce_max_sync(0xffffffffu, longest);
-	if ((threadIdx.x & 31) == 0 && longest > *reinterpret_cast<volatile uint32_t *>(info + 1)) atomicMax(info + 1, longest);
+	if ((threadIdx.x & 31) == 0) atomicMax(&most, longest);
+	__syncthreads();
+	if (threadIdx.x == 0 && most > *reinterpret_cast<volatile uint32_t *>(info + 1)) atomicMax(info + 1, most);
 }
 
 // Each right row's number into its key's run, in any order; entry x moves to the run's end.
