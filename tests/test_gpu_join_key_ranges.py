@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from vectisdb_b200 import GpuEngine, make_aggregate, make_column, make_group_by, make_join, make_scan
-from vectisdb_b200.engine import GpuAggregateKind as A, GpuValueType as T
+from vectisdb_b200.engine import GpuAggregateKind as A, GpuValueType as T, profile_drain, profile_enable
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +36,32 @@ def test_unmatched_right_rows_do_not_widen_the_keys(keys, repeat):
     got = np.stack([c.data.astype(np.int64) for c in r.columns[:-1]], axis=1)
     sort = np.lexsort(got.T[::-1])
     assert np.array_equal(got[sort], groups) and np.array_equal(r.columns[-1].data[sort], counts)
+
+
+@pytest.mark.parametrize("extra", [False, True])
+@pytest.mark.parametrize("outlier", [False, True])
+def test_an_unmatched_outlier_keeps_the_shared_memory_table(outlier, extra):
+    """Two hundred codes and one far off that no left row meets; with a second right column they are read by row."""
+    rng = np.random.default_rng(3)
+    n = 200_000
+    rk = rng.permutation(n).astype(np.int64)
+    code = rng.integers(0, 200, n).astype(np.int32)
+    if outlier:
+        code[rk == n - 1] = np.iinfo(np.int32).min
+    y = rng.integers(0, 9, n)
+    lk = rng.integers(0, n - 1, 300_001).astype(np.int64)
+    right = [make_column("rk", T.INT64, rk), make_column("code", T.INT32, code)] + ([make_column("y", T.INT64, y)] if extra else [])
+    plan = make_group_by(["code"], [make_aggregate(A.COUNT_STAR, "", T.INT64)] + ([make_aggregate(A.MAX, "y", T.INT64)] if extra else []),
+                         make_join("lk", "rk", ["code"] + (["y"] if extra else []), make_scan(["lk"]), make_scan([c.name for c in right])))
+    profile_drain()
+    profile_enable(True)
+    try:
+        r = GpuEngine.instance().execute_plan(plan, [make_column("lk", T.INT64, lk)] + right)
+        names = [rec[0] for rec in profile_drain()]
+    finally:
+        profile_enable(False)
+    assert r.success, r.error_message
+    assert "vgpu_gb_direct" in names and ("vgpu_stats" in names) == outlier, names
+    at = np.argsort(rk)[lk]
+    keys, counts = np.unique(code[at], return_counts=True)
+    assert np.array_equal(r.columns[0].data, keys) and np.array_equal(r.columns[1].data, counts)

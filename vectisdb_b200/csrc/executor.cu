@@ -966,7 +966,16 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin, boo
 		}
 	};
 	pack();
-	if (shift > 63 && pin.spec.join) {  // right rows without a match may hold any value
+	// Right rows of a join that no left row meets may hold any value. Where that may be what makes the keys too wide to
+	// pack, or one with few values too wide for a shared-memory table, the join is run for the ranges of the rows it keeps.
+	bool joined = pin.spec.join && shift > 63;
+	for (size_t i = 0; pin.spec.join && shift > 13 && i < key_cols.size(); i++) {
+		const PipeColumn &vc = cg.visible()[key_cols[i]];
+		if (vc.source < 0 || pin.spec.sources[vc.source].side != 1) continue;
+		const DevColumn &src = pin.sources[vc.source];
+		joined = joined || ((!src.has_stats || src.unjoined_stats) && gb.keys[i].bits > 13 && distinct[i] && distinct[i] <= (1u << 13));
+	}
+	if (joined) {
 		ComputeStats(pin, cg, key_cols, ranges, distinct, true);
 		pack();
 	}
@@ -1809,6 +1818,7 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 	}
 	// range of the inline column's raw bits, once known
 	uint32_t vmin = 0, vmax = 0;
+	uint64_t vdistinct = 0;  // about how many values it has, 0 = not known
 	bool have_vrange = false;
 	auto add_sources = [&](bool sorted_side, const uint32_t *perm) {
 		for (size_t i = 0; i < outs.size(); i++) {
@@ -1832,6 +1842,7 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 				if ((vmin & sign) == (vmax & sign)) {
 					const uint64_t high = (vmin & sign) ? ~0ull << (8 * w) : 0ull;
 					c.has_stats = c.unjoined_stats = true;
+					c.distinct = vdistinct;
 					c.min = c.type == ValueType::BOOLEAN ? 0 : static_cast<int64_t>(vmin | high);
 					c.max = c.type == ValueType::BOOLEAN ? 1 : static_cast<int64_t>(vmax | high);
 				}
@@ -1907,14 +1918,17 @@ Relation Executor::JoinForPipeline(const PlanNode &node, PipelineInput &pin, boo
 			const size_t vw = inline_col ? TypeSize(inline_col->type) : 4;
 			const kern::BoundsColumn want[2] = {{rk->data, rn, kern::RawBoundsKind(kw)},
 			                                    {inline_col ? inline_col->data : nullptr, rn, kern::RawBoundsKind(vw)}};
-			uint64_t *words = arena_.AllocT<uint64_t>(4);
-			kern::ColumnBounds(want, inline_col ? 2 : 1, words, stream_);
-			const std::vector<uint64_t> host = ReadWords(words, inline_col ? 4 : 2);
+			const int measured = inline_col ? 2 : 1;
+			const size_t count = kern::BoundsWords(measured, inline_col != nullptr);
+			uint64_t *words = arena_.AllocT<uint64_t>(count);
+			kern::ColumnBounds(want, measured, words, stream_, inline_col != nullptr);
+			const std::vector<uint64_t> host = ReadWords(words, count);
 			lo = kern::BoundsLow(&host[0], want[0].kind);
 			hi = kern::BoundsHigh(&host[0], want[0].kind);
 			if (inline_col) {
 				vmin = static_cast<uint32_t>(kern::BoundsLow(&host[2], want[1].kind));
 				vmax = static_cast<uint32_t>(kern::BoundsHigh(&host[2], want[1].kind));
+				vdistinct = kern::DistinctEstimate(host.data(), measured, 1, want[1].kind);
 			}
 		}
 		have_vrange = inline_col != nullptr;
