@@ -995,9 +995,12 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin, boo
 	const bool direct_l2 = direct && direct_f64 > 0 && env_dl2 && std::strcmp(env_dl2, "1") == 0;
 	// Past the shared-memory tables: one pass into a table of the whole key space in global memory while L2
 	// holds it (64 MB of its 126; the same reductions run at a third of the rate from 128 MB on), else the
-	// partitioned strategies. Below that size it wins at every row count, key distribution and number of
-	// aggregates measured, SUM and COUNT or SUM, SUM and MAX: 300K rows into 2^20 keys 0.11 against 0.14 ms, 20M
-	// 0.36 against 0.94 ms uniform and 0.62 against 0.94 ms Zipf(1.1), 1.34e8 skewed rows 2.1 against 2.4 ms.
+	// partitioned strategies. One reduction a row and state word: with two words it wins at every row count and key
+	// distribution measured (300K rows into 2^20 keys 0.11 against 0.14 ms, 20M 0.36 against 0.94 ms uniform and 0.62
+	// against 0.94 ms Zipf(1.1)), and up to a million rows with any number. With more of both the partitioned bucket
+	// pass, in shared memory, is the faster, the sooner the fewer the slots that the reductions meet in (8M evenly
+	// spread rows into 2^12 slots, five words 0.56 against 0.43 ms, into 2^18 0.42 and 0.45, into 2^21 0.82 and 0.46; 30M,
+	// four words, into 2^13 1.21 and 0.71, into 2^18 0.72 and 1.09; ten words 8M into 2^14 0.64 and 0.52, into 2^18 0.58 and 0.54).
 	// Few rows leave most of such a table unused: it is taken only where the budget has room for it (4096 rows into 2^22
 	// keys 0.124 against 0.143 ms, but 67 MB against 0.2).
 	// VGPU_GB_STRATEGY: "l2" or one of the partitioned ones (testing); the partition overrides keep those too.
@@ -1014,13 +1017,14 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin, boo
 		}
 		ag.sum64 = most <= ((1ull << 63) - 1) / n;
 	}
-	// Up to 128 MB where the rows are neither few to a key (the table's own two passes take 0.13 ms) nor many: SUM and
-	// COUNT of 9M rows by 4.3M keys 0.52 ms of kernels partitioned, 0.33 in one pass; 17M rows by 8M keys 0.86 and
-	// 0.83; 34M skewed rows by 3.2M keys, four aggregates, 0.83 and 0.75 ms, but 2.6M of them by 2.1M keys 0.158 and
-	// 0.184, and 1.34e8 by 3.2M 2.40 and 2.53.
-	const uint64_t l2_most = PipelineCodegen::kL2TableBytes * (domain <= n && n / 8 <= domain ? 2 : 1);
-	bool l2 = waits && !direct && shift >= 10 && shift <= 26 &&
-	          domain * static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2)) * 8 <= l2_most &&
+	const uint64_t l2_words = static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2));
+	const bool l2_pays = l2_words <= 2 || n <= (1u << 20) || l2_words * n <= (l2_words <= 7 ? 820 : 60) * domain;
+	// Up to 128 MB with two words where the rows are neither few to a key (the table's own two passes take 0.13 ms) nor
+	// many: SUM and COUNT of 9M rows by 4.3M keys 0.52 ms of kernels partitioned, 0.33 in one pass; 17M rows by 8M keys
+	// 0.86 and 0.83. With three, 8M rows by 4M keys take 0.51 against 0.37 ms.
+	const uint64_t l2_most = PipelineCodegen::kL2TableBytes * (l2_words <= 2 && domain <= n && n / 8 <= domain ? 2 : 1);
+	bool l2 = waits && !direct && shift >= 10 && shift <= 26 && l2_pays &&
+	          domain * l2_words * 8 <= l2_most &&
 	          cg.L2ChainWord(gb_l2) + 1 < kKeyWord;
 	if (const char *env = std::getenv("VGPU_GB_STRATEGY")) l2 = l2 && std::strcmp(env, "l2") == 0;
 	if (std::getenv("VGPU_GB_TABLE_SLOTS") || std::getenv("VGPU_GB_PARTITIONS")) l2 = false;
@@ -1032,7 +1036,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin, boo
 		const uint64_t rows = pin.spec.join_multi ? domain : std::min<uint64_t>(domain, n);
 		return Room(slots * slot + slots / 64 + (64 << 10) + rows * out_row);
 	};
-	l2 = l2 && table_room(domain, 8 * static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2)));
+	l2 = l2 && table_room(domain, 8 * l2_words);
 	// Direct-partitioned when the packed key space is dense enough to be walked slot by slot
 	// (at most 4 slots per input row) and splits into at most 2^14 partitions of the largest
 	// shared-memory table: a row then costs no hashing and no probing.
@@ -1054,7 +1058,7 @@ Relation Executor::GroupByPipeline(const PlanNode &node, PipelineInput &pin, boo
 	// early, and the rows are partitioned. 8M rows of 600K ids, SUM and COUNT: 0.62 -> 0.28 ms, of 100 ids 2.17 ->
 	// 0.26; 70K rows of 1000 ids 0.139 -> 0.104; 3M or 30M different ids as before. What several keys come to together is
 	// not known: see vgpu_gb_l2_guess.
-	const uint64_t l2_slot = 8 * (1 + static_cast<uint64_t>(PipelineCodegen::StateWords(gb_l2)));
+	const uint64_t l2_slot = 8 * (1 + l2_words);
 	uint64_t l2_slots = std::min<uint64_t>(FloorPow2(PipelineCodegen::kL2TableBytes / l2_slot),
 	                                       std::max<uint64_t>(2048, NextPow2(2 * std::min<uint64_t>(n, 1ull << 32))));
 	// one key whose distinct values are known to be few: no larger a table to fill and to walk than they need
