@@ -1,0 +1,62 @@
+"""The one-pass row filter's larger tiles for narrow rows on the B200, against numpy: every width around the choice of the
+tile, rows around its size, columns that start off a vector's boundary, and predicates over more than the outputs."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from vectisdb_b200 import GpuEngine, make_column, make_expr, make_filter, make_projection, make_scan
+from vectisdb_b200.engine import GpuValueType as T, make_device_column, profile_drain, profile_enable
+
+pytestmark = pytest.mark.gpu
+WIDTHS = {1: [T.BOOLEAN], 2: [T.INT16], 4: [T.INT32], 5: [T.INT32, T.BOOLEAN], 8: [T.INT32, T.INT32], 12: [T.INT64, T.INT32],
+          13: [T.INT64, T.INT32, T.BOOLEAN]}
+NP = {T.BOOLEAN: np.uint8, T.INT16: np.int16, T.INT32: np.int32, T.INT64: np.int64}
+C = {T.BOOLEAN: "bool", T.INT16: "short", T.INT32: "int", T.INT64: "long long"}
+
+
+def _run(plan, cols):
+    profile_drain()
+    profile_enable(True)
+    try:
+        r = GpuEngine.instance().execute_plan(plan, cols)
+        names = [rec[0] for rec in profile_drain()]
+    finally:
+        profile_enable(False)
+    assert r.success, r.error_message
+    assert "vgpu_mat_onepass" in names, names
+    return [c.data for c in r.columns]
+
+
+@pytest.mark.parametrize("skip", [0, 1])
+@pytest.mark.parametrize("rows", [1, 15, 2047, 2048, 2049, 4097, 300_001])
+@pytest.mark.parametrize("width", WIDTHS)
+def test_every_width(width, rows, skip):
+    rng = np.random.default_rng(rows + width)
+    values, cols, keep = [], [], []
+    for i, t in enumerate(WIDTHS[width]):
+        v = rng.integers(0, 2 if t == T.BOOLEAN else 100, rows + skip).astype(NP[t])
+        dev = torch.from_numpy(v).cuda()
+        keep.append(dev)
+        values.append(v[skip:])
+        cols.append(make_device_column(f"c{i}", t, dev.data_ptr() + skip * dev.element_size(), rows))
+    torch.cuda.synchronize()
+    bound = 1 if WIDTHS[width][0] == T.BOOLEAN else 43
+    plan = make_filter([make_expr(f"((bool*)out)[idx] = ((const {C[WIDTHS[width][0]]}*)inputs[0])[row] < {bound};", ["c0"], T.BOOLEAN)],
+                       make_scan([c.name for c in cols]))
+    got = _run(plan, cols)
+    for g, v in zip(got, values):
+        assert np.array_equal(g, v[values[0] < bound])
+
+
+def test_a_narrow_output_of_wide_predicates():
+    rng = np.random.default_rng(1)
+    n = 100_003
+    xs = [rng.standard_normal(n) for _ in range(5)]
+    k = rng.integers(0, 1000, n).astype(np.int32)
+    cond = " && ".join(f"((const double*)inputs[{i}])[row] < 1.0" for i in range(5))
+    names = [f"x{i}" for i in range(5)]
+    plan = make_projection([make_expr("((int*)out)[idx] = ((const int*)inputs[0])[row];", ["k"], T.INT32)],
+                           make_filter([make_expr(f"((bool*)out)[idx] = {cond};", names, T.BOOLEAN)], make_scan(names + ["k"])))
+    got = _run(plan, [make_column(f"x{i}", T.FLOAT64, x) for i, x in enumerate(xs)] + [make_column("k", T.INT32, k)])
+    assert np.array_equal(got[0], k[np.all([x < 1.0 for x in xs], axis=0)])

@@ -644,7 +644,8 @@ uint64_t PipelineCodegen::OnePassRowBytes(const std::vector<int> &outs) const {
 // bytes keeping 43% 0.179 ms in the three launches -> 0.104 ms (4.6 TB/s; 0.196 ms when each tile was written
 // as soon as its start was known, 0.133 ms without the loads in flight), 6M fact rows against a 200K-row
 // dimension 0.105 -> 0.055 ms. 128 threads x 4 rows: the smallest tile that still writes full sectors keeps
-// the most CTAs apart in their phases (256 x 4 0.110 ms, 128 x 8 0.121 ms, 64 x 8 0.141 ms).
+// the most CTAs apart in their phases (256 x 4 0.110 ms, 128 x 8 0.121 ms, 64 x 8 0.141 ms); the caller takes more rows
+// a thread where they are narrow.
 // Arguments: cb = total rows (u64, the top bit set on failure), ticket, tile counts (u32, an even number of
 // them), tile starts, all zero at launch; outputs as in the two-pass form. Dynamic shared memory:
 // two tiles of OnePassRowBytes per row.
