@@ -60,3 +60,21 @@ def test_a_narrow_output_of_wide_predicates():
                            make_filter([make_expr(f"((bool*)out)[idx] = {cond};", names, T.BOOLEAN)], make_scan(names + ["k"])))
     got = _run(plan, [make_column(f"x{i}", T.FLOAT64, x) for i, x in enumerate(xs)] + [make_column("k", T.INT32, k)])
     assert np.array_equal(got[0], k[np.all([x < 1.0 for x in xs], axis=0)])
+
+
+@pytest.mark.parametrize("rows,columns,one_pass", [(1 << 20, 11, True), ((1 << 20) + 1, 11, False), ((1 << 20) + 1, 6, True),
+                                                   ((1 << 20) + 1, 7, False)])
+def test_wide_rows_of_large_inputs_take_two_passes(rows, columns, one_pass):
+    x = (np.arange(rows) % 100).astype(np.int32)
+    y = np.arange(rows, dtype=np.int64)
+    names = ["x"] + [f"y{i}" for i in range(columns)]
+    plan = make_filter([make_expr("((bool*)out)[idx] = ((const int*)inputs[0])[row] < 30;", ["x"], T.BOOLEAN)], make_scan(names))
+    profile_drain()
+    profile_enable(True)
+    try:
+        r = GpuEngine.instance().execute_plan(plan, [make_column("x", T.INT32, x)] + [make_column(n, T.INT64, y) for n in names[1:]])
+        launched = [rec[0] for rec in profile_drain()]
+    finally:
+        profile_enable(False)
+    assert r.success and ("vgpu_mat_onepass" in launched) == one_pass, launched
+    assert all(np.array_equal(c.data, v[x < 30]) for c, v in zip(r.columns, [x] + [y] * columns))

@@ -556,9 +556,11 @@ Relation Executor::Materialize(PipelineInput &pin, const std::vector<int> &out_c
 	// while that is at most 8 GiB and within the budget (with as much again three times over for the operators above,
 	// where there are any), and unless the plan's own estimate says that under
 	// two rows in five survive (what the admission estimate charges for the outputs then stays near what
-	// they take). Its two staged tiles of 512 rows allow 96 bytes a row (96 KB a CTA, two CTAs per SM).
+	// they take). Its two staged tiles of 512 rows allow 96 bytes a row (96 KB a CTA, two CTAs per SM); over more than a
+	// million rows 56, since few CTAs and many registers then cost more than the second pass (30% of 4M rows kept, of 52
+	// bytes 0.133 against 0.158 ms, of 60 0.160 and 0.157, of 84 0.264 and 0.209; 1M rows of 92 bytes 0.109 and 0.129).
 	// VGPU_MAT_PASSES=2: always two (testing).
-	bool one_pass = waits && cg.has_filter() && n > 0 && !pin.spec.join_multi && row_bytes > 0 && row_bytes <= 96 &&
+	bool one_pass = waits && cg.has_filter() && n > 0 && !pin.spec.join_multi && row_bytes > 0 && row_bytes <= (n <= (1u << 20) ? 96u : 56u) &&
 	                n <= (8ull << 30) / row_bytes && Room((at_root ? 1 : 4) * n * row_bytes);
 	for (const PlanNode *node : pin.spec.chain) {
 		if (node->op == OpType::FILTER && node->estimated_rows && 5 * node->estimated_rows < 2 * n) one_pass = false;
