@@ -5,7 +5,8 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from vectisdb_b200 import GpuEngine, make_column, make_expr, make_filter, make_projection, make_scan
+from vectisdb_b200 import (ExecuteOptions, GpuEngine, device_to_host, make_column, make_expr, make_filter, make_projection,
+                           make_scan)
 from vectisdb_b200.engine import GpuValueType as T, make_device_column, profile_drain, profile_enable
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +79,27 @@ def test_wide_rows_of_large_inputs_take_two_passes(rows, columns, one_pass):
         profile_enable(False)
     assert r.success and ("vgpu_mat_onepass" in launched) == one_pass, launched
     assert all(np.array_equal(c.data, v[x < 30]) for c, v in zip(r.columns, [x] + [y] * columns))
+
+
+@pytest.mark.parametrize("bound,estimate,one_pass", [(0, 0, False), (5, 0, False), (60, 0, True), (5, 40_000_000, True)])
+def test_a_sample_of_a_large_input_chooses_the_form(bound, estimate, one_pass):
+    rows = 46_000_001  # of 12 bytes
+    x = (torch.arange(rows, device="cuda") // 7 % 100).to(torch.int32)
+    y = torch.arange(rows, device="cuda")
+    cols = [make_device_column("x", T.INT32, x.data_ptr(), rows), make_device_column("y", T.INT64, y.data_ptr(), rows)]
+    plan = make_filter([make_expr(f"((bool*)out)[idx] = ((const int*)inputs[0])[row] < {bound};", ["x"], T.BOOLEAN)],
+                       make_scan(["x", "y"]))
+    plan.estimated_rows = estimate
+    torch.cuda.synchronize()
+    profile_drain()
+    profile_enable(True)
+    try:
+        r = GpuEngine.instance().execute_plan(plan, cols, ExecuteOptions(output_on_device=True))
+        names = [rec[0] for rec in profile_drain()]
+    finally:
+        profile_enable(False)
+    got = [device_to_host(c) for c in r.columns]
+    r.free()
+    assert ("vgpu_mat_onepass" in names) == one_pass and ("vgpu_mat_sample" in names) == (estimate == 0), names
+    keep = (x < bound).cpu().numpy()
+    assert np.array_equal(got[0], x.cpu().numpy()[keep]) and np.array_equal(got[1], np.flatnonzero(keep))

@@ -670,6 +670,15 @@ std::string PipelineCodegen::EmitMaterializeOnePass(const std::vector<int> &outs
 		voff[c] = bytes;
 		bytes += g.tile();
 	}
+	// How many of kSampleRows rows, spread over the input, pass: for the caller's choice over large inputs.
+	Geometry one = g;
+	one.items = 1;
+	const auto first = NeededSources({});
+	o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_mat_sample(KArgs a) {\n" << kKernelHead
+	  << "\tconst u64 sample = blockIdx.x * (u64)blockDim.x + threadIdx.x, apart = n / " << kSampleRows << "ull;\n"
+	  << LoadBlock(one, first, true, "sample * apart + mix64(sample) % apart") << "\t\tint passed = 0;\n" << ItemOpen(one, first)
+	  << chain_code_ << "\t\tpassed = keep ? 1 : 0;\n" << ItemClose() << "\tconst int all = __syncthreads_count(passed);\n"
+	  << "\tif (threadIdx.x == 0) atomicAdd((u64*)a.w[" << cb << "], (u64)all);\n}\n\n";
 	o << "extern \"C\" __global__ void __launch_bounds__(" << g.block << ") vgpu_mat_onepass(KArgs a) {\n"
 	  << kKernelHead << "\textern __shared__ __align__(16) char vgpu_st[];\n"
 	  << "\t__shared__ u32 scan_scratch[33];\n\t__shared__ u32 vgpu_next;\n\t__shared__ u64 vgpu_base;\n"

@@ -110,7 +110,9 @@ public:
 	//! vgpu_mat_write exists and writes row-aligned.
 	std::string EmitMaterialize(const std::vector<int> &out_columns, const Geometry &g) const;
 	//! The form that reads its inputs once (a row filter, no multi-match join): kernel vgpu_mat_onepass, with
-	//! 2 * tile rows * OnePassRowBytes of dynamic shared memory.
+	//! 2 * tile rows * OnePassRowBytes of dynamic shared memory; and vgpu_mat_sample over kSampleRows rows (its only
+	//! argument: the count of those that pass, u64, zero at launch).
+	static constexpr uint64_t kSampleRows = 1 << 16;
 	std::string EmitMaterializeOnePass(const std::vector<int> &out_columns, const Geometry &g) const;
 	uint64_t OnePassRowBytes(const std::vector<int> &out_columns) const;
 
